@@ -64,7 +64,7 @@ struct tlr_plan {
   double *T = nullptr, *P = nullptr, *Z = nullptr, *C = nullptr, *gscr = nullptr, *gsv = nullptr;
   double *parts = nullptr, *fparts = nullptr;
   // recompression scratch
-  int nslots = 0, nsm = 148;
+  int nslots = 0, nslots_general = 0, nsm = 148;
   size_t slot_doubles = 0;
   double* rcs = nullptr;
   int* rc_next = nullptr;  // per factorization step: claims of trailing pairs past the grid
@@ -130,12 +130,13 @@ struct tlr_plan {
   size_t d_split_cap = 0;
   tlr::TcOperands* d_tcops = nullptr;
   size_t d_tcops_cap = 0;
-  // forward pass (compression, factorization, solve) captured once per precision in a CUDA graph
-  // on a private stream and replayed on `stream`; the launch sequence depends only on the plan
+  // forward pass (compression, factorization, solve) captured once per precision and kind of rule
+  // (rounded storage or not) in a CUDA graph on a private stream and replayed on `stream`; the launch
+  // sequence depends on nothing else
   bool use_graphs = true;
   cudaStream_t cap_stream = nullptr;
-  cudaGraphExec_t fwd_exec[2] = {nullptr, nullptr};
-  long long fwd_launch[2][TLR_NKINDS] = {};
+  cudaGraphExec_t fwd_exec[4] = {nullptr, nullptr, nullptr, nullptr};
+  long long fwd_launch[4][TLR_NKINDS] = {};
   // block-row cyclic partition (tlr_plan_set_partition): this plan holds block rows i with
   // i % pworld == prank; tmap lists their tiles (nown of them) for the compression
   int prank = 0, pworld = 1;
@@ -269,10 +270,15 @@ int run_factorization(tlr_plan* p) {
                                                    p->status, sd));
       TRY(cuda_check(cudaEventRecord(p->ev_diag, sd), "event"));
     }
-    LAUNCH(TLR_K_RECOMPRESS, tlr::launch_recompress(p->n, p->b, k, p->nB, p->U, p->V, p->rank, p->cap, p->rcs,
-                                                    p->slot_doubles, p->nslots, p->rc_next + k,
-                                                    p->rlog + p->rlog_off[k], p->blog + p->rlog_off[k], 0, 1,
-                                                    p->status, s));
+    if (p->round_store)  // rounded factors are not orthogonal
+      LAUNCH(TLR_K_RECOMPRESS, tlr::launch_recompress_general(p->n, p->b, k, p->nB, p->U, p->V, p->rank, p->cap, p->rcs,
+                                                              p->slot_doubles, p->nslots_general, p->rc_next + k,
+                                                              p->rlog + p->rlog_off[k], p->blog + p->rlog_off[k],
+                                                              p->status, s));
+    else
+      LAUNCH(TLR_K_RECOMPRESS, tlr::launch_recompress(p->n, p->b, k, p->nB, p->U, p->V, p->rank, p->cap, p->rcs,
+                                                      p->slot_doubles, p->nslots, p->rc_next + k,
+                                                      p->rlog + p->rlog_off[k], 0, 1, p->status, s));
     if (ahead) TRY(cuda_check(cudaStreamWaitEvent(s, p->ev_diag, 0), "wait"));
   }
   LAUNCH(TLR_K_FINISH, tlr::launch_finish(p->nB, p->n, p->ldpart, p->qpart, p->out, p->status, s));
@@ -323,11 +329,11 @@ int capture_forward(tlr_plan* p, int g) {
   return rc;
 }
 
-// One forward pass on the plan's stream: the captured graph of the plan's precision (captured on
-// first use), or the launches themselves while per-kernel event timing is on or graphs are off.
+// One forward pass on the plan's stream: the captured graph of the plan's precision and kind of
+// rule (captured on first use), or the launches themselves while per-kernel event timing is on or graphs are off.
 int run_forward(tlr_plan* p) {
   if (!p->use_graphs || p->prof) return forward_sequence(p);
-  const int g = p->precision == TLR_PRECISION_MIXED ? 1 : 0;
+  const int g = (p->precision == TLR_PRECISION_MIXED ? 1 : 0) + (p->round_store ? 2 : 0);
   if (!p->fwd_exec[g]) TRY(capture_forward(p, g));
   TRY(cuda_check(cudaGraphLaunch(p->fwd_exec[g], p->stream), "forward graph launch"));
   for (int i = 0; i < TLR_NKINDS; ++i) p->klaunch[i] += p->fwd_launch[g][i];
@@ -745,9 +751,10 @@ int tlr_plan_create(tlr_plan** plan, int n, int b, int cap, int device, void* st
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   p->nsm = nsm;
-  p->nslots = nsm * tlr::rc_blocks_per_sm();  // resident recompression CTAs
-  p->slot_doubles = tlr::rc_slot_doubles(b, cap);
-  A(dalloc(p, &p->rcs, (size_t)p->nslots * p->slot_doubles));
+  p->nslots = nsm * tlr::rc_blocks_per_sm(b);  // resident recompression CTAs
+  p->nslots_general = nsm * tlr::rc_general_blocks_per_sm();
+  p->slot_doubles = std::max(tlr::rc_slot_doubles(b, cap), tlr::rc_general_slot_doubles(b, cap));
+  A(dalloc(p, &p->rcs, (size_t)std::max(p->nslots, p->nslots_general) * p->slot_doubles));
   A(dalloc(p, &p->rc_next, (size_t)p->nB));
   // rank map: the initial ranks, then the trailing pairs of every step
   p->rlog_off.assign((size_t)p->nB + 1, 0);
@@ -1412,7 +1419,7 @@ int tlr_dist_update_step(tlr_plan* p, int k) {
   }
   LAUNCH(TLR_K_RECOMPRESS, tlr::launch_recompress(p->n, p->b, k, p->nB, p->U, p->V, p->rank, p->cap, p->rcs,
                                                   p->slot_doubles, p->nslots, p->rc_next + k, p->rlog + p->rlog_off[k],
-                                                  p->blog + p->rlog_off[k], p->prank, p->pworld, p->status, s));
+                                                  p->prank, p->pworld, p->status, s));
   if (ahead) TRY(cuda_check(cudaStreamWaitEvent(s, p->ev_diag, 0), "wait"));
   return 0;
 }

@@ -9,7 +9,8 @@
 //   k_trsm(k)         V_ik <- L_kk^{-1} V_ik for i > k; W_ik = V_ik^T V_ik; Y_ik = U_ik W_ik;
 //                     rhs_i -= U_ik (V_ik^T z_k)
 //   k_recompress(k)   A_ij <- truncate([U_ij, -U_ik W], [V_ij, U_jk]) for k < j < i, W = V_ik^T V_jk,
-//                     skipped when r_ik = 0 or r_jk = 0 (17:189-194)
+//                     skipped when r_ik = 0 or r_jk = 0 (17:189-194): tlr_recompress.cu, and
+//                     k_recompress_general below under the storage rule 'mixed'
 // Layout in HBM: diagonal tiles column-major (ld b); off-diagonal factors U, V column-major
 // (ld b, cap columns per tile); tile (i, j), i > j, has index i (i - 1) / 2 + j.
 #include "tlr_device.cuh"
@@ -265,55 +266,38 @@ __global__ void __launch_bounds__(256) k_trsm(const double* TLR_RESTRICT D, int 
 }
 
 // ----------------------------------------------------------------------------------------
-// Recompression of the trailing tiles at step k.  Persistent grid; each CTA owns one slot of
-// global scratch (L2-resident working arrays).
-struct RcScratch {
-  double *W, *Cc, *Dd, *X, *Y, *Ru, *Rv, *M, *Vs, *G, *Hh, *Uo, *Vo;
+// Recompression under the storage rule 'mixed' (the other rules: tlr_recompress.cu).  Persistent grid;
+// each CTA owns one slot of global scratch (L2-resident working arrays).
+struct GenScratch {
+  double *W, *Ru, *Rv, *M, *Vs, *A, *B;
 };
 
-__device__ RcScratch rc_slot(double* base, int b, int cap) {
-  const size_t c2 = (size_t)cap * cap, s2 = (size_t)4 * cap * cap, bc = (size_t)b * cap;
-  RcScratch s;
-  double* p = base;
-  s.W = p; p += c2;
-  s.Cc = p; p += c2;
-  s.Dd = p; p += c2;
-  s.X = p; p += bc;
-  s.Y = p; p += bc;
-  s.Ru = p; p += s2;
-  s.Rv = p; p += s2;
-  s.M = p; p += s2;
-  s.Vs = p; p += s2;
-  s.G = p; p += 2 * c2;
-  s.Hh = p; p += c2;
-  s.Uo = p; p += bc;
-  s.Vo = p; p += bc;
-  return s;
-}
-
-size_t rc_slot_doubles(int b, int cap) {
+static __host__ __device__ inline size_t gen_slot(double* base, int b, int cap, GenScratch* out) {
   const size_t c2 = (size_t)cap * cap, bc = (size_t)b * cap;
-  return 3 * c2 + 2 * bc + 4 * 4 * c2 + 2 * c2 + c2 + 2 * bc;
+  size_t o = 0;
+  auto take = [&](size_t n) {
+    double* p = base + o;
+    o += n;
+    return p;
+  };
+  GenScratch s;
+  s.W = take(c2);
+  s.Ru = take(4 * c2);
+  s.Rv = take(4 * c2);
+  s.M = take(4 * c2);
+  s.Vs = take(4 * c2);
+  s.A = take(2 * bc);
+  s.B = take(2 * bc);
+  if (out) *out = s;
+  return (o + 1) & ~(size_t)1;
 }
 
-// C (p x q, ld p) = A^T B with A (m x p, lda), B (m x q, ldb): one warp per entry.
-__device__ void cta_atb(const double* A, int lda, const double* B, int ldb, int m, int p, int q, double* C,
-                        int ldc) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  for (int e = warp; e < p * q; e += nwarp) {
-    const int u = e % p, v = e / p;
-    const double* a = A + (size_t)u * lda;
-    const double* bb = B + (size_t)v * ldb;
-    double s = 0.0;
-    for (int t = lane; t < m; t += 32) s += a[t] * bb[t];
-    s = warp_sum(s);
-    if (lane == 0) C[(size_t)v * ldc + u] = s;
-  }
-}
+size_t rc_general_slot_doubles(int b, int cap) { return gen_slot(nullptr, b, cap, nullptr); }
 
-// One task of cta_atb4 (task e of p * ceil(q / 4): row u of C, four consecutive columns), by one warp.
+// C = A^T B (p x q, column v of C at C + v ldc), task e of p * ceil(q / 4) by one warp: row u of C, four
+// consecutive columns, so a column of A is read once for four dots.
 __device__ __forceinline__ void atb4_task(const double* A, int lda, const double* B, int ldb, int m, int p, int q,
-                                          double* C, int ldc, const double* scale, int e) {
+                                          double* C, int ldc, int e) {
   const int lane = threadIdx.x & 31;
   {
     const int u = e % p, v0 = (e / p) * 4;
@@ -335,24 +319,12 @@ __device__ __forceinline__ void atb4_task(const double* A, int lda, const double
     s2 = warp_sum(s2);
     s3 = warp_sum(s3);
     if (lane == 0) {
-      const double sc = scale ? scale[u] : 1.0;
-      C[(size_t)v0 * ldc + u] = scale ? s0 * sc : s0;
-      if (v0 + 1 < q) C[(size_t)(v0 + 1) * ldc + u] = scale ? s1 * sc : s1;
-      if (v0 + 2 < q) C[(size_t)(v0 + 2) * ldc + u] = scale ? s2 * sc : s2;
-      if (v0 + 3 < q) C[(size_t)(v0 + 3) * ldc + u] = scale ? s3 * sc : s3;
+      C[(size_t)v0 * ldc + u] = s0;
+      if (v0 + 1 < q) C[(size_t)(v0 + 1) * ldc + u] = s1;
+      if (v0 + 2 < q) C[(size_t)(v0 + 2) * ldc + u] = s2;
+      if (v0 + 3 < q) C[(size_t)(v0 + 3) * ldc + u] = s3;
     }
   }
-}
-
-// C[v][u] = (sum_t A[u][t] B[v][t]) (times scale[u] when scale is given) for u < p, v < q, column v
-// of C at C + v ldc.  One warp per (u, four consecutive v), so A's column is read once for four
-// dots; every entry is summed as in cta_atb (lane t = lane, lane + 32, ..., then the butterfly),
-// so the results are cta_atb's bit for bit.
-__device__ void cta_atb4(const double* A, int lda, const double* B, int ldb, int m, int p, int q, double* C,
-                         int ldc, const double* scale) {
-  const int warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  const int ntask = p * ((q + 3) >> 2);
-  for (int e = warp; e < ntask; e += nwarp) atb4_task(A, lda, B, ldb, m, p, q, C, ldc, scale, e);
 }
 
 // General recompression of one trailing pair, the reference's recompress as written
@@ -363,15 +335,15 @@ __device__ void cta_atb4(const double* A, int lda, const double* B, int ldb, int
 // pair overwrites the tile (i, j); with round_store it is then rounded under the budget left after
 // truncation (17:203-204).  Returns the new rank, or -1 after setting an error status.
 __device__ int rc_general_pair(int bi, int bj, int b, int cap, int r1, int ri, int rj, const double* Uik,
-                               const double* Ujk, const double* W, double* Uw, double* Vw, RcScratch& S,
+                               const double* Ujk, const double* W, double* Uw, double* Vw, GenScratch& S,
                                double* sig, int* perm, int* iflag, double* red, int* rsel, int rule_fixed,
                                double thr_rel, double thr_abs, int round_store, int* rlog_pp, int* blog_pp,
                                int rmode, int* status) {
   const int tid = threadIdx.x, nt = blockDim.x;
   const int s = r1 + rj, ls = 2 * cap;
   const int ku = min(bi, s), kv = min(bj, s);
-  double* A = S.X;   // b x 2 cap (X and Y are contiguous)
-  double* B = S.Uo;  // b x 2 cap (Uo and Vo are contiguous)
+  double* A = S.A;  // b x 2 cap
+  double* B = S.B;  // b x 2 cap
   for (int q = 0; q < r1; ++q) {
     for (int a = tid; a < bi; a += nt) A[(size_t)q * b + a] = Uw[(size_t)q * b + a];
     for (int a = tid; a < bj; a += nt) B[(size_t)q * b + a] = Vw[(size_t)q * b + a];
@@ -450,77 +422,36 @@ __device__ int rc_general_pair(int bi, int bj, int b, int cap, int r1, int ri, i
   return rn;
 }
 
-// The mixed path uses this kernel as it stands.  Three ways of making it cheaper there were measured
-// on the N = 50,000 bench workload and withdrawn: one Gram-Schmidt pass without re-orthogonalising
-// Q3 (5.53 against 5.09 evals/s, but 0.024 nats and 2e-3 of the gradient from FP64, over the
-// budget), a core Jacobi that stops at |cos| <= 1e-10 (no faster, 0.0079 nats, over budget on three
-// N = 20,000 sweep fields), 128-thread CTAs at 6 or 8 per SM (recompression 279 / 318 ms
-// against 175 ms per evaluation), and 256-thread CTAs at 5 or 6 per SM (48 / 40 registers, which
-// spill: 237 / 272 ms against 188 ms in the same run, batched mixed 4.30 / 4.05 against 4.83
-// evals/s).
-constexpr int kRcSmemS = 32;  // cores with s <= 32 are solved in shared memory
-#ifndef TLR_RC_THREADS
-#define TLR_RC_THREADS 256
-#endif
-constexpr int kRcT = TLR_RC_THREADS;  // threads per pair
-constexpr int kRcW = kRcT / 32;
-#ifndef TLR_RC_BLOCKS
-#define TLR_RC_BLOCKS 3
-#endif
-#ifndef TLR_RC_CHUNK
-#define TLR_RC_CHUNK 8
-#endif
-constexpr int kRcCW = TLR_RC_CHUNK;  // output columns per pass over a row in the row loops
-constexpr int kRcMinBlocks = TLR_RC_BLOCKS;  // resident CTAs per SM (the register cap follows)
+constexpr int kGcT = 256;       // threads per pair
+constexpr int kGcBlocks = 3;    // resident CTAs per SM
 
-int rc_blocks_per_sm() { return kRcMinBlocks; }
+int rc_general_blocks_per_sm() { return kGcBlocks; }
 
-// Trailing pairs held by the first m of a rank's rows ii0, ii0 + w, ... (row ii holds ii pairs).
-__host__ __device__ inline long rc_pairs_before(long m, long ii0, long w) { return m * ii0 + w * m * (m - 1) / 2; }
-
-__global__ void __launch_bounds__(kRcT, kRcMinBlocks) k_recompress(int n, int b, int k, int nB, double* TLR_RESTRICT U,
-                                                   double* TLR_RESTRICT V, int* TLR_RESTRICT rank, int cap,
-                                                   double* TLR_RESTRICT scratch, size_t slot_doubles,
-                                                   int* TLR_RESTRICT next_pair, int* TLR_RESTRICT rlog,
-                                                   int* TLR_RESTRICT blog, int prank, int pworld,
-                                                   int* TLR_RESTRICT status) {
+__global__ void __launch_bounds__(kGcT, kGcBlocks)
+    k_recompress_general(int n, int b, int k, int nB, double* TLR_RESTRICT U, double* TLR_RESTRICT V,
+                         int* TLR_RESTRICT rank, int cap, double* TLR_RESTRICT scratch, size_t slot_doubles,
+                         int* TLR_RESTRICT next_pair, int* TLR_RESTRICT rlog, int* TLR_RESTRICT blog,
+                         int* TLR_RESTRICT status) {
   if (*status != 0) return;
   const EvalParams& prm = *eval_params(status);
-  const int rule_fixed = prm.rule_fixed, rmode = prm.rmode, round_store = prm.round_store;
-  const int general = round_store;  // rounded factors are not orthogonal: the general recompression
+  const int rule_fixed = prm.rule_fixed, rmode = prm.rmode;
   const double thr_rel = prm.thr_rel, thr_abs = prm.thr_abs;
-  const int mB = nB - k - 1;  // trailing tiles
-  // the pairs (i, j), k < j < i, of this rank's trailing rows ii = ii0 + m pworld (i = k + 1 + ii,
-  // i % pworld == prank; every row when pworld = 1): row ii holds ii pairs, so rows 0..m-1 of the
-  // rank hold C(m) = m ii0 + pworld m (m - 1) / 2
-  const long ii0 = ((prank - (k + 1)) % pworld + pworld) % pworld;
-  const long mown = ii0 < mB ? (mB - 1 - ii0) / pworld + 1 : 0;
-  const long npairs = rc_pairs_before(mown, ii0, pworld);
-  RcScratch S = rc_slot(scratch + (size_t)blockIdx.x * slot_doubles, b, cap);
-  extern __shared__ double rc_smem[];
-  double* Msm = rc_smem;                            // kRcSmemS^2
-  double* Vsm = rc_smem + kRcSmemS * kRcSmemS;      // kRcSmemS^2
-  double* Zsm = rc_smem + 2 * kRcSmemS * kRcSmemS;  // kRcSmemS^2
+  const long mB = nB - k - 1, npairs = mB * (mB - 1) / 2;  // trailing tiles, their pairs (i, j), k < j < i
+  GenScratch S;
+  gen_slot(scratch + (size_t)blockIdx.x * slot_doubles, b, cap, &S);
   __shared__ double red[40];
-  __shared__ double n1[128];
-  __shared__ double ninv[128];
-  __shared__ double nvv[128];
-  __shared__ double nvinv[128];
   __shared__ double sig[256];
   __shared__ int perm[256];
   __shared__ int iflag[2];
-  __shared__ int rsel;
   __shared__ __align__(8) int gsel[4];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ls = 2 * cap;
+  const int tid = threadIdx.x, warp = tid >> 5;
   if (blockIdx.x == 0 && tid == 0) {  // the panel column k is read once per step
     double by = 0.0;
     for (int i = k + 1; i < nB; ++i) by += 8.0 * 2.0 * b * rank[tidx(i, k)];
     add_work(status, 10, 0.0, by);
   }
-  // pairs are handed out dynamically: each CTA starts on pair blockIdx.x and then takes the next
-  // unclaimed one (*next_pair counts the claims past the grid; zero at launch), so CTAs that drew
-  // low-rank pairs take more of them
+  // each CTA starts on pair blockIdx.x and then takes the next unclaimed one (*next_pair counts the
+  // claims past the grid; zero at launch)
   __shared__ long q_next;
   auto claim = [&]() -> long {
     __syncthreads();
@@ -528,308 +459,44 @@ __global__ void __launch_bounds__(kRcT, kRcMinBlocks) k_recompress(int n, int b,
     __syncthreads();
     return q_next;
   };
-  for (long qq = blockIdx.x; qq < npairs; qq = claim()) {
-    // decode qq -> (row m of the rank, jj), then pp = the pair's index among all trailing pairs
-    const double hb = (double)ii0 - 0.5 * pworld;
-    long m = (long)((-hb + sqrt(hb * hb + 2.0 * pworld * (double)qq)) / pworld);
-    while (m > 0 && rc_pairs_before(m, ii0, pworld) > qq) --m;
-    while (rc_pairs_before(m + 1, ii0, pworld) <= qq) ++m;
-    const int ii = (int)(ii0 + m * pworld);
-    const int jj = (int)(qq - rc_pairs_before(m, ii0, pworld));
-    const long pp = (long)ii * (ii - 1) / 2 + jj;
-    const int i = k + 1 + ii, j = k + 1 + jj;
+  for (long pp = blockIdx.x; pp < npairs; pp = claim()) {
+    long ii = (long)((1.0 + sqrt(1.0 + 8.0 * (double)pp)) * 0.5);
+    while (ii * (ii - 1) / 2 > pp) --ii;
+    while ((ii + 1) * ii / 2 <= pp) ++ii;
+    const int i = k + 1 + (int)ii, j = k + 1 + (int)(pp - ii * (ii - 1) / 2);
     const int tij = tidx(i, j), tik = tidx(i, k), tjk = tidx(j, k);
     const int r1 = rank[tij], ri = rank[tik], rj = rank[tjk];
     if (ri == 0 || rj == 0) continue;
     const int bi = min(b, n - i * b), bj = min(b, n - j * b), bk = min(b, n - k * b);
-    const double* Uij = U + (size_t)tij * b * cap;
-    const double* Vij = V + (size_t)tij * b * cap;
-    const double* Uik = U + (size_t)tik * b * cap;
     const double* Vik = V + (size_t)tik * b * cap;
-    const double* Ujk = U + (size_t)tjk * b * cap;
     const double* Vjk = V + (size_t)tjk * b * cap;
     const int s = r1 + rj;
-    const bool core_in_smem = s <= kRcSmemS;
-    double* Mc = core_in_smem ? Msm : S.M;
-    double* Vc = core_in_smem ? Vsm : S.Vs;
-    double* Zc = core_in_smem ? Zsm : S.Ru;  // R_u is no longer needed once M is formed
-    const int lc = core_in_smem ? kRcSmemS : ls;
     __syncthreads();
-    // W = V_ik^T V_jk (ri x rj); column norms of U_ij
-    // W's dot tasks and the column norms share one round-robin over the warps
-    const int nW = ri * ((rj + 3) >> 2);
-    for (int e = warp; e < nW + r1; e += kRcW) {
-      if (e < nW) {
-        atb4_task(Vik, b, Vjk, b, bk, ri, rj, S.W, cap, nullptr, e);
-        continue;
-      }
-      const int c = e - nW;
-      const double* u = Uij + (size_t)c * b;
-      const double* v = Vij + (size_t)c * b;
-      double a = 0.0, av = 0.0;
-      for (int t = lane; t < bi; t += 32) a += u[t] * u[t];
-      for (int t = lane; t < bj; t += 32) av += v[t] * v[t];
-      a = warp_sum(a);
-      av = warp_sum(av);
-      if (lane == 0) {
-        n1[c] = sqrt(a);
-        ninv[c] = a > 0.0 ? 1.0 / sqrt(a) : 0.0;
-        nvv[c] = sqrt(av);
-        nvinv[c] = av > 0.0 ? 1.0 / sqrt(av) : 0.0;
-      }
-    }
+    const int nW = ri * ((rj + 3) >> 2);  // W = V_ik^T V_jk (ri x rj)
+    for (int e = warp; e < nW; e += kGcT / 32) atb4_task(Vik, b, Vjk, b, bk, ri, rj, S.W, cap, e);
     __syncthreads();
-    if (general) {  // storage rule 'mixed': the reference's recompression as written
-      const int rn = rc_general_pair(bi, bj, b, cap, r1, ri, rj, Uik, Ujk, S.W, U + (size_t)tij * b * cap,
-                                     V + (size_t)tij * b * cap, S, sig, perm, iflag, red, gsel, rule_fixed,
-                                     thr_rel, thr_abs, round_store, rlog + pp, blog + pp, rmode, status);
-      if (rn < 0) return;
-      if (tid == 0) {
-        rank[tij] = rn;
-        add_work(status, 10, 4.0 * b * ri * rj + 16.0 * b * s * s + 4.0 * b * s * rn,
-                 8.0 * ((double)(bi + bj) * r1 + (double)(bi + bj) * rn));
-      }
-      __syncthreads();
-      continue;
-    }
-    // X = -U_ik W (bi x rj), kRcCW columns per pass over a row of U_ik
-    for (int a = tid; a < bi; a += kRcT)
-      for (int q0 = 0; q0 < rj; q0 += kRcCW) {
-        double acc[kRcCW] = {};
-        for (int p = 0; p < ri; ++p) {
-          const double x = Uik[(size_t)p * b + a];
-#pragma unroll
-          for (int w = 0; w < kRcCW; ++w) acc[w] = fma(x, S.W[(size_t)min(q0 + w, rj - 1) * cap + p], acc[w]);
-        }
-#pragma unroll
-        for (int w = 0; w < kRcCW; ++w)
-          if (q0 + w < rj) S.X[(size_t)(q0 + w) * b + a] = -acc[w];
-      }
-    __syncthreads();
-    // block Gram-Schmidt twice against Q1 = U_ij diag(1/n1): C = Q1^T X, X -= Q1 C
-    for (int pass = 0; pass < 2; ++pass) {
-      if (r1 > 0) {
-        cta_atb4(Uij, b, S.X, b, bi, r1, rj, S.G, cap, ninv);  // C increment
-        __syncthreads();
-        for (int a = tid; a < bi; a += kRcT)
-          for (int v0 = 0; v0 < rj; v0 += kRcCW) {
-            double acc[kRcCW] = {};
-            for (int u = 0; u < r1; ++u) {
-              const double x = Uij[(size_t)u * b + a] * ninv[u];
-#pragma unroll
-              for (int w = 0; w < kRcCW; ++w) acc[w] = fma(x, S.G[(size_t)min(v0 + w, rj - 1) * cap + u], acc[w]);
-            }
-#pragma unroll
-            for (int w = 0; w < kRcCW; ++w)
-              if (v0 + w < rj) S.X[(size_t)(v0 + w) * b + a] -= acc[w];
-          }
-        for (int e = tid; e < r1 * rj; e += kRcT) {
-          const int u = e % r1, v = e / r1;
-          const double inc = S.G[(size_t)v * cap + u];
-          S.Cc[(size_t)v * cap + u] = pass == 0 ? inc : S.Cc[(size_t)v * cap + u] + inc;
-        }
-      }
-      __syncthreads();
-    }
-    // R2 from Householder QR of the projected X (bi x rj); its reflectors are not needed
-    cta_geqr2_r(S.X, b, bi, rj, red);
-    // V side: D = V_ij^T U_jk, Y = U_jk - V_ij D (twice; the first pass reads U_jk itself)
-    if (r1 == 0) {
-      for (int v = 0; v < rj; ++v)
-        for (int a = tid; a < bj; a += kRcT) S.Y[(size_t)v * b + a] = Ujk[(size_t)v * b + a];
-      __syncthreads();
-    }
-    for (int pass = 0; pass < 2; ++pass) {
-      if (r1 > 0) {
-        const double* Yin = pass == 0 ? Ujk : S.Y;
-        cta_atb4(Vij, b, Yin, b, bj, r1, rj, S.G, cap, nvinv);
-        __syncthreads();
-        for (int a = tid; a < bj; a += kRcT)
-          for (int v0 = 0; v0 < rj; v0 += kRcCW) {
-            double acc[kRcCW] = {};
-            for (int u = 0; u < r1; ++u) {
-              const double x = Vij[(size_t)u * b + a] * nvinv[u];
-#pragma unroll
-              for (int w = 0; w < kRcCW; ++w) acc[w] = fma(x, S.G[(size_t)min(v0 + w, rj - 1) * cap + u], acc[w]);
-            }
-#pragma unroll
-            for (int w = 0; w < kRcCW; ++w)
-              if (v0 + w < rj) S.Y[(size_t)(v0 + w) * b + a] = Yin[(size_t)(v0 + w) * b + a] - acc[w];
-          }
-        for (int e = tid; e < r1 * rj; e += kRcT) {
-          const int u = e % r1, v = e / r1;
-          const double inc = S.G[(size_t)v * cap + u];
-          S.Dd[(size_t)v * cap + u] = pass == 0 ? inc : S.Dd[(size_t)v * cap + u] + inc;
-        }
-      }
-      __syncthreads();
-    }
-    // R_u = [[diag(n1), C], [0, R2]] (s x s, ld ls)
-    for (int e = tid; e < s * s; e += kRcT) {  // entry (a, c); every small loop below is flat too
-        const int a = e % s, c = e / s;
-        double vu = 0.0;
-        if (a < r1) vu = (c < r1) ? (a == c ? n1[a] : 0.0) : S.Cc[(size_t)(c - r1) * cap + a];
-        else if (c >= r1 && a <= c && a - r1 < bi) vu = S.X[(size_t)(c - r1) * b + (a - r1)];
-        S.Ru[(size_t)c * ls + a] = vu;
-      }
-    __syncthreads();
-    double* tau3 = sig + 128;
-    cta_geqr2(S.Y, b, bj, rj, tau3, red);
-    // R_v = [[I, D], [0, R3]]
-    for (int e = tid; e < s * s; e += kRcT) {
-        const int a = e % s, c = e / s;
-        double vv = 0.0;
-        if (a < r1) vv = (c < r1) ? (a == c ? nvv[a] : 0.0) : S.Dd[(size_t)(c - r1) * cap + a];
-        else if (c >= r1 && a <= c && a - r1 < bj) vv = S.Y[(size_t)(c - r1) * b + (a - r1)];
-        S.Rv[(size_t)c * ls + a] = vv;
-      }
-    __syncthreads();
-    cta_org2r(S.Y, b, bj, rj, tau3);
-    if (rj > bj) {  // a ragged tile shorter than the rank: the extra basis columns are zero
-      for (int v = bj; v < rj; ++v)
-        for (int a = tid; a < bj; a += kRcT) S.Y[(size_t)v * b + a] = 0.0;
-      __syncthreads();
-    }
-    // re-orthogonalise Q3 against the normalised V_ij once
-    if (r1 > 0) {
-      cta_atb4(Vij, b, S.Y, b, bj, r1, rj, S.G, cap, nullptr);
-      __syncthreads();
-      for (int a = tid; a < bj; a += kRcT)
-        for (int v0 = 0; v0 < rj; v0 += kRcCW) {
-          double acc[kRcCW] = {};
-          for (int u = 0; u < r1; ++u) {
-            const double x = Vij[(size_t)u * b + a] * nvinv[u];
-#pragma unroll
-            for (int w = 0; w < kRcCW; ++w)
-              acc[w] = fma(x, S.G[(size_t)min(v0 + w, rj - 1) * cap + u] * nvinv[u], acc[w]);
-          }
-#pragma unroll
-          for (int w = 0; w < kRcCW; ++w)
-            if (v0 + w < rj) S.Y[(size_t)(v0 + w) * b + a] -= acc[w];
-        }
-      __syncthreads();
-    }
-    // core M = R_u R_v^T (s x s); both factors are upper triangular
-    for (int e = tid; e < s * s; e += kRcT) {
-        const int a = e % s, c = e / s;
-        double acc = 0.0;
-        const int t0 = a > c ? a : c;
-        for (int t = t0; t < s; ++t) acc = fma(S.Ru[(size_t)t * ls + a], S.Rv[(size_t)t * ls + c], acc);
-        Mc[(size_t)c * lc + a] = acc;
-      }
-    __syncthreads();
-    // SVD of the core: Householder QR M = Q_M R_M, then one-sided Jacobi on R_M^T (R_M^T W = Z,
-    // orthogonal columns, sigma = column norms), so M = Q_M W Z^T and the right singular vectors
-    // are the normalised columns of Z.  The QR grades the columns, so the Jacobi needs 3-5 sweeps
-    // instead of 6-16 on M itself.
-    cta_geqr2_r(Mc, lc, s, s, red);
-    for (int e = tid; e < s * s; e += kRcT) {
-      const int a = e % s, c = e / s;
-      Zc[(size_t)c * lc + a] = (a >= c) ? Mc[(size_t)a * lc + c] : 0.0;
-    }
-    __syncthreads();
-    // columns below 1e-14 of the largest singular value (the projections' rounding noise) are not
-    // rotated: their relative orthogonality test would otherwise run to the sweep limit
-    cta_jacobi_svd(Zc, lc, s, s, nullptr, lc, sig, perm, iflag, 40, 1e-28);  // only Z is used
-    // Vc <- normalised Z (right singular vectors of M); the rotation matrix is not formed
-    for (int c = warp; c < s; c += kRcW) {
-      const double inv = sig[c] > 0.0 ? 1.0 / sig[c] : 0.0;
-      for (int a = lane; a < s; a += 32) Vc[(size_t)c * lc + a] = Zc[(size_t)c * lc + a] * inv;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      double srt[256];
-      double fro2 = 0.0;
-      for (int q = 0; q < s; ++q) srt[q] = sig[perm[q]];
-      for (int q = s - 1; q >= 0; --q) fro2 += srt[q] * srt[q];
-      const double thr = rule_fixed ? thr_rel * sqrt(fro2) : thr_abs;
-      int r = select_rank(srt, s, 0.0, thr, nullptr);
-      if (r < 0) r = s;
-      if (rmode == kRankReplay) r = min(rlog[pp], s);  // frozen: the rank recorded at another theta
-      else if (rmode == kRankRecord) rlog[pp] = r;
-      if (r > cap) {
-        atomicCAS(status, 0, -2);
-        r = -1;
-      }
-      rsel = r;
-    }
-    __syncthreads();
-    const int rn = rsel;
+    const int rn = rc_general_pair(bi, bj, b, cap, r1, ri, rj, U + (size_t)tik * b * cap, U + (size_t)tjk * b * cap, S.W,
+                                   U + (size_t)tij * b * cap, V + (size_t)tij * b * cap, S, sig, perm, iflag, red, gsel,
+                                   rule_fixed, thr_rel, thr_abs, 1, rlog + pp, blog + pp, rmode, status);
     if (rn < 0) return;
-    if (tid == 0)  // 4 b r_ik r_jk + 8 b s^2 + 4 b s r' flops; old and new pair read / written
-      add_work(status, 10, 4.0 * b * ri * rj + 8.0 * b * s * s + 4.0 * b * s * rn,
+    if (tid == 0) {
+      rank[tij] = rn;
+      add_work(status, 10, 4.0 * b * ri * rj + 16.0 * b * s * s + 4.0 * b * s * rn,
                8.0 * ((double)(bi + bj) * r1 + (double)(bi + bj) * rn));
-    // G = R_v^T Vs_r (s x rn), H = W G_bottom (ri x rn)
-    for (int e = tid; e < s * rn; e += kRcT) {
-        const int t = e % s, c = e / s;
-        const double* vc = Vc + (size_t)perm[c] * lc;
-        double acc = 0.0;
-        for (int a = 0; a <= t; ++a) acc = fma(S.Rv[(size_t)t * ls + a], vc[a], acc);
-        S.G[(size_t)c * ls + t] = acc;
-      }
-    __syncthreads();
-    for (int e = tid; e < ri * rn; e += kRcT) {
-      const int p = e % ri, c = e / ri;
-      double acc = 0.0;
-      for (int q = 0; q < rj; ++q) acc = fma(S.W[(size_t)q * cap + p], S.G[(size_t)c * ls + r1 + q], acc);
-      S.Hh[(size_t)c * cap + p] = acc;
     }
-    __syncthreads();
-    // U' = U_ij G_top - U_ik H ; V' = V_ij Vs_top + Q3 Vs_bottom, kRcCW columns per pass over a row.
-    // With rn <= kRcCW one pass makes a row's every output after reading all its inputs (each thread
-    // reads and writes its own rows only), so the new pair goes straight over the old one.
-    double* Uw = U + (size_t)tij * b * cap;
-    double* Vw = V + (size_t)tij * b * cap;
-    const bool direct = rn <= kRcCW;
-    double* Uout = direct ? Uw : S.Uo;
-    double* Vout = direct ? Vw : S.Vo;
-    for (int a = tid; a < bi; a += kRcT)
-      for (int c0 = 0; c0 < rn; c0 += kRcCW) {
-        double acc[kRcCW] = {};
-        for (int t = 0; t < r1; ++t) {
-          const double x = Uij[(size_t)t * b + a];
-#pragma unroll
-          for (int w = 0; w < kRcCW; ++w) acc[w] = fma(x, S.G[(size_t)min(c0 + w, rn - 1) * ls + t], acc[w]);
-        }
-        for (int p = 0; p < ri; ++p) {
-          const double x = -Uik[(size_t)p * b + a];
-#pragma unroll
-          for (int w = 0; w < kRcCW; ++w) acc[w] = fma(x, S.Hh[(size_t)min(c0 + w, rn - 1) * cap + p], acc[w]);
-        }
-#pragma unroll
-        for (int w = 0; w < kRcCW; ++w)
-          if (c0 + w < rn) Uout[(size_t)(c0 + w) * b + a] = acc[w];
-      }
-    for (int a = tid; a < bj; a += kRcT)
-      for (int c0 = 0; c0 < rn; c0 += kRcCW) {
-        int vo[kRcCW];  // offsets of the chunk's right singular vectors in Vc
-#pragma unroll
-        for (int w = 0; w < kRcCW; ++w) vo[w] = perm[min(c0 + w, rn - 1)] * lc;
-        double acc[kRcCW] = {};
-        for (int t = 0; t < r1; ++t) {
-          const double x = Vij[(size_t)t * b + a] * nvinv[t];
-#pragma unroll
-          for (int w = 0; w < kRcCW; ++w) acc[w] = fma(x, Vc[vo[w] + t], acc[w]);
-        }
-        for (int t = 0; t < rj; ++t) {
-          const double x = S.Y[(size_t)t * b + a];
-#pragma unroll
-          for (int w = 0; w < kRcCW; ++w) acc[w] = fma(x, Vc[vo[w] + r1 + t], acc[w]);
-        }
-#pragma unroll
-        for (int w = 0; w < kRcCW; ++w)
-          if (c0 + w < rn) Vout[(size_t)(c0 + w) * b + a] = acc[w];
-      }
-    if (!direct) {
-      __syncthreads();
-      for (int c = 0; c < rn; ++c) {
-        for (int a = tid; a < bi; a += kRcT) Uw[(size_t)c * b + a] = S.Uo[(size_t)c * b + a];
-        for (int a = tid; a < bj; a += kRcT) Vw[(size_t)c * b + a] = S.Vo[(size_t)c * b + a];
-      }
-    }
-    if (tid == 0) rank[tij] = rn;
     __syncthreads();
   }
+}
+
+int launch_recompress_general(int n, int b, int k, int nB, double* U, double* V, int* rank, int cap, double* scratch,
+                              size_t slot_doubles, int nslots, int* next_pair, int* rlog_step, int* blog_step,
+                              int* status, cudaStream_t s) {
+  const long mB = nB - k - 1, npairs = mB * (mB - 1) / 2;
+  if (npairs <= 0) return 0;
+  const int grid = (int)std::min<long>(npairs, nslots);
+  k_recompress_general<<<grid, kGcT, 0, s>>>(n, b, k, nB, U, V, rank, cap, scratch, slot_doubles, next_pair, rlog_step,
+                                             blog_step, status);
+  return (int)cudaGetLastError();
 }
 
 // ----------------------------------------------------------------------------------------
@@ -860,21 +527,6 @@ int launch_trsm(const double* D, int n, int b, int k, int nB, double* U, double*
   if (nB - k - 1 <= 0) return 0;
   k_trsm<<<nB - k - 1, 256, 0, s>>>(D, n, b, k, nB, U, V, Wd, Y, rank, cap, z, rhs, prec, blog_trsm, prank, pworld,
                                     status);
-  return (int)cudaGetLastError();
-}
-
-int launch_recompress(int n, int b, int k, int nB, double* U, double* V, int* rank, int cap, double* scratch,
-                      size_t slot_doubles, int nslots, int* next_pair, int* rlog_step, int* blog_step, int prank,
-                      int pworld, int* status, cudaStream_t s) {
-  const long mB = nB - k - 1;
-  const long ii0 = ((prank - (k + 1)) % pworld + pworld) % pworld;
-  const long npairs = rc_pairs_before(ii0 < mB ? (mB - 1 - ii0) / pworld + 1 : 0, ii0, pworld);
-  if (npairs <= 0) return 0;
-  const int grid = (int)std::min<long>(npairs, nslots);
-  const size_t sm = (size_t)3 * kRcSmemS * kRcSmemS * 8;
-  cudaFuncSetAttribute(k_recompress, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_recompress<<<grid, kRcT, sm, s>>>(n, b, k, nB, U, V, rank, cap, scratch, slot_doubles, next_pair, rlog_step,
-                                     blog_step, prank, pworld, status);
   return (int)cudaGetLastError();
 }
 

@@ -80,13 +80,18 @@ int launch_potrf_batched(double* D, int n, int b, int k, double* rhs, double* z,
 int launch_trsm(const double* D, int n, int b, int k, int nB, double* U, double* V, double* Wd, double* Y,
                 const int* rank, int cap, const double* z, double* rhs, int* prec, int* blog_trsm, int prank,
                 int pworld, const int* status, cudaStream_t s);
-size_t rc_slot_doubles(int b, int cap);
 // every trailing pair of step k; next_pair: a counter that is zero at launch (the CTAs claim
-// pairs past the grid through it)
-int rc_blocks_per_sm();  // k_recompress CTAs resident per SM
+// pairs past the grid through it).  The general form serves the storage rule 'mixed'.
+int rc_blocks_per_sm(int b);  // k_recompress CTAs resident per SM
+size_t rc_slot_doubles(int b, int cap);
 int launch_recompress(int n, int b, int k, int nB, double* U, double* V, int* rank, int cap, double* scratch,
-                      size_t slot_doubles, int nslots, int* next_pair, int* rlog_step, int* blog_step, int prank,
-                      int pworld, int* status, cudaStream_t s);
+                      size_t slot_doubles, int nslots, int* next_pair, int* rlog_step, int prank, int pworld,
+                      int* status, cudaStream_t s);
+int rc_general_blocks_per_sm();
+size_t rc_general_slot_doubles(int b, int cap);
+int launch_recompress_general(int n, int b, int k, int nB, double* U, double* V, int* rank, int cap, double* scratch,
+                              size_t slot_doubles, int nslots, int* next_pair, int* rlog_step, int* blog_step,
+                              int* status, cudaStream_t s);
 // assembled-matrix rule: dense Sigma^TLR from the initial compression (N x N, leading dimension ldk)
 int launch_assemble(const double* xy, int n, int b, double sigma2, double inv_range, int nu5, double nugget,
                     const double* U, const double* V, const int* rank, int cap, double* K, long long ldk,
