@@ -261,11 +261,15 @@ int run_factorization(tlr_plan* p) {
     const bool ahead = k + 1 < p->nB;
     if (ahead) {
       // A_{k+1,k+1} needs only the panels m <= k, all final once the panel solve of step k is
-      // done; step k's recompression touches tiles (i, j) with j > k + 1 only.
+      // done; step k's recompression touches tiles (i, j) with j > k + 1 only.  The recompression is a
+      // persistent grid that fills every SM, so the tile is built ahead of both: POTRF, on a stream of
+      // higher priority, then takes its SMs first and runs beside the recompression (with the build
+      // beside it too, POTRF found no SM until the recompression's last CTAs left: 235 against 203 ms
+      // for the forward pass at N = 50,000, b = 500)
+      LAUNCH(TLR_K_DIAG, tlr::launch_diag_build(p->xy, p->n, p->b, k + 1, p->U, p->Yd, p->rank, p->cap, p->D,
+                                                p->status, s));
       TRY(cuda_check(cudaEventRecord(p->ev_panel, s), "event"));
       TRY(cuda_check(cudaStreamWaitEvent(sd, p->ev_panel, 0), "wait"));
-      LAUNCH_ON(sd, TLR_K_DIAG, tlr::launch_diag_build(p->xy, p->n, p->b, k + 1, p->U, p->Yd, p->rank, p->cap,
-                                                       p->D, p->status, sd));
       LAUNCH_ON(sd, TLR_K_POTRF, tlr::launch_potrf(p->D, p->n, p->b, k + 1, p->rhs, p->z, p->ldpart, p->qpart,
                                                    p->status, sd));
       TRY(cuda_check(cudaEventRecord(p->ev_diag, sd), "event"));
@@ -771,7 +775,9 @@ int tlr_plan_create(tlr_plan** plan, int n, int b, int cap, int device, void* st
   A(dalloc(p, &p->fro0, nt));
   A(dalloc(p, &p->prec, nt));
   if (rc == 0) {
-    rc = cuda_check(cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking), "side stream");
+    int lo = 0, hi = 0;
+    cudaDeviceGetStreamPriorityRange(&lo, &hi);
+    rc = cuda_check(cudaStreamCreateWithPriority(&p->side, cudaStreamNonBlocking, hi), "side stream");
     if (!rc) rc = cuda_check(cudaEventCreateWithFlags(&p->ev_panel, cudaEventDisableTiming), "event");
     if (!rc) rc = cuda_check(cudaEventCreateWithFlags(&p->ev_diag, cudaEventDisableTiming), "event");
   }
@@ -1329,11 +1335,15 @@ int dist_ready(tlr_plan* p, int k) {
   return cuda_check(cudaSetDevice(p->device), "cudaSetDevice");
 }
 
-// Step k's diagonal tile on its owner: A_kk with the deferred updates, then POTRF and z_k.
-int dist_diag(tlr_plan* p, int k, cudaStream_t st) {
+// Step k's diagonal tile on its owner: A_kk with the deferred updates; then POTRF and z_k.
+int dist_build(tlr_plan* p, int k, cudaStream_t st) {
   if (k % p->pworld != p->prank) return 0;
   LAUNCH_ON(st, TLR_K_DIAG, tlr::launch_diag_build(p->xy, p->n, p->b, k, p->U, p->Yd, p->rank, p->cap, p->D,
                                                    p->status, st));
+  return 0;
+}
+int dist_potrf(tlr_plan* p, int k, cudaStream_t st) {
+  if (k % p->pworld != p->prank) return 0;
   LAUNCH_ON(st, TLR_K_POTRF, tlr::launch_potrf(p->D, p->n, p->b, k, p->rhs, p->z, p->ldpart, p->qpart, p->status,
                                                st));
   return 0;
@@ -1363,7 +1373,8 @@ int tlr_dist_begin(tlr_plan* p, const double theta[3], int rule, double value) {
   if (p->ntiles > 0)
     TRY(cuda_check(cudaMemcpyAsync(p->rank0, p->rank, sizeof(int) * p->ntiles, cudaMemcpyDeviceToDevice, s),
                    "rank0"));
-  return dist_diag(p, 0, s);
+  TRY(dist_build(p, 0, s));
+  return dist_potrf(p, 0, s);
 }
 
 int tlr_dist_pack_diag(tlr_plan* p, int k, double* buf) {
@@ -1411,10 +1422,11 @@ int tlr_dist_update_step(tlr_plan* p, int k) {
   TRY(dist_ready(p, k));
   cudaStream_t s = p->stream, sd = p->side;
   const bool ahead = k + 1 < p->nB && (k + 1) % p->pworld == p->prank;
-  if (ahead) {  // the next diagonal tile on the side stream, beside this step's recompression
+  if (ahead) {  // the next diagonal tile's POTRF on the side stream, beside this step's recompression
+    TRY(dist_build(p, k + 1, s));
     TRY(cuda_check(cudaEventRecord(p->ev_panel, s), "event"));
     TRY(cuda_check(cudaStreamWaitEvent(sd, p->ev_panel, 0), "wait"));
-    TRY(dist_diag(p, k + 1, sd));
+    TRY(dist_potrf(p, k + 1, sd));
     TRY(cuda_check(cudaEventRecord(p->ev_diag, sd), "event"));
   }
   LAUNCH(TLR_K_RECOMPRESS, tlr::launch_recompress(p->n, p->b, k, p->nB, p->U, p->V, p->rank, p->cap, p->rcs,
