@@ -74,9 +74,6 @@ int launch_diag_build(const double* xy, int n, int b, int k, const double* U, co
                       int cap, double* D, const int* status, cudaStream_t s);
 int launch_potrf(double* D, int n, int b, int k, double* rhs, double* z, double* ldpart, double* qpart,
                  int* status, cudaStream_t s);
-// nbatch tiles, tile q at D + q sD, rhs / z + q sV, ldpart / qpart / status + q sS
-int launch_potrf_batched(double* D, int n, int b, int k, double* rhs, double* z, double* ldpart, double* qpart,
-                         int* status, int nbatch, size_t sD, size_t sV, int sS, cudaStream_t s);
 int launch_trsm(const double* D, int n, int b, int k, int nB, double* U, double* V, double* Wd, double* Y,
                 const int* rank, int cap, const double* z, double* rhs, int* prec, int* blog_trsm, int prank,
                 int pworld, const int* status, cudaStream_t s);

@@ -3,21 +3,24 @@
 // Reference: codes/17_tlr_cholesky_pilot.py:171-177 (scipy.linalg.cholesky of A_kk; a pivot that
 // is not positive stops the factorization, failed_at = k) and 230-240 (z_k = L_kk^{-1} rhs_k).
 //
-// A cluster of kPC CTAs works on the column-major lower triangle of A_kk (L2-resident),
-// right-looking in panels of 32 columns, with the cluster's hardware barrier between phases:
-//   every CTA factors the 32 x 32 diagonal block redundantly (warp 0, the rows in registers;
-//   identical inputs give identical results, so a non-positive pivot stops every CTA at the same
-//   panel) and inverts it (lane c forms column c of L11^{-1});
-//   the panel rows below are split across the cluster, four threads per row: X = A21 L11^{-T} as
-//   independent dot products (no substitution chain), and rhs_rows -= X z_p with
-//   z_p = L11^{-1} rhs_p (the fused forward solve);
-//   cluster barrier; every CTA stages the whole panel X in shared memory once, and the
-//   lower-triangular 32 x 32 blocks of the trailing matrix are split across the cluster
-//   (A22 -= X X^T, no block barrier between blocks); cluster barrier.
-// Several tiles (one per parameter vector of a batch) are factored by independent clusters of
-// one launch.  The status word is read once by rank 0 and shared through distributed shared
-// memory, so every CTA of a cluster takes the same branch even when another stream writes the
-// status meanwhile.
+// A cluster of G CTAs works on the column-major lower triangle of A_kk (L2-resident),
+// right-looking in panels of 32 columns.  The tile is far too small to be bound by FP64 rate or bytes
+// (b = 500: 42 MFLOP, 2 MB): what counts is the chain through the 32 x 32 diagonal blocks, one
+// reciprocal square root, two multiply-adds and a shuffle per column (about 150 cycles), so everything
+// else is kept off it:
+//   * every CTA keeps the chain to itself: warp 1 solves the 32 rows below the diagonal block, warp 0
+//     updates the next diagonal block with them and factors it (redundantly: identical inputs give
+//     identical results, so no broadcast, and a non-positive pivot stops every CTA at the same panel);
+//   * the other rows are dealt out to the cluster and solved by substitution in registers, a thread
+//     per row, with the tile's right-hand side as one more row (z_p); then rhs_rows -= X z_p (the fused
+//     forward solve);
+//   * the trailing matrix advances in 32 x 16 pieces on the FP64 tensor cores, one piece per warp, while
+//     warp 0 factors; its fragments are read from L2 through L1 (a panel's lines enter L1 only after
+//     the panel is final, because every other access to the tile bypasses L1);
+//   * two cluster barriers per panel, split into arrive and wait: warp 0 runs past the first.
+// Measured (one tile alone): b = 100: 109 -> 35 us, b = 250: 300 -> 72 us, b = 500: 820 -> 162 us,
+// b = 1000: 8400 -> 610 us against the form that inverted each diagonal block and updated with
+// CUDA-core products from a staged panel.
 #include <cooperative_groups.h>
 
 #include "tlr_device.cuh"
@@ -27,37 +30,102 @@ namespace cg = cooperative_groups;
 
 namespace tlr {
 
-constexpr int kPB = 32;  // panel width
-constexpr int kPC = 8;   // CTAs per cluster (one cluster per tile)
+namespace {
 
-__global__ void __cluster_dims__(kPC, 1, 1) __launch_bounds__(256)
-    k_potrf_cluster(double* TLR_RESTRICT D, int n, int b, int k, double* TLR_RESTRICT rhs, double* TLR_RESTRICT z,
-                    double* TLR_RESTRICT ldpart, double* TLR_RESTRICT qpart, int* TLR_RESTRICT status,
-                    size_t sD, size_t sV, int sS, int staged) {
-  cg::cluster_group cluster = cg::this_cluster();
-  const int g = (int)cluster.block_rank(), G = kPC;
-  const int bz = blockIdx.x / kPC;  // which tile of the batch
-  D += bz * sD;
-  rhs += bz * sV;
-  z += bz * sV;
-  ldpart += bz * (size_t)sS;
-  qpart += bz * (size_t)sS;
-  status += bz * sS;
-  __shared__ double L11[kPB][kPB + 1];
-  __shared__ double Li[kPB][kPB + 1];  // L11^{-1}
-  __shared__ double dinv[kPB];
-  __shared__ double zp[kPB];
-  extern __shared__ double Ps[];  // the panel below the diagonal block, b x (kPB + 1), when staged
-  __shared__ double Pa[kPB][kPB + 1];
-  __shared__ double Pc[kPB][kPB + 1];
-  __shared__ int go, fail;
-  __shared__ double logdet_acc, quad_acc;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) {
-    go = (g == 0) ? (*status == 0) : 0;
-    logdet_acc = 0.0;
-    quad_acc = 0.0;
+constexpr int kPB = 32;        // panel width
+constexpr int kPL = kPB + 2;   // column pitch of a 32 x 32 block in shared memory (16-byte columns)
+
+// Substitution with L11 (columns of lc, pitch kPL; dinv = 1 / diagonal): a <- a L11^{-T} for one row
+// held in registers.  A column's entries are loaded while the column before is applied.
+__device__ __forceinline__ void solve_row(double (&a)[kPB], const double* lc, const double* dinv) {
+  double l[2][kPB], di[2];
+  auto fetch = [&](int c, double (&v)[kPB], double& d) {
+    d = dinv[c];
+#pragma unroll
+    for (int j = (c + 1) & ~1; j < kPB; j += 2) {
+      const double2 x = *reinterpret_cast<const double2*>(lc + c * kPL + j);
+      v[j] = x.x;
+      v[j + 1] = x.y;
+    }
+  };
+  fetch(0, l[0], di[0]);
+#pragma unroll
+  for (int c = 0; c < kPB; ++c) {
+    if (c + 1 < kPB) fetch(c + 1, l[(c + 1) & 1], di[(c + 1) & 1]);
+    a[c] *= di[c & 1];
+#pragma unroll
+    for (int j = c + 1; j < kPB; ++j) a[j] = fma(-a[c], l[c & 1][j], a[j]);
   }
+}
+
+// Cholesky of a 32 x 32 block by one warp, lane = row, the row in registers (the lower part; a block
+// narrower than 32 is padded with the identity).  Column c of L goes to lc + c kPL, the reciprocal of
+// its diagonal entry to dinv[c].  Returns 1 when a pivot is not positive.
+__device__ __forceinline__ int factor_block(double (&row)[kPB], double* lc, double* dinv) {
+  const int lane = threadIdx.x & 31;
+  int bad = 0;
+  double d = __shfl_sync(0xffffffffu, row[0], 0);
+#pragma unroll
+  for (int c = 0; c < kPB; ++c) {
+    bad |= !(d > 0.0);
+    const double rs = rsqrt(d);
+    const double l = row[c] * rs;  // at lane c: sqrt(d)
+    row[c] = l;
+    if (c + 1 < kPB) {
+      // the next pivot from its own lane, ahead of the other updates
+      d = __shfl_sync(0xffffffffu, fma(-l, l, row[c + 1]), c + 1);
+      row[c + 1] = fma(-l, __shfl_sync(0xffffffffu, l, c + 1), row[c + 1]);
+    }
+    lc[c * kPL + lane] = l;
+    if (lane == c) dinv[c] = rs;
+    __syncwarp();
+    if (c + 2 < kPB) {
+      if (c & 1) row[c + 2] = fma(-l, lc[c * kPL + c + 2], row[c + 2]);
+#pragma unroll
+      for (int j = (c + 3) & ~1; j < kPB; j += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(lc + c * kPL + j);
+        row[j] = fma(-l, v.x, row[j]);
+        row[j + 1] = fma(-l, v.y, row[j + 1]);
+      }
+    }
+  }
+  return bad;
+}
+
+// Fragments of all eight k steps (the 32 panel columns) for NR 8-row tiles from row r0 of the panel rows
+// P (column pitch ld, m rows below the diagonal block).
+template <int NR>
+__device__ __forceinline__ void panel_frag(double (&f)[8][NR], const double* P, int ld, int m, int r0) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk) {
+    const double* col = P + (size_t)(4 * kk + t) * ld;
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      const int r = r0 + 8 * i + g;
+      f[kk][i] = r < m ? col[r] : 0.0;
+    }
+  }
+}
+
+// G CTAs per tile, 8 warps each: 0 the diagonal chain, 1 the 32 rows below it, 2 to 6 the other rows, 7
+// the right-hand side; 1 to 7 the trailing pieces
+template <int G>
+__global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(256)
+    k_potrf_cluster(double* TLR_RESTRICT D, int n, int b, int k, double* TLR_RESTRICT rhs, double* TLR_RESTRICT z,
+                    double* TLR_RESTRICT ldpart, double* TLR_RESTRICT qpart, int* TLR_RESTRICT status) {
+  constexpr int NW = 8;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int g = (int)cluster.block_rank();
+  __shared__ __align__(16) double Lc[2][kPB * kPL];
+  __shared__ __align__(16) double Cs[kPB * kPL];  // the 32 solved rows, then the next diagonal block
+  __shared__ double dinv[2][kPB];
+  __shared__ double zp[kPB];
+  __shared__ int go, fail[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fg = lane >> 2, ft = lane & 3;
+  // the status word is read once by rank 0 and shared through distributed shared memory, so every CTA
+  // takes the same branch even when another stream writes the status meanwhile
+  if (tid == 0) go = (g == 0) ? (*status == 0) : 0;
   cluster.sync();
   const int ok = *cluster.map_shared_rank(&go, 0);
   cluster.sync();  // rank 0's shared memory stays valid until every CTA has read it
@@ -65,223 +133,197 @@ __global__ void __cluster_dims__(kPC, 1, 1) __launch_bounds__(256)
   const int bk = min(b, n - k * b);
   double* A = D + (size_t)k * b * b;
   double* rk = rhs + (size_t)k * b;
+  const bool al = (b & 1) == 0;
   if (g == 0 && tid == 0) add_work(status, 8, (double)bk * bk * bk / 3.0 + (double)bk * bk, 8.0 * bk * bk);
-  for (int p0 = 0; p0 < bk; p0 += kPB) {
-    const int pw = min(kPB, bk - p0);
-    const int m = bk - p0 - pw;
-    if (warp == 0) {
-      // Cholesky of the pw x pw diagonal block, lane = row, the row in registers
-      double row[kPB];
+  double row[kPB];  // warp 0: the current diagonal block; row warps: a row below it
+  double ldacc = 0.0, qacc = 0.0;
+  if (warp == 0) {
+    const int pw = min(kPB, bk);
 #pragma unroll
-      for (int j = 0; j < kPB; ++j)
-        row[j] = (lane < pw && j <= lane) ? A[(size_t)(p0 + j) * b + p0 + lane] : 0.0;
-      int bad = 0;
-      double dl = 0.0;  // 1 / L11[lane][lane]
-#pragma unroll
-      for (int c = 0; c < kPB; ++c) {
-        if (c < pw && !bad) {
-          const double d = __shfl_sync(0xffffffffu, row[c], c);
-          if (!(d > 0.0)) {
-            bad = 1;  // the same pivot in every lane: the whole warp stops here
-          } else {
-            // one reciprocal square root per pivot on the column chain (sqrt d = d / sqrt d);
-            // an IEEE square root followed by a division costs several times as long here
-            const double rsd = rsqrt(d), sd = d * rsd;
-            if (lane == c) {
-              row[c] = sd;
-              dl = rsd;
-            }
-            if (lane > c) row[c] *= rsd;
-#pragma unroll
-            for (int j = c + 1; j < kPB; ++j) {
-              const double ljc = __shfl_sync(0xffffffffu, row[c], j);
-              if (lane >= j) row[j] = fma(-row[c], ljc, row[j]);
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kPB; ++j) L11[lane][j] = (j <= lane && lane < pw && j < pw) ? row[j] : 0.0;
-      if (lane == 0) fail = bad;
-      __syncwarp();
-      dinv[lane] = (!bad && lane < pw) ? dl : 0.0;
-      __syncwarp();
-      if (!bad) {
-        // column `lane` of L11^{-1} by forward substitution
-        double x[kPB];
-#pragma unroll
-        for (int r = 0; r < kPB; ++r) {
-          double s = (r == lane) ? 1.0 : 0.0;
-#pragma unroll
-          for (int q = 0; q < r; ++q) s = fma(-L11[r][q], x[q], s);
-          x[r] = (r < pw) ? s * dinv[r] : 0.0;
-        }
-#pragma unroll
-        for (int r = 0; r < kPB; ++r) Li[r][lane] = x[r];
-        __syncwarp();
-        // z_p = L11^{-1} rhs_p (one load per lane, broadcast by shuffles), log det
-        const double rv = lane < pw ? rk[p0 + lane] : 0.0;
-        double v = 0.0;
-#pragma unroll
-        for (int q = 0; q < kPB; ++q) v = fma(Li[lane][q], __shfl_sync(0xffffffffu, rv, q), v);
-        zp[lane] = lane < pw ? v : 0.0;
-        if (g == 0) {
-          const double ld = warp_sum(lane < pw ? log(L11[lane][lane]) : 0.0);
-          if (lane == 0) logdet_acc += ld;
-        }
-      }
-    }
-    __syncthreads();
-    if (fail) {
+    for (int j = 0; j < kPB; ++j)
+      row[j] = (lane < pw && j <= lane) ? __ldcg(A + (size_t)j * b + lane) : (j == lane ? 1.0 : 0.0);
+    const int bad = factor_block(row, Lc[0], dinv[0]);
+    if (lane == 0) fail[0] = bad;
+  }
+  __syncthreads();
+  int cur = 0;
+  for (int p0 = 0; p0 < bk; p0 += kPB, cur ^= 1) {
+    if (fail[cur]) {
       if (g == 0 && tid == 0) atomicCAS(status, 0, k + 1);
       return;  // every CTA of the cluster leaves at the same panel
     }
-    // panel rows below, split across the cluster, four threads per row (eight outputs each)
-    {
-      const int per = (m + G - 1) / G;
-      const int r0 = g * per, r1 = min(m, r0 + per);
-      const int quarter = tid & 3;
-      for (int base = r0; base < r1; base += 64) {  // the same trip count in every thread (shuffles)
-        const int row = base + (tid >> 2);
-        const bool act = row < r1;
-        const size_t ar = (size_t)p0 + pw + (act ? row : 0);
-        double a[kPB];
+    const int pw = min(kPB, bk - p0), m = bk - p0 - pw;
+    double* P = A + (size_t)p0 * b + p0 + pw;         // the panel's rows below the diagonal block
+    double* T = A + (size_t)(p0 + pw) * b + p0 + pw;  // the trailing matrix
+    const double* lc = Lc[cur];
+    // ---- rows below: block 0 in every CTA, the others dealt out to the cluster; the right-hand side
+    const int nrb = (m + 31) / 32;
+    static_assert(5 * G + 1 >= (G == 4 ? 8 : 32), "a row warp takes at most one block of rows");
+    const bool rhs_warp = warp == NW - 1;
+    const int rb = warp == 1 ? 0 : 1 + g + G * (warp - 2), r = rb * 32 + lane;
+    const bool rows = warp > 0 && !rhs_warp && rb < nrb;
+    const bool act = rhs_warp ? lane == 0 : r < m;
+    if (rhs_warp || rows) {
 #pragma unroll
-        for (int q = 0; q < kPB; ++q) a[q] = (act && q < pw) ? A[(size_t)(p0 + q) * b + ar] : 0.0;
-        double xo[8];
-        double dz = 0.0;
+      for (int q = 0; q < kPB; ++q)
+        row[q] = (act && q < pw) ? __ldcg(rhs_warp ? rk + p0 + q : P + (size_t)q * b + r) : 0.0;
+      solve_row(row, lc, dinv[cur]);
+      if (rhs_warp) {
+        if (lane == 0) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int c = quarter * 8 + u;
-          double s = 0.0;
-#pragma unroll
-          for (int q = 0; q < kPB; ++q) s = fma(a[q], Li[c][q], s);
-          xo[u] = s;
-          dz = fma(s, zp[c], dz);
+          for (int q = 0; q < kPB; ++q) zp[q] = row[q];
         }
-        dz += __shfl_xor_sync(0xffffffffu, dz, 1);
-        dz += __shfl_xor_sync(0xffffffffu, dz, 2);
-        if (act) {
+      } else {
+        if (warp == 1) {
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int c = quarter * 8 + u;
-            if (c < pw) A[(size_t)(p0 + c) * b + ar] = xo[u];
+          for (int q = 0; q < kPB; ++q) Cs[q * kPL + lane] = row[q];
+        }
+        if (act && (warp > 1 || g == 0)) {
+#pragma unroll
+          for (int q = 0; q < kPB; ++q)
+            if (q < pw) __stcg(P + (size_t)q * b + r, row[q]);
+        }
+      }
+    } else if (warp == 0 && g == 0) {
+#pragma unroll
+      for (int j = 0; j < kPB; ++j)
+        if (lane < pw && j <= lane) __stcg(A + (size_t)(p0 + j) * b + p0 + lane, row[j]);
+      if (lane < pw) ldacc += log(lc[lane * kPL + lane]);
+    }
+    __syncthreads();
+    if (rows && r < m && (warp > 1 || g == 0)) {  // rhs -= X z_p
+      double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int q = 0; q < kPB; ++q) s[q & 3] = fma(row[q], zp[q], s[q & 3]);
+      __stcg(rk + p0 + pw + r, __ldcg(rk + p0 + pw + r) - ((s[0] + s[1]) + (s[2] + s[3])));
+    }
+    if (rhs_warp && lane == 0) {
+#pragma unroll
+      for (int q = 0; q < kPB; ++q) {
+        qacc = fma(row[q], row[q], qacc);
+        if (g == 0 && q < pw) z[(size_t)k * b + p0 + q] = row[q];
+      }
+    }
+    if (m == 0) break;
+    cluster.barrier_arrive();  // this CTA's part of the panel is final
+    if (warp == 0) {
+      // ---- the next diagonal block: C - X X^T on its lower 8 x 8 tiles, then its factor
+      const int pn = min(kPB, m);
+      double acc[4][4][2];  // tile (columns 8 nj, rows 8 mi): lane holds column fg, rows 2 ft, 2 ft + 1
+#pragma unroll
+      for (int nj = 0; nj < 4; ++nj)
+#pragma unroll
+        for (int mi = nj; mi < 4; ++mi)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int c = 8 * nj + fg, q = 8 * mi + 2 * ft + h;
+            acc[nj][mi][h] = (q < pn && c <= q) ? __ldcg(T + (size_t)c * b + q) : 0.0;
           }
-          if (quarter == 0) rk[ar] -= dz;
-        }
-      }
-    }
-    cluster.sync();
-    if (g == 0) {
-      for (int e = tid; e < pw * pw; e += blockDim.x) {
-        const int i = e % pw, j = e / pw;
-        if (i >= j) A[(size_t)(p0 + j) * b + p0 + i] = L11[i][j];
-      }
-      if (tid == 0) {
-        double q = quad_acc;
-        for (int c = 0; c < pw; ++c) {
-          z[(size_t)k * b + p0 + c] = zp[c];
-          q += zp[c] * zp[c];
-        }
-        quad_acc = q;
-      }
-    }
-    // trailing update of the lower triangle in 32 x 32 blocks.  staged: from the whole panel put in
-    // shared memory once (rows below the diagonal block, ld kPB + 1); otherwise (tiles too tall for
-    // that) each block's two 32 x 32 panel pieces are loaded from L2 in turn
-    if (staged) {
-      for (int e = tid; e < m * kPB; e += blockDim.x) {
-        const int row = e % m, t = e / m;
-        Ps[(size_t)row * (kPB + 1) + t] = t < pw ? A[(size_t)(p0 + t) * b + p0 + pw + row] : 0.0;
-      }
-      __syncthreads();
-    }
-    const int mb = (m + 31) / 32;
-    const int nblk = mb * (mb + 1) / 2;
-    for (int blk = g; blk < nblk; blk += G) {
-      if (!staged) {
-        int rb = (int)((sqrt(8.0 * blk + 1.0) - 1.0) * 0.5);
-        while (rb * (rb + 1) / 2 > blk) --rb;
-        while ((rb + 1) * (rb + 2) / 2 <= blk) ++rb;
-        const int cb = blk - rb * (rb + 1) / 2;
-        const int a0 = rb * 32, c0 = cb * 32;
-        __syncthreads();
-        for (int t = warp; t < kPB; t += 8) {
-          const double* col = A + (size_t)(p0 + t) * b + p0 + pw;
-          Pa[lane][t] = (t < pw && a0 + lane < m) ? col[a0 + lane] : 0.0;
-          Pc[lane][t] = (t < pw && c0 + lane < m) ? col[c0 + lane] : 0.0;
-        }
-        __syncthreads();
-        const int cl = tid & 31, rl = tid >> 5;  // column cl, rows rl + 8q
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 8
-        for (int t = 0; t < kPB; ++t) {
-          const double pc = Pc[cl][t];
+      double f[8][4];
+      panel_frag<4>(f, Cs, kPL, kPB, 0);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) acc[q] = fma(Pa[rl + 8 * q][t], pc, acc[q]);
-        }
-        const int cg2 = c0 + cl;
-        if (cg2 < m) {
-          double* colp = A + (size_t)(p0 + pw + cg2) * b + p0 + pw;
+      for (int kk = 0; kk < 8; ++kk)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int ag = a0 + rl + 8 * q;
-            if (ag < m && ag >= cg2) colp[ag] -= acc[q];
+        for (int nj = 0; nj < 4; ++nj) {
+          const double a = -f[kk][nj];
+#pragma unroll
+          for (int mi = nj; mi < 4; ++mi) dmma884(acc[nj][mi][0], acc[nj][mi][1], a, f[kk][mi]);
+        }
+      __syncwarp();
+#pragma unroll
+      for (int nj = 0; nj < 4; ++nj)
+#pragma unroll
+        for (int mi = nj; mi < 4; ++mi)
+          *reinterpret_cast<double2*>(Cs + (8 * nj + fg) * kPL + 8 * mi + 2 * ft) =
+              make_double2(acc[nj][mi][0], acc[nj][mi][1]);
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < kPB; ++j)
+        row[j] = (lane < pn && j <= lane) ? Cs[j * kPL + lane] : (j == lane ? 1.0 : 0.0);
+      __syncwarp();
+      const int bad = factor_block(row, Lc[cur ^ 1], dinv[cur ^ 1]);
+      if (lane == 0) fail[cur ^ 1] = bad;
+      cluster.barrier_wait();
+    } else {
+      // ---- the rest of the trailing lower triangle in pieces of 32 rows x 16 columns.  Warp 4, which
+      // shares warp 0's scheduler, takes pieces only where the update outweighs the diagonal chain
+      const bool helper = nrb > 12;
+      const int nwork = helper ? NW - 1 : NW - 2, wid = warp - 1 - (!helper && warp > 4 ? 1 : 0);
+      const int npiece = warp == 4 && !helper ? 0 : nrb * (nrb + 1);
+      bool waited = false;
+      for (int pc = 2 + g + G * wid; pc < npiece; pc += G * nwork) {
+        const int blk = pc >> 1;
+        int rbk = (int)((sqrtf(8.0f * blk + 1.0f) - 1.0f) * 0.5f);
+        while (rbk * (rbk + 1) / 2 > blk) --rbk;
+        while ((rbk + 1) * (rbk + 2) / 2 <= blk) ++rbk;
+        const int cb = blk - rbk * (rbk + 1) / 2;
+        const int r0 = rbk * 32, c0 = cb * 32 + (pc & 1) * 16;
+        double acc[2][4][2];
+#pragma unroll
+        for (int nj = 0; nj < 2; ++nj)
+#pragma unroll
+          for (int mi = 0; mi < 4; ++mi) {
+            const int c = c0 + 8 * nj + fg, q = r0 + 8 * mi + 2 * ft;
+            const double* cp = T + (size_t)c * b + q;
+            if (al && c < m && q + 1 < m) {
+              const double2 v = __ldcg(reinterpret_cast<const double2*>(cp));
+              acc[nj][mi][0] = v.x;
+              acc[nj][mi][1] = v.y;
+            } else {
+              acc[nj][mi][0] = c < m && q < m ? __ldcg(cp) : 0.0;
+              acc[nj][mi][1] = c < m && q + 1 < m ? __ldcg(cp + 1) : 0.0;
+            }
           }
-        }
-        continue;
-      }
-      int rb = (int)((sqrt(8.0 * blk + 1.0) - 1.0) * 0.5);
-      while (rb * (rb + 1) / 2 > blk) --rb;
-      while ((rb + 1) * (rb + 2) / 2 <= blk) ++rb;
-      const int cb = blk - rb * (rb + 1) / 2;
-      const int a0 = rb * 32, c0 = cb * 32;
-      const int cl = tid & 31, rl = tid >> 5;  // column cl, rows rl + 8q
-      const int cg2 = c0 + cl;
-      double* colp = A + (size_t)(p0 + pw + min(cg2, m - 1)) * b + p0 + pw;
-      double old[4];
+        if (!waited) cluster.barrier_wait();  // the panel is final
+        waited = true;
+        double fa[8][2], fb[8][4];
+        panel_frag<2>(fa, P, b, m, c0);
+        panel_frag<4>(fb, P, b, m, r0);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {  // the block's current values, loaded before the products
-        const int ag = a0 + rl + 8 * q;
-        old[q] = (cg2 < m && ag < m && ag >= cg2) ? colp[ag] : 0.0;
-      }
-      const double* pcr = Ps + (size_t)min(cg2, m - 1) * (kPB + 1);
-      double acc[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 8
-      for (int t = 0; t < kPB; ++t) {
-        const double pc = pcr[t];
+        for (int kk = 0; kk < 8; ++kk)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[q] = fma(Ps[(size_t)min(a0 + rl + 8 * q, m - 1) * (kPB + 1) + t], pc, acc[q]);
-      }
-      if (cg2 < m) {
+          for (int nj = 0; nj < 2; ++nj) {
+            const double a = -fa[kk][nj];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int ag = a0 + rl + 8 * q;
-          if (ag < m && ag >= cg2) colp[ag] = old[q] - acc[q];
-        }
+            for (int mi = 0; mi < 4; ++mi) dmma884(acc[nj][mi][0], acc[nj][mi][1], a, fb[kk][mi]);
+          }
+#pragma unroll
+        for (int nj = 0; nj < 2; ++nj)
+#pragma unroll
+          for (int mi = 0; mi < 4; ++mi) {
+            const int c = c0 + 8 * nj + fg, q = r0 + 8 * mi + 2 * ft;
+            double* cp = T + (size_t)c * b + q;
+            if (c >= m) continue;
+            if (al && q + 1 < m && q >= c)
+              __stcg(reinterpret_cast<double2*>(cp), make_double2(acc[nj][mi][0], acc[nj][mi][1]));
+            else {
+              if (q < m && q >= c) __stcg(cp, acc[nj][mi][0]);
+              if (q + 1 < m && q + 1 >= c) __stcg(cp + 1, acc[nj][mi][1]);
+            }
+          }
       }
+      if (!waited) cluster.barrier_wait();
     }
-    cluster.sync();
+    cluster.sync();  // the trailing matrix and the next diagonal block's factor are in place
   }
-  if (g == 0 && tid == 0) {
-    ldpart[k] = 2.0 * logdet_acc;
-    qpart[k] = quad_acc;
+  if (g == 0) {
+    if (warp == 0) {
+      ldacc = warp_sum(ldacc);
+      if (lane == 0) ldpart[k] = 2.0 * ldacc;
+    } else if (warp == NW - 1 && lane == 0) {
+      qpart[k] = qacc;
+    }
   }
 }
+
+}  // namespace
 
 int launch_potrf(double* D, int n, int b, int k, double* rhs, double* z, double* ldpart, double* qpart,
                  int* status, cudaStream_t s) {
-  return launch_potrf_batched(D, n, b, k, rhs, z, ldpart, qpart, status, 1, 0, 0, 0, s);
-}
-
-int launch_potrf_batched(double* D, int n, int b, int k, double* rhs, double* z, double* ldpart, double* qpart,
-                         int* status, int nbatch, size_t sD, size_t sV, int sS, cudaStream_t s) {
-  // the staged panel needs b (kPB + 1) doubles beside the 34 KB of static shared memory
-  const size_t sm_staged = (size_t)b * (kPB + 1) * sizeof(double);
-  const int staged = sm_staged <= 190 * 1024;
-  const size_t sm = staged ? sm_staged : 0;
-  cudaFuncSetAttribute(k_potrf_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_potrf_cluster<<<kPC * nbatch, 256, sm, s>>>(D, n, b, k, rhs, z, ldpart, qpart, status, sD, sV, sS, staged);
+  // four CTAs share the rows and the trailing pieces of the smaller tiles (one CTA takes 41 us at
+  // b = 100 against 35: its chain and its update meet on one SM), eight those past 256 rows
+  if (b <= 256) k_potrf_cluster<4><<<4, 256, 0, s>>>(D, n, b, k, rhs, z, ldpart, qpart, status);
+  else k_potrf_cluster<8><<<8, 256, 0, s>>>(D, n, b, k, rhs, z, ldpart, qpart, status);
   return (int)cudaGetLastError();
 }
 
