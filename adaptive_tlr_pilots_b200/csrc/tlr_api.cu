@@ -73,6 +73,7 @@ struct tlr_plan {
   cudaEvent_t ev_panel = nullptr, ev_diag = nullptr;
   // backward: the TLR solve for alpha runs on the side stream, one event per block row
   std::vector<cudaEvent_t> ev_alpha;
+  double* solve_work = nullptr;  // inverses of the 32 x 32 diagonal blocks, allocated at the first solve
   // results
   double *ldpart = nullptr, *qpart = nullptr, *out = nullptr;
   int* status = nullptr;
@@ -1482,8 +1483,9 @@ int tlr_factor_solve(tlr_plan* p, double* x_dev, int m, int trans) {
   if (!p->factor_ok) return fail(TLR_ERR_NOT_READY, "the plan holds no completed factorization");
   if (m == 0) return 0;
   TRY(cuda_check(cudaSetDevice(p->device), "cudaSetDevice"));
+  if (!p->solve_work) TRY(dalloc(p, &p->solve_work, tlr::solve_work_doubles(p->b, p->nB)));
   const int rc = tlr::launch_factor_solve(p->D, p->U, p->V, p->rank, p->cap, p->n, p->b, p->nB, x_dev, m, trans,
-                                          p->stream);
+                                          p->solve_work, p->stream);
   if (rc) return fail(TLR_ERR_CUDA, std::string("solve launch: ") + cudaGetErrorString((cudaError_t)rc));
   return cuda_check(cudaStreamSynchronize(p->stream), "solve");
 }

@@ -146,8 +146,10 @@ int launch_dtrace_step(const double* xy, int n, int b, int m, int nB, double sig
 int launch_grad_finish(const double* part, long nparts, double* grad, const int* status, cudaStream_t s);
 
 // solves and products with the factor (tlr_solve.cu); column-major n x m, ld n
+// work: solve_work_doubles(b, nB) doubles
+size_t solve_work_doubles(int b, int nB);
 int launch_factor_solve(const double* D, const double* U, const double* V, const int* rank, int cap, int n, int b,
-                        int nB, double* X, int m, int trans, cudaStream_t s);
+                        int nB, double* X, int m, int trans, double* work, cudaStream_t s);
 int launch_factor_matvec(const double* D, const double* U, const double* V, const int* rank, int cap, int n, int b,
                          int nB, const double* Z, double* Y, int m, cudaStream_t s);
 

@@ -6,6 +6,13 @@
 // Right-looking block order: after the diagonal block X_k is solved, its contribution leaves
 // every other block row at once (one CTA per block row and 32-column chunk), so a solve is 2 nB
 // launches whatever m.  Column-major N x m operands (ld = N), in place.
+//
+// A solve is one chain through the N rows, so its time is the chain's latency (the products are
+// m N b flops, microseconds).  The inverses of the 32 x 32 diagonal blocks of every L_kk come first, all
+// at once (k_diag_inv: 640 warps at N = 20,000); a panel step is then a 32 x 32 by 32 x 8 product and
+// an update of the other rows, both on the FP64 tensor cores with the operands that do not depend on X
+// loaded ahead of the barrier.  Kriging at N = 20,000, b = 500 with 300 sites (two solves of one
+// column, one of 300): 174 -> 10 ms against the substitution with one thread per column.
 #include "tlr_device.cuh"
 #include "tlr_kernels.h"
 
@@ -15,114 +22,222 @@ namespace {
 
 __device__ __forceinline__ int stidx(int i, int j) { return i * (i - 1) / 2 + j; }
 
-constexpr int kSC = 16;  // columns per CTA in the diagonal solves
+constexpr int kSC = 8;       // columns per CTA in the diagonal solves
+constexpr int kSW = 8;       // warps per CTA
+constexpr int kSPitch = 34;  // column pitch of a 32 x 32 block in shared memory
 
-// X_k <- L_kk^{-1} X_k (trans 0) or L_kk^{-T} X_k (trans 1), kSC columns per CTA staged in shared
-// memory, panels of 32 rows.
-__global__ void __launch_bounds__(256) k_tri_solve(const double* TLR_RESTRICT D, int n, int b, int k,
-                                                  double* TLR_RESTRICT X, int ldx, int m, int trans) {
-  const int bk = min(b, n - k * b);
+__device__ __forceinline__ double2 pair_at(const double* s, int row, int m, bool al) {
+  if (al && row + 1 < m) return *reinterpret_cast<const double2*>(s + row);
+  return make_double2(row < m ? s[row] : 0.0, row + 1 < m ? s[row + 1] : 0.0);
+}
+
+// inv (32 x 32, column-major, zero above the diagonal) = the inverse of diagonal block p of L_kk, padded
+// with the identity: one warp per block, lane j solves L x = e_j in registers.
+__global__ void __launch_bounds__(64) k_diag_inv(const double* TLR_RESTRICT D, int n, int b, int np,
+                                                double* TLR_RESTRICT inv, int total) {
+  __shared__ __align__(16) double lc[2][32 * kSPitch];
+  __shared__ double dinv[2][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int q = blockIdx.x * 2 + w;
+  if (q >= total) return;
+  const int k = q / np, p0 = (q - k * np) * 32;
+  const int pw = max(0, min(32, min(b, n - k * b) - p0));
+  const double* L = D + (size_t)k * b * b + (size_t)p0 * b + p0;
+#pragma unroll 8
+  for (int c = 0; c < 32; ++c) {
+    const double v = (lane < pw && c < pw && lane >= c) ? L[(size_t)c * b + lane] : (lane == c ? 1.0 : 0.0);
+    lc[w][c * kSPitch + lane] = v;
+    if (lane == c) dinv[w][c] = 1.0 / v;
+  }
+  __syncwarp();
+  double x[32];
+#pragma unroll
+  for (int r = 0; r < 32; ++r) x[r] = r == lane ? 1.0 : 0.0;
+#pragma unroll
+  for (int c = 0; c < 32; ++c) {
+    x[c] *= dinv[w][c];
+#pragma unroll
+    for (int j = c + 1; j < 32; ++j) x[j] = fma(-x[c], lc[w][c * kSPitch + j], x[j]);
+  }
+  double* o = inv + (size_t)q * 1024 + lane * 32;
+#pragma unroll
+  for (int r = 0; r < 32; r += 2) *reinterpret_cast<double2*>(o + r) = make_double2(x[r], x[r + 1]);
+}
+
+// X_k <- L_kk^{-1} X_k (TRANS false) or L_kk^{-T} X_k (true), kSC columns per CTA in shared memory, panels
+// of 32 rows: X_p <- inv_p X_p, then the other rows lose L[., p] X_p.  Tiles of the products have a column
+// of X as their row (lane (g, t) holds column g, rows 2t and 2t + 1).
+template <bool TRANS>
+__global__ void __launch_bounds__(kSW * 32) k_tri_solve(const double* TLR_RESTRICT D, const double* TLR_RESTRICT inv,
+                                                       int n, int b, int np, int k, double* TLR_RESTRICT X, int ldx,
+                                                       int m) {
+  const int bk = min(b, n - k * b), npk = (bk + 31) / 32;
   const int c0 = blockIdx.x * kSC, nc = min(kSC, m - c0);
   const double* L = D + (size_t)k * b * b;
-  extern __shared__ double xs[];  // bk x (kSC + 1)
-  __shared__ double L11[32][33];
-  __shared__ double dinv[32];
-  const int tid = threadIdx.x;
-  const int ld = kSC + 1;
-  for (int e = tid; e < bk * kSC; e += 256) {
-    const int r = e % bk, c = e / bk;
-    xs[(size_t)r * ld + c] = c < nc ? X[(size_t)(c0 + c) * ldx + (size_t)k * b + r] : 0.0;
+  inv += (size_t)k * np * 1024;
+  extern __shared__ __align__(16) double xs[];  // kSC columns, pitch ld: disjoint banks for the fragments
+  __shared__ __align__(16) double xp[kSC * 40];
+  const int ld = npk * 32 + 8;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  for (int e = tid; e < npk * 32 * kSC; e += kSW * 32) {
+    const int r = e % (npk * 32), c = e / (npk * 32);
+    xs[c * ld + r] = (c < nc && r < bk) ? X[(size_t)(c0 + c) * ldx + (size_t)k * b + r] : 0.0;
   }
   __syncthreads();
-  const int np = (bk + 31) / 32;
-  for (int pi = 0; pi < np; ++pi) {
-    const int p = trans ? np - 1 - pi : pi;
-    const int p0 = p * 32, pw = min(32, bk - p0);
-    for (int e = tid; e < 32 * 32; e += 256) {
-      const int a = e & 31, c = e >> 5;
-      L11[a][c] = (a < pw && c < pw && a >= c) ? L[(size_t)(p0 + c) * b + p0 + a] : 0.0;
+  for (int pi = 0; pi < npk; ++pi) {
+    const int p = TRANS ? npk - 1 - pi : pi, p0 = p * 32;
+    // row blocks of 8 that are still to be solved, the next panel's first
+    const int nrest = TRANS ? p * 4 : (npk - 1 - p) * 4;
+    auto row0 = [&](int q) { return TRANS ? p0 - 8 - 8 * q : p0 + 32 + 8 * q; };
+    // L[row r0 + g, p0 + 4 kk + t] (or its transpose), zero past the tile's last row
+    auto frag = [&](double (&f)[8], int q) {
+      const int r = row0(q) + g;
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) {
+        const int c = p0 + 4 * kk + t;
+        f[kk] = q < nrest && r < bk && c < bk ? (TRANS ? L[(size_t)r * b + c] : L[(size_t)c * b + r]) : 0.0;
+      }
+    };
+    double f0[8], f1[8];
+    frag(f0, warp);
+    frag(f1, warp + kSW);
+    if (warp < 4) {  // rows 8 warp .. of X_p
+      const double* ip = inv + (size_t)p * 1024;
+      double w[8], a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk)  // inv[row 8 warp + g][col 4 kk + t], or inv^T
+        w[kk] = TRANS ? ip[(8 * warp + g) * 32 + 4 * kk + t] : ip[(4 * kk + t) * 32 + 8 * warp + g];
+#pragma unroll
+      for (int kk = 0; kk < 8; kk += 2) {
+        dmma884(a0[0], a0[1], xs[g * ld + p0 + 4 * kk + t], w[kk]);
+        dmma884(a1[0], a1[1], xs[g * ld + p0 + 4 * kk + 4 + t], w[kk + 1]);
+      }
+      *reinterpret_cast<double2*>(xp + g * 40 + 8 * warp + 2 * t) = make_double2(a0[0] + a1[0], a0[1] + a1[1]);
     }
-    if (tid < 32) dinv[tid] = tid < pw ? 1.0 / L[(size_t)(p0 + tid) * b + p0 + tid] : 0.0;
-    if (trans) {
-      // x_p -= L[below, p]^T x_below, one thread per (panel row q, column c) pair
-      for (int e = tid; e < 32 * kSC; e += 256) {
-        const int q = e / kSC, c = e % kSC;
-        if (q < pw) {
-          const double* lc = L + (size_t)(p0 + q) * b;
-          double acc = 0.0;
-          for (int r = p0 + pw; r < bk; ++r) acc = fma(lc[r], xs[(size_t)r * ld + c], acc);
-          xs[(size_t)(p0 + q) * ld + c] -= acc;
+    __syncthreads();
+    if (tid < 128) {  // the solved panel back to xs (read again at the end only)
+      const int c = tid >> 4, r = 2 * (tid & 15);
+      *reinterpret_cast<double2*>(xs + c * ld + p0 + r) = *reinterpret_cast<const double2*>(xp + c * 40 + r);
+    }
+    double a[8];
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) a[kk] = -xp[g * 40 + 4 * kk + t];
+    for (int q = warp; q < nrest; q += 2 * kSW) {
+      double g0[8], g1[8];  // the pair after this one
+      frag(g0, q + 2 * kSW);
+      frag(g1, q + 3 * kSW);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (q + u * kSW < nrest) {
+          double2* xr = reinterpret_cast<double2*>(xs + g * ld + row0(q + u * kSW) + 2 * t);
+          double2 v = *xr;
+          double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+          for (int kk = 0; kk < 8; kk += 2) {
+            dmma884(v.x, v.y, a[kk], u ? f1[kk] : f0[kk]);
+            dmma884(s0, s1, a[kk + 1], u ? f1[kk + 1] : f0[kk + 1]);
+          }
+          *xr = make_double2(v.x + s0, v.y + s1);
         }
+      }
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) {
+        f0[kk] = g0[kk];
+        f1[kk] = g1[kk];
       }
     }
     __syncthreads();
-    if (tid < kSC) {  // the 32 x 32 diagonal block, one thread per column
-      const int c = tid;
-      if (!trans) {
-        for (int a = 0; a < pw; ++a) {
-          double s = xs[(size_t)(p0 + a) * ld + c];
-          for (int q = 0; q < a; ++q) s = fma(-L11[a][q], xs[(size_t)(p0 + q) * ld + c], s);
-          xs[(size_t)(p0 + a) * ld + c] = s * dinv[a];
-        }
-      } else {
-        for (int a = pw - 1; a >= 0; --a) {
-          double s = xs[(size_t)(p0 + a) * ld + c];
-          for (int q = a + 1; q < pw; ++q) s = fma(-L11[q][a], xs[(size_t)(p0 + q) * ld + c], s);
-          xs[(size_t)(p0 + a) * ld + c] = s * dinv[a];
-        }
-      }
-    }
-    __syncthreads();
-    if (!trans) {  // rows below the panel: x_below -= L[below, p] x_p
-      for (int e = tid; e < (bk - p0 - pw) * kSC; e += 256) {
-        const int r = p0 + pw + e / kSC, c = e % kSC;
-        double acc = 0.0;
-        for (int q = 0; q < pw; ++q) acc = fma(L[(size_t)(p0 + q) * b + r], xs[(size_t)(p0 + q) * ld + c], acc);
-        xs[(size_t)r * ld + c] -= acc;
-      }
-      __syncthreads();
-    }
   }
-  for (int e = tid; e < bk * nc; e += 256) {
-    const int r = e % bk, c = e / bk;
-    X[(size_t)(c0 + c) * ldx + (size_t)k * b + r] = xs[(size_t)r * ld + c];
+  for (int e = tid; e < npk * 32 * nc; e += kSW * 32) {
+    const int r = e % (npk * 32), c = e / (npk * 32);
+    if (r < bk) X[(size_t)(c0 + c) * ldx + (size_t)k * b + r] = xs[c * ld + r];
   }
 }
 
 // trans 0: X_i -= U_ik (V_ik^T X_k) for i > k;  trans 1: X_j -= V_kj (U_kj^T X_k) for j < k.
-// One CTA per (block row, 32-column chunk).
-__global__ void __launch_bounds__(256) k_solve_update(const double* TLR_RESTRICT U, const double* TLR_RESTRICT V,
-                                                     const int* TLR_RESTRICT rank, int cap, int n, int b, int k,
-                                                     double* TLR_RESTRICT X, int ldx, int m, int trans) {
+// One CTA per (block row, chunk of 8 NC columns): T = P^T X_k with the rows split over the warps in blocks
+// of 8, then X_o -= E T, both on the FP64 tensor cores.
+template <int NC>
+__global__ void __launch_bounds__(kSW * 32) k_solve_update(const double* TLR_RESTRICT U, const double* TLR_RESTRICT V,
+                                                          const int* TLR_RESTRICT rank, int cap, int n, int b, int k,
+                                                          double* TLR_RESTRICT X, int ldx, int m, int trans) {
   const int o = trans ? (int)blockIdx.x : k + 1 + (int)blockIdx.x;  // the block row updated
-  const int t = trans ? stidx(k, o) : stidx(o, k);
-  const int r = rank[t];
+  const int t0 = trans ? stidx(k, o) : stidx(o, k);
+  const int r = rank[t0];
   if (r == 0) return;
-  const int c0 = blockIdx.y * 32, nc = min(32, m - c0);
+  const int c0 = blockIdx.y * 8 * NC;
   const int bk = min(b, n - k * b), bo = min(b, n - o * b);
   // project with the factor on the k side, expand with the one on the other side
-  const double* P = (trans ? U : V) + (size_t)t * b * cap;
-  const double* E = (trans ? V : U) + (size_t)t * b * cap;
-  __shared__ double T[64][33];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int q0 = 0; q0 < r; q0 += 64) {
-    const int rq = min(64, r - q0);
-    __syncthreads();
-    for (int e = warp; e < rq * nc; e += 8) {
-      const int q = e % rq, c = e / rq;
-      const double* pc = P + (size_t)(q0 + q) * b;
-      const double* xc = X + (size_t)(c0 + c) * ldx + (size_t)k * b;
-      double acc = 0.0;
-      for (int a = lane; a < bk; a += 32) acc = fma(pc[a], xc[a], acc);
-      acc = warp_sum(acc);
-      if (lane == 0) T[q][c] = acc;
+  const double* P = (trans ? U : V) + (size_t)t0 * b * cap;
+  const double* E = (trans ? V : U) + (size_t)t0 * b * cap;
+  __shared__ double red[kSW / 2][NC * 64];
+  __shared__ double T[128][8 * NC + 1];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  // 16-byte row pairs of the factor and of X (whose base comes from the caller)
+  const bool alp = (b & 1) == 0, alx = alp && (ldx & 1) == 0 && (reinterpret_cast<size_t>(X) & 15) == 0;
+  const double* xk = X + (size_t)k * b;
+  for (int u0 = 0; u0 < r; u0 += 8) {
+    const double* pc = P + (size_t)min(u0 + g, r - 1) * b;
+    double acc[NC][2];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c][0] = acc[c][1] = 0.0;
+#pragma unroll 2
+    for (int row = 8 * warp; row < bk; row += 8 * kSW) {
+      const double2 a = pair_at(pc, row + 2 * t, bk, alp);
+      double2 x[NC];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) x[c] = pair_at(xk + (size_t)min(c0 + 8 * c + g, m - 1) * ldx, row + 2 * t, bk, alx);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        dmma884(acc[c][0], acc[c][1], a.x, x[c].x);
+        dmma884(acc[c][0], acc[c][1], a.y, x[c].y);
+      }
+    }
+    // the upper warps hand their parts to the lower ones, whose sums are added below
+    for (int half = 1; half >= 0; --half) {
+      if (warp / (kSW / 2) == half) {
+        double* rd = red[warp % (kSW / 2)] + g * 8 + 2 * t;
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) rd[c * 64 + h] = half ? acc[c][h] : acc[c][h] + rd[c * 64 + h];
+      }
+      __syncthreads();
+    }
+    for (int e = tid; e < NC * 64; e += kSW * 32) {
+      const int c = e >> 6, u = (e >> 3) & 7, v = e & 7;
+      double s = 0.0;
+#pragma unroll
+      for (int w = 0; w < kSW / 2; ++w) s += red[w][e];
+      if (u0 + u < r) T[u0 + u][8 * c + v] = s;
     }
     __syncthreads();
-    for (int e = tid; e < bo * nc; e += 256) {
-      const int a = e % bo, c = e / bo;
-      double acc = 0.0;
-      for (int q = 0; q < rq; ++q) acc = fma(E[(size_t)(q0 + q) * b + a], T[q][c], acc);
-      X[(size_t)(c0 + c) * ldx + (size_t)o * b + a] -= acc;
+  }
+  double* xo = X + (size_t)o * b;
+#pragma unroll 2
+  for (int row = 8 * warp; row < bo; row += 8 * kSW) {
+    double acc[NC][2];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const double2 v = pair_at(xo + (size_t)min(c0 + 8 * c + g, m - 1) * ldx, row + 2 * t, bo, alx);
+      acc[c][0] = v.x;
+      acc[c][1] = v.y;
+    }
+    for (int q0 = 0; q0 < r; q0 += 4) {
+      const int u = q0 + t;
+      const double e = (u < r && row + g < bo) ? E[(size_t)u * b + row + g] : 0.0;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) dmma884(acc[c][0], acc[c][1], u < r ? -T[u][8 * c + g] : 0.0, e);
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      if (c0 + 8 * c + g >= m) continue;
+      double* d = xo + (size_t)(c0 + 8 * c + g) * ldx + row + 2 * t;
+      if (alx && row + 2 * t + 1 < bo) *reinterpret_cast<double2*>(d) = make_double2(acc[c][0], acc[c][1]);
+      else {
+        if (row + 2 * t < bo) d[0] = acc[c][0];
+        if (row + 2 * t + 1 < bo) d[1] = acc[c][1];
+      }
     }
   }
 }
@@ -177,18 +292,22 @@ __global__ void __launch_bounds__(256) k_matvec_L(const double* TLR_RESTRICT D, 
 
 }  // namespace
 
+size_t solve_work_doubles(int b, int nB) { return (size_t)nB * ((b + 31) / 32) * 1024; }
+
 int launch_factor_solve(const double* D, const double* U, const double* V, const int* rank, int cap, int n, int b,
-                        int nB, double* X, int m, int trans, cudaStream_t s) {
-  const size_t sm = (size_t)b * (kSC + 1) * sizeof(double);
-  cudaFuncSetAttribute(k_tri_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  const dim3 gu(1, (m + 31) / 32);
+                        int nB, double* X, int m, int trans, double* work, cudaStream_t s) {
+  const int np = (b + 31) / 32, total = nB * np;
+  const size_t sm = (size_t)kSC * (np * 32 + 8) * sizeof(double);
+  const auto tri = trans ? k_tri_solve<true> : k_tri_solve<false>;
+  cudaFuncSetAttribute(tri, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_diag_inv<<<(total + 1) / 2, 64, 0, s>>>(D, n, b, np, work, total);
   for (int q = 0; q < nB; ++q) {
     const int k = trans ? nB - 1 - q : q;
-    k_tri_solve<<<(m + kSC - 1) / kSC, 256, sm, s>>>(D, n, b, k, X, n, m, trans);
+    tri<<<(m + kSC - 1) / kSC, kSW * 32, sm, s>>>(D, work, n, b, np, k, X, n, m);
     const int rows = trans ? k : nB - k - 1;
     if (rows > 0) {
-      const dim3 g(rows, gu.y);
-      k_solve_update<<<g, 256, 0, s>>>(U, V, rank, cap, n, b, k, X, n, m, trans);
+      if (m <= 8) k_solve_update<1><<<dim3(rows, 1), kSW * 32, 0, s>>>(U, V, rank, cap, n, b, k, X, n, m, trans);
+      else k_solve_update<4><<<dim3(rows, (m + 31) / 32), kSW * 32, 0, s>>>(U, V, rank, cap, n, b, k, X, n, m, trans);
     }
   }
   return (int)cudaGetLastError();
