@@ -740,7 +740,7 @@ int tlr_plan_create(tlr_plan** plan, int n, int b, int cap, int device, void* st
   A(dalloc(p, &p->ti, nt));
   A(dalloc(p, &p->tj, nt));
   // compression chunk: bounded so T + panels stay within ~4 GB
-  const size_t per_tile = (B * B + 4 * B * kMaxK + 2 * (size_t)kMaxK * kMaxK) * 8;
+  const size_t per_tile = (B * B + 3 * B * kMaxK + tlr::orth_slot_doubles(b, kMaxK) + 2 * (size_t)kMaxK * kMaxK) * 8;
   p->chunk = (int)std::max<size_t>(1, std::min<size_t>(nt, (size_t)4 * 1024 * 1024 * 1024 / per_tile));
   p->nblk = (b + 63) / 64;
   const size_t ch = (size_t)p->chunk;
@@ -749,7 +749,7 @@ int tlr_plan_create(tlr_plan** plan, int n, int b, int cap, int device, void* st
   A(dalloc(p, &p->P, ch * B * kMaxK));
   A(dalloc(p, &p->Z, ch * B * kMaxK));
   A(dalloc(p, &p->C, ch * B * kMaxK));
-  A(dalloc(p, &p->gscr, ch * B * kMaxK));
+  A(dalloc(p, &p->gscr, ch * tlr::orth_slot_doubles(b, kMaxK)));
   A(dalloc(p, &p->gsv, ch * 2 * (size_t)kMaxK * kMaxK));
   A(dalloc(p, &p->parts, ch * p->nblk));
   A(dalloc(p, &p->fparts, ch * p->nblk));

@@ -15,10 +15,14 @@
 //   the threshold; otherwise the tile is redone with k doubled (16, 32, 64, 128).
 // The truncated pair is U = C W_r (= Q_C U_w Sigma_r), V = P W_r, so U has orthogonal
 // columns and V orthonormal columns, exactly the structure of the reference's U*s, Vt^T.
-#include "tlr_device.cuh"
+#include <type_traits>
+
 #include "tlr_kernels.h"
+#include "tlr_panel.cuh"
 
 namespace tlr {
+
+constexpr int kMaxSketch = 128;  // widest sketch level
 
 __device__ __forceinline__ double omega_entry(uint32_t tile, uint32_t row, uint32_t col) {
   // splitmix64 (Steele, Lea, Flood 2014) on (tile, row, col): a fixed, reproducible test matrix
@@ -381,181 +385,119 @@ __global__ void __launch_bounds__(kSkW * 32, 1)
 }
 
 // ----------------------------------------------------------------------------------------
-// P <- Q of the Householder QR of Z (bj x k); the panel is staged in shared memory.
-__global__ void __launch_bounds__(1024) k_orth(double* TLR_RESTRICT Z, int n, int b, int k, int ldp,
-                                             int tile_base, const int* TLR_RESTRICT tj,
-                                             const int* TLR_RESTRICT need, double* TLR_RESTRICT gscratch,
-                                             int in_smem, const int* TLR_RESTRICT status) {
+// Blocked Householder QR of a bt x k panel by one CTA (a tlr::Side of GW warps): blocks of 8 columns go
+// through the earlier reflector blocks and their own QR in registers, products and updates on the FP64
+// tensor cores.  Bound by its chain of k column steps (about 800 cycles each, one barrier) and, for k > 8,
+// the block applications between them; per FP64 evaluation at N = 50,000, b = 500: k_orth 25.8 -> 11.9 ms,
+// k_finalize 15.9 -> 5.5 ms against a column-by-column QR with the core's SVD in shared memory; at
+// N = 1,030, b = 100: 0.54 -> 0.29 and 0.68 -> 0.16 ms.
+template <int GW, int NBLK>
+struct PanelShared {
+  static constexpr int kLdx = Side<GW, NBLK>::kLdx;
+  double red[kRu * GW * 64], redn[kRu * GW * 8];
+  double coef[64], tmp[64], zt[64], tau[16];
+  double qred[2 * (8 * GW + 8)];
+  double tf[16 * 64];  // T of every reflector block (k <= 128)
+};
+
+template <int GW, int NBLK>
+__device__ __forceinline__ Side<GW, NBLK> panel_side(int m, bool al) {
+  Side<GW, NBLK> sd;
+  sd.tg = threadIdx.x;
+  sd.gw = threadIdx.x >> 5;
+  sd.lane = threadIdx.x & 31;
+  sd.g = sd.lane >> 2;
+  sd.t = sd.lane & 3;
+  sd.bar = 1;
+  sd.m = m;
+  sd.al = al;
+  return sd;
+}
+
+// x <- (I - V T^T V^T) x (trans) or (I - V T V^T) x for one reflector block
+template <int GW, int NBLK>
+__device__ __forceinline__ void apply_block(const Side<GW, NBLK>& sd, double (&x)[NBLK][2], const double* panel,
+                                            const double* tf, bool trans, PanelShared<GW, NBLK>& sh) {
+  using S = Side<GW, NBLK>;
+  sd.dot(x, panel, S::kLdx, 8, S::kRows, true, sh.red, sh.redn,
+         [&](int u, int v, double sum, double) { sh.tmp[u * 8 + v] = sum; });
+  for (int e = sd.tg; e < 64; e += S::GT) {
+    const int u = e >> 3, v = e & 7;
+    double acc = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc = fma(trans ? tf[k * 8 + u] : tf[u * 8 + k], sh.tmp[k * 8 + v], acc);
+    sh.coef[e] = acc;
+  }
+  sd.sync();
+  sd.update(x, panel, S::kLdx, 8, S::kRows, sh.coef, 8, -1.0);
+}
+
+// QR of the panel src (leading dimension ld, ke columns): reflector blocks in panel (shared memory when
+// in_smem, block vb at panel + 8 vb kLdx) with their T factors in sh.tf; xs is the transpose buffer (one
+// block; the block itself when the panel is in shared memory).  R (row-major, pitch ldr, nrow rows) when
+// given.  The last block's reflectors are kept only when keep_last.
+template <int GW, int NBLK>
+__device__ __forceinline__ void panel_qr(const Side<GW, NBLK>& sd, const double* src, int ld, int ke, double* panel,
+                                         double* xs, bool in_smem, double* R, int ldr, int nrow, bool keep_last,
+                                         PanelShared<GW, NBLK>& sh) {
+  constexpr int kLdx = Side<GW, NBLK>::kLdx;
+  const int nb = (ke + 7) >> 3;
+#pragma unroll 1
+  for (int vb = 0; vb < nb; ++vb) {
+    const int nv = min(8, ke - 8 * vb);
+    double x[NBLK][2];
+    sd.load(x, src, ld, 8 * vb, nv);
+#pragma unroll 1
+    for (int pb = 0; pb < vb; ++pb) apply_block(sd, x, panel + (size_t)pb * 8 * kLdx, sh.tf + pb * 64, true, sh);
+    double* blk = panel + (size_t)vb * 8 * kLdx;
+    sd.qr(x, in_smem ? blk : xs, 8 * vb, nv, nrow, sh.qred, R + 8 * vb, ldr, sh.zt, sh.tau, sh.tf + vb * 64,
+          (keep_last || vb + 1 < nb) ? blk : nullptr);
+  }
+}
+
+// Z <- Q of the Householder QR of Z (bj x k).  One CTA per tile.
+template <int GW, int NBLK>
+__global__ void __launch_bounds__(GW * 32, 16 / GW) k_orth(double* TLR_RESTRICT Z, int n, int b, int k, int ldp,
+                                                          int tile_base, const int* TLR_RESTRICT tj,
+                                                          const int* TLR_RESTRICT need, double* TLR_RESTRICT gscratch,
+                                                          size_t slot, int in_smem, const int* TLR_RESTRICT status) {
   if (*status != 0) return;
   const int c = blockIdx.x;
   if (!need[c]) return;
+  constexpr int kLdx = Side<GW, NBLK>::kLdx;
   const int bj = min(b, n - tj[tile_at(status, tile_base + c)] * b);
   const int ke = min(k, bj);  // a tile narrower than k gets a full basis and zero columns
   if (threadIdx.x == 0) add_work(status, 3, 4.0 * bj * ke * ke, 16.0 * bj * k);
-  extern __shared__ double smem[];
-  double* red = smem;         // 33
-  double* tau = smem + 40;    // k
-  double* A = tau + 136;      // bj x k (ld bj) when it fits, else global scratch
-  const size_t pbase = (size_t)c * b * ldp;
-  double* W = in_smem ? A : gscratch + pbase;
-  for (int e = threadIdx.x; e < bj * ke; e += blockDim.x) {
-    const int row = e % bj, q = e / bj;
-    W[(size_t)q * bj + row] = Z[pbase + (size_t)q * b + row];
-  }
-  __syncthreads();
-  cta_geqr2(W, bj, bj, ke, tau, red);
-  cta_org2r(W, bj, bj, ke, tau);
-  for (int e = threadIdx.x; e < bj * k; e += blockDim.x) {
-    const int row = e % bj, q = e / bj;
-    Z[pbase + (size_t)q * b + row] = (q < ke) ? W[(size_t)q * bj + row] : 0.0;
-  }
-}
-
-// ----------------------------------------------------------------------------------------
-// The same orthonormalisation for k = 16 and 32 (8 or 16 warps) and tiles up to 512 rows with the
-// panel in registers: warp w holds columns 2w and 2w + 1, lane l rows l + 32 i (i < 16).  Per column c the owning
-// warp forms the reflector (LAPACK dlarfg convention, as cta_geqr2) and publishes it to shared
-// memory; every warp applies it to its own later columns (one warp reduction per column), so a
-// column costs two block barriers and no shared-memory traffic for the panel itself.  Q is formed
-// backwards from the reflectors kept in the owners' registers (dorg2r order, as cta_org2r).
-constexpr int kOrCpw = 2;   // columns per warp
-constexpr int kOrRpl = 16;  // rows per lane (tiles up to 512 rows)
-
-// One column of k_orth_reg's QR: the reflector of column cc, held by this warp as its column
-// `sel` (lane l rows l + 32 i), in the dlarfg convention; v (unit at cc) to vs, tau to taus[cc],
-// beta on the diagonal.  The column is picked by value (sel ? a[1] : a[0]) so that the register
-// panel is never indexed at run time.
-__device__ __forceinline__ void orth_reflector(double (&a)[kOrCpw][kOrRpl], int sel, int cc, int bj, double* vs,
-                                               double* taus) {
-  const int lane = threadIdx.x & 31;
-  double s2 = 0.0, xa = 0.0;
+  extern __shared__ __align__(16) double smem[];
+  auto& sh = *reinterpret_cast<PanelShared<GW, NBLK>*>(smem);
+  double* xs = smem + sizeof(PanelShared<GW, NBLK>) / sizeof(double);
+  double* panel = in_smem ? xs : gscratch + (size_t)c * slot;
+  double* Zc = Z + (size_t)c * b * ldp;
+  const auto sd = panel_side<GW, NBLK>(bj, (b & 1) == 0);
+  panel_qr(sd, Zc, b, ke, panel, xs, in_smem != 0, Zc, 0, 0, true, sh);
+  const int nb = (ke + 7) >> 3;
+#pragma unroll 1
+  for (int vb = (k >> 3) - 1; vb >= 0; --vb) {  // Q from the last block of columns on
+    double x[NBLK][2];
 #pragma unroll
-  for (int i = 0; i < kOrRpl; ++i) {
-    const int row = lane + 32 * i;
-    const double x = sel ? a[1][i] : a[0][i];
-    if (row > cc && row < bj) s2 = fma(x, x, s2);
-    if (i == cc / 32) xa = x;
-  }
-  const double sig2 = warp_sum(s2);
-  const double alpha = __shfl_sync(0xffffffffu, xa, cc % 32);
-  double beta, tc, scale;
-  if (sig2 == 0.0) { tc = 0.0; beta = alpha; scale = 1.0; }
-  else {
-    beta = -copysign(sqrt(alpha * alpha + sig2), alpha);
-    tc = (beta - alpha) / beta;
-    scale = 1.0 / (alpha - beta);
-  }
+    for (int p = 0; p < NBLK; ++p)
 #pragma unroll
-  for (int i = 0; i < kOrRpl; ++i) {
-    const int row = lane + 32 * i;
-    const double x = sel ? a[1][i] : a[0][i];
-    double v = 0.0, y = x;
-    if (row > cc && row < bj) {
-      y = tc != 0.0 ? x * scale : x;
-      v = y;
-    } else if (row == cc) {
-      v = 1.0;
-      y = beta;
-    }
-    if (sel) a[1][i] = y; else a[0][i] = y;
-    vs[row] = v;
-  }
-  if (lane == 0) taus[cc] = tc;
-}
-
-// The reflector of column cc (kept below its diagonal in column `sel`) back to vs for Q.
-__device__ __forceinline__ void orth_publish(const double (&a)[kOrCpw][kOrRpl], int sel, int cc, int bj, double* vs) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int i = 0; i < kOrRpl; ++i) {
-    const int row = lane + 32 * i;
-    const double x = sel ? a[1][i] : a[0][i];
-    vs[row] = (row > cc && row < bj) ? x : (row == cc ? 1.0 : 0.0);
-  }
-}
-
-template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) k_orth_reg(double* TLR_RESTRICT Z, int n, int b, int ldp,
-                                                                   int tile_base, const int* TLR_RESTRICT tj,
-                                                                   const int* TLR_RESTRICT need,
-                                                                   const int* TLR_RESTRICT status) {
-  if (*status != 0) return;
-  const int c = blockIdx.x;
-  if (!need[c]) return;
-  constexpr int k = WARPS * kOrCpw;
-  const int bj = min(b, n - tj[tile_at(status, tile_base + c)] * b);
-  const int ke = min(k, bj);  // a tile narrower than k gets a full basis and zero columns
-  if (threadIdx.x == 0) add_work(status, 3, 4.0 * bj * ke * ke, 16.0 * bj * k);
-  __shared__ double vs[32 * kOrRpl];  // the current reflector, zero above its pivot
-  __shared__ double taus[k];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const size_t pbase = (size_t)c * b * ldp;
-  double a[kOrCpw][kOrRpl];
-#pragma unroll
-  for (int j = 0; j < kOrCpw; ++j) {
-    const int col = warp * kOrCpw + j;
-#pragma unroll
-    for (int i = 0; i < kOrRpl; ++i) {
-      const int row = lane + 32 * i;
-      a[j][i] = (col < ke && row < bj) ? Z[pbase + (size_t)col * b + row] : 0.0;
-    }
-  }
-  // ---- QR: reflectors below the diagonal of their columns, R on and above it
-  for (int cc = 0; cc < ke; ++cc) {
-    if (warp == cc / kOrCpw) {
-      orth_reflector(a, cc % kOrCpw, cc, bj, vs, taus);
-    }
-    __syncthreads();
-    const double tc = taus[cc];
-#pragma unroll
-    for (int j = 0; j < kOrCpw; ++j) {
-      const int col = warp * kOrCpw + j;
-      if (col > cc && col < ke) {
-        double w = 0.0;
-#pragma unroll
-        for (int i = 0; i < kOrRpl; ++i) w = fma(vs[lane + 32 * i], a[j][i], w);
-        w = warp_sum(w) * tc;
-#pragma unroll
-        for (int i = 0; i < kOrRpl; ++i) a[j][i] = fma(-w, vs[lane + 32 * i], a[j][i]);
+      for (int h = 0; h < 2; ++h) {
+        const int row = 8 * (sd.gw + GW * p) + 2 * sd.t + h, col = 8 * vb + sd.g;
+        x[p][h] = (row == col && col < ke) ? 1.0 : 0.0;
       }
-    }
-    __syncthreads();  // vs is rewritten for the next column
-  }
-  // ---- Q = H_0 ... H_{ke-1} [I; 0], backwards
-  for (int cc = ke - 1; cc >= 0; --cc) {
-    const double tc = taus[cc];
-    if (warp == cc / kOrCpw) {
-      orth_publish(a, cc % kOrCpw, cc, bj, vs);
-    }
-    __syncthreads();
+#pragma unroll 1
+    for (int pb = min(vb, nb - 1); pb >= 0 && vb < nb; --pb)
+      apply_block(sd, x, panel + (size_t)pb * 8 * kLdx, sh.tf + pb * 64, false, sh);
+    double* z = Zc + (size_t)(8 * vb + sd.g) * b;
 #pragma unroll
-    for (int j = 0; j < kOrCpw; ++j) {
-      const int col = warp * kOrCpw + j;
-      if (col > cc && col < ke && tc != 0.0) {
-        double w = 0.0;
-#pragma unroll
-        for (int i = 0; i < kOrRpl; ++i) w = fma(vs[lane + 32 * i], a[j][i], w);
-        w = warp_sum(w) * tc;
-#pragma unroll
-        for (int i = 0; i < kOrRpl; ++i) a[j][i] = fma(-w, vs[lane + 32 * i], a[j][i]);
+    for (int p = 0; p < NBLK; ++p) {
+      const int row = 8 * (sd.gw + GW * p) + 2 * sd.t;
+      if (sd.al && row + 1 < bj) *reinterpret_cast<double2*>(z + row) = make_double2(x[p][0], x[p][1]);
+      else {
+        if (row < bj) z[row] = x[p][0];
+        if (row + 1 < bj) z[row + 1] = x[p][1];
       }
-      if (col == cc) {
-#pragma unroll
-        for (int i = 0; i < kOrRpl; ++i) {
-          const int row = lane + 32 * i;
-          a[j][i] = row < cc || row >= bj ? 0.0 : (row == cc ? 1.0 - tc : -tc * vs[row]);
-        }
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int j = 0; j < kOrCpw; ++j) {
-    const int col = warp * kOrCpw + j;
-#pragma unroll
-    for (int i = 0; i < kOrRpl; ++i) {
-      const int row = lane + 32 * i;
-      if (row < bj) Z[pbase + (size_t)col * b + row] = col < ke ? a[j][i] : 0.0;
     }
   }
 }
@@ -633,104 +575,154 @@ __global__ void __launch_bounds__(256) k_resid(const double* TLR_RESTRICT T, int
 }
 
 // ----------------------------------------------------------------------------------------
-// Rank decision and output of the truncated pair for every tile still in need.
-__global__ void __launch_bounds__(1024) k_finalize(int n, int b, int k, int ldp, int cap, int margin,
-                                                 int tile_base, const int* TLR_RESTRICT ti,
-                                                 const int* TLR_RESTRICT tj, int* TLR_RESTRICT need,
-                                                 const double* TLR_RESTRICT P, const double* TLR_RESTRICT C,
-                                                 const double* TLR_RESTRICT parts,
-                                                 const double* TLR_RESTRICT fparts, int nblk,
-                                                 double* TLR_RESTRICT gscratch, double* TLR_RESTRICT gsv,
-                                                 double* TLR_RESTRICT Uo,
-                                                 double* TLR_RESTRICT Vo, int* TLR_RESTRICT rank,
-                                                 int last_level, int w_in_smem, int* TLR_RESTRICT rlog,
-                                                 double* TLR_RESTRICT tail0, double* TLR_RESTRICT fro0,
-                                                 int* TLR_RESTRICT blog, int* TLR_RESTRICT status) {
+// Rank decision and output of the truncated pair for every tile still in need: R of the Householder QR
+// of C, one-sided Jacobi on the rows of R (right singular vectors and values of C), the rank rule with the
+// residual's rho^2, U = C W_r, V = P W_r.  One CTA per tile.
+template <int GW, int NBLK>
+__global__ void __launch_bounds__(GW * 32, 16 / GW)
+    k_finalize(int n, int b, int k, int ldp, int cap, int margin, int tile_base, const int* TLR_RESTRICT ti,
+               const int* TLR_RESTRICT tj, int* TLR_RESTRICT need, const double* TLR_RESTRICT P,
+               const double* TLR_RESTRICT C, const double* TLR_RESTRICT parts, const double* TLR_RESTRICT fparts,
+               int nblk, double* TLR_RESTRICT gscratch, size_t slot, double* TLR_RESTRICT gsv, double* TLR_RESTRICT Uo,
+               double* TLR_RESTRICT Vo, int* TLR_RESTRICT rank, int last_level, int in_smem, int* TLR_RESTRICT rlog,
+               double* TLR_RESTRICT tail0, double* TLR_RESTRICT fro0, int* TLR_RESTRICT blog, int* TLR_RESTRICT status) {
   if (*status != 0) return;
   const EvalParams& prm = *eval_params(status);
   const int rule_fixed = prm.rule_fixed, rmode = prm.rmode, round_store = prm.round_store;
   const double thr_rel = prm.thr_rel, thr_abs = prm.thr_abs;
   const int c = blockIdx.x;
   if (!need[c]) return;
+  constexpr int GT = GW * 32;
   const int t = tile_at(status, tile_base + c);
   const int bi = min(b, n - ti[t] * b), bj = min(b, n - tj[t] * b);
-  if (threadIdx.x == 0) add_work(status, 6, 4.0 * bi * k * k + 6.0 * 8.0 * k * k * k, 8.0 * (bi + bj) * k);
-  extern __shared__ double smem[];
-  double* red = smem;             // 33 (+pad)
-  double* tau = smem + 40;        // k
-  double* sig = tau + 136;        // k
-  int* perm = reinterpret_cast<int*>(sig + 136);  // k
-  int* iflag = perm + 136;
-  int* rsel = iflag + 2;
-  double* M = (k <= 64) ? smem + 40 + 136 * 3 + 8 : gsv + (size_t)c * 2 * k * k;  // k x k
-  double* Vw = M + k * k;                                                             // k x k
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) add_work(status, 6, 4.0 * bi * k * k + 6.0 * 8.0 * k * k * k, 8.0 * (bi + bj) * k);
+  __shared__ double red[40], nn[128], val[128], inv[128], srt[129];
+  __shared__ unsigned long long mx[2];
+  __shared__ int perm[128], flag[2], rsel;
+  extern __shared__ __align__(16) double smem[];
+  auto& sh = *reinterpret_cast<PanelShared<GW, NBLK>*>(smem);
+  const int ldm = k + 1;
+  double* M = smem + sizeof(PanelShared<GW, NBLK>) / sizeof(double);  // k x (k + 1)
+  double* xs = M + ((k * ldm + 1) & ~1);
+  double* panel = in_smem ? xs : gscratch + (size_t)c * slot;
   const size_t pbase = (size_t)c * b * ldp;
-  // bi x k copy of C for the QR: in shared memory (ld bi) when it fits, else global scratch (ld b)
-  double* W = w_in_smem ? smem + 40 + 136 * 3 + 8 + 2 * (size_t)k * k : gscratch + pbase;
-  const int ldw = w_in_smem ? bi : b;
-  for (int e = threadIdx.x; e < bi * k; e += blockDim.x) {
-    const int row = e % bi, q = e / bi;
-    W[(size_t)q * ldw + row] = C[pbase + (size_t)q * b + row];
-  }
-  __syncthreads();
-  const int kk = min(k, bi);
-  cta_geqr2(W, ldw, bi, k, tau, red);
-  cta_copy_r(W, ldw, bi, k, M, k);
-  cta_jacobi_svd(M, k, k, k, Vw, k, sig, perm, iflag);
-  if (threadIdx.x == 0) {
-    double rho2 = 0.0, fro2 = 0.0;
-    for (int q = 0; q < nblk; ++q) { rho2 += parts[c * nblk + q]; fro2 += fparts[c * nblk + q]; }
-    double sorted[128];
-    for (int q = 0; q < k; ++q) sorted[q] = sig[perm[q]];
-    const double thr = rule_fixed ? thr_rel * sqrt(fro2) : thr_abs;
-    int r = select_rank(sorted, k, rho2, thr, nullptr);
-    if (rmode == kRankReplay) r = rlog[t];  // frozen: the rank recorded at another theta
-    const bool exact = (k >= bj) || (k >= bi);
-    int out;
-    if (r >= 0 && (r <= k - margin || exact)) out = r;
-    else if (last_level) out = -2;  // compression limit reached
-    else out = -1;                  // redo with a larger k
-    if (out >= 0 && out > cap) out = -3;
-    if (out >= 0) {  // truncation error ||T - T_r||_F and ||T||_F of the accepted tile
-      double acc = rho2;
-      for (int q = out; q < k; ++q) acc += sorted[q] * sorted[q];
-      tail0[t] = sqrt(acc);
-      fro0[t] = sqrt(fro2);
+  auto sd = panel_side<GW, NBLK>(bi, (b & 1) == 0);
+  // every column runs, past the tile's rows too (zero rows and no reflector there)
+  panel_qr(sd, C + pbase, b, k, panel, xs, in_smem != 0, M, ldm, k, false, sh);
+  sd.sync();
+  if (k <= 32) {
+    if (warp == 0) {
+      if (k <= 16) jacobi_warp<4, 4>(M, ldm, k);
+      else jacobi_warp<2, 16>(M, ldm, k);
     }
-    *rsel = out;
+  } else {
+    jacobi_group<GT>(M, ldm, k, nn, mx, flag, tid, 1);
   }
-  __syncthreads();
-  const int r = *rsel;
-  (void)kk;
+  sd.sync();
+  for (int q0 = 0; q0 < k; q0 += GT / 4) {  // singular values: the row norms
+    const int q = q0 + (tid >> 2), h = tid & 3;
+    double a0 = 0.0, a1 = 0.0;
+    if (q < k)
+      for (int e = h; e < k; e += 8) {
+        a0 = fma(M[q * ldm + e], M[q * ldm + e], a0);
+        if (e + 4 < k) a1 = fma(M[q * ldm + e + 4], M[q * ldm + e + 4], a1);
+      }
+    double a = a0 + a1;
+    a += __shfl_xor_sync(0xffffffffu, a, 2);
+    a += __shfl_xor_sync(0xffffffffu, a, 1);
+    if (q < k && h == 0) {
+      const double nr = sqrt(a);
+      val[q] = nr;
+      inv[q] = nr > 0.0 ? 1.0 / nr : 0.0;
+      perm[q] = q;
+    }
+  }
+  sd.sync();
+  for (int q = tid; q < k; q += GT) {  // descending order, ties by index
+    const double vq = val[q];
+    int pos = 0;
+#pragma unroll 4
+    for (int d = 0; d < k; ++d) {
+      const double v = val[d];
+      pos += (v > vq) || (v == vq && d < q);
+    }
+    perm[pos] = q;
+    srt[pos] = vq * vq;
+  }
+  sd.sync();
+  if (tid == 0) {
+    double rho2 = 0.0, fro2 = 0.0;
+    for (int q = 0; q < nblk; ++q) {
+      rho2 += parts[c * nblk + q];
+      fro2 += fparts[c * nblk + q];
+    }
+    double acc = rho2;  // srt[q] <- rho^2 + sum_{u >= q} sigma_u^2, from the smallest up (17:113)
+    srt[k] = acc;
+    for (int q = k - 1; q >= 0; --q) {
+      acc += srt[q];
+      srt[q] = acc;
+    }
+    red[0] = rho2;
+    red[1] = fro2;
+  }
+  sd.sync();
+  if (warp == 0) {
+    const double fro2 = red[1], thr = rule_fixed ? thr_rel * sqrt(fro2) : thr_abs;
+    int r = -1;
+    for (int q0 = 0; q0 <= k && r < 0; q0 += 32) {
+      const unsigned hit = __ballot_sync(0xffffffffu, q0 + lane <= k && sqrt(srt[min(q0 + lane, k)]) <= thr);
+      if (hit) r = q0 + __ffs(hit) - 1;
+    }
+    if (lane == 0) {
+      if (rmode == kRankReplay) r = rlog[t];  // frozen: the rank recorded at another theta
+      const bool exact = (k >= bj) || (k >= bi);
+      int out;
+      if (r >= 0 && (r <= k - margin || exact)) out = r;
+      else if (last_level) out = -2;  // compression limit reached
+      else out = -1;                  // redo with a larger k
+      if (out >= 0 && out > cap) out = -3;
+      if (out >= 0) {  // truncation error ||T - T_r||_F and ||T||_F of the accepted tile
+        tail0[t] = sqrt(srt[min(out, k)]);
+        fro0[t] = sqrt(fro2);
+      }
+      rsel = out;
+    }
+  }
+  sd.sync();
+  const int r = rsel;
   if (r == -1) return;
   if (r < 0) {
-    if (threadIdx.x == 0) atomicCAS(status, 0, r == -2 ? -5 : -2);
+    if (tid == 0) atomicCAS(status, 0, r == -2 ? -5 : -2);
     return;
   }
-  // U = C W_r, V = P W_r (columns in descending singular-value order)
+  // U = C W_r, V = P W_r: column q of W is row perm[q] of M over its norm
   double* Ut = Uo + (size_t)t * b * cap;
   double* Vt = Vo + (size_t)t * b * cap;
-  for (int e = threadIdx.x; e < bi * r; e += blockDim.x) {
-    const int row = e % bi, q = e / bi;
-    const double* w = Vw + (size_t)perm[q] * k;
-    double s = 0.0;
-    for (int u = 0; u < k; ++u) s = fma(C[pbase + (size_t)u * b + row], w[u], s);
-    Ut[(size_t)q * b + row] = s;
-  }
-  for (int e = threadIdx.x; e < bj * r; e += blockDim.x) {
-    const int row = e % bj, q = e / bj;
-    const double* w = Vw + (size_t)perm[q] * k;
-    double s = 0.0;
-    for (int u = 0; u < k; ++u) s = fma(P[pbase + (size_t)u * b + row], w[u], s);
-    Vt[(size_t)q * b + row] = s;
+  if (r > 0) {
+    double* cf = k <= 32 ? xs : gsv + (size_t)c * 2 * k * k;  // the reflector panel is done
+    const int ldc = k;
+    for (int e = tid; e < k * r; e += GT) {
+      const int q = e / k, u = e - q * k;
+      cf[u * ldc + q] = M[perm[q] * ldm + u] * inv[perm[q]];
+    }
+    sd.sync();
+    for (int s = 0; s < 2; ++s) {
+      sd.m = s ? bj : bi;
+      const double* src = (s ? P : C) + pbase;
+      double* out = s ? Vt : Ut;
+      if (r <= 8) sd.template output<1>(out, b, r, src, 0, cf, src, b, k, sd.m, cf, ldc);
+      else if (r <= 16) sd.template output<2>(out, b, r, src, 0, cf, src, b, k, sd.m, cf, ldc);
+      else if (r <= 32) sd.template output<4>(out, b, r, src, 0, cf, src, b, k, sd.m, cf, ldc);
+      else sd.template output<16>(out, b, r, src, 0, cf, src, b, k, sd.m, cf, ldc);
+    }
   }
   if (round_store) {  // storage rule 'mixed': rounded under the budget left after truncation (17:163-164)
     __syncthreads();
-    const int bits = cta_round_pair(Ut, Vt, bi, bj, r, b, thr_abs - tail0[t], red,
-                                    rmode == kRankReplay ? blog[t] : 0);
-    if (threadIdx.x == 0 && rmode == kRankRecord) blog[t] = bits;
+    const int bits = cta_round_pair(Ut, Vt, bi, bj, r, b, thr_abs - tail0[t], red, rmode == kRankReplay ? blog[t] : 0);
+    if (tid == 0 && rmode == kRankRecord) blog[t] = bits;
   }
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     rank[t] = r;
     need[c] = 0;
     if (rmode == kRankRecord) rlog[t] = r;
@@ -788,24 +780,42 @@ int launch_project_resid(const double* T, int n, int b, int tile_base, const int
   return (int)cudaGetLastError();
 }
 
+// The CTA shape of the panel kernels for a tile size: calls f with (warps, row blocks per warp)
+template <class F>
+static int panel_shape(int b, F f) {
+  if (b <= 128) return f(std::integral_constant<int, 4>{}, std::integral_constant<int, 4>{});
+  if (b <= 256) return f(std::integral_constant<int, 4>{}, std::integral_constant<int, 8>{});
+  if (b <= 512) return f(std::integral_constant<int, 8>{}, std::integral_constant<int, 8>{});
+  return f(std::integral_constant<int, 8>{}, std::integral_constant<int, 16>{});
+}
+
+// doubles of the global panel scratch per tile (the reflectors of the widest level)
+size_t orth_slot_doubles(int b, int kmax) {
+  size_t n = 0;
+  panel_shape(b, [&](auto gw, auto nblk) {
+    n = (size_t)Side<decltype(gw)::value, decltype(nblk)::value>::kLdx * kmax;
+    return 0;
+  });
+  return n;
+}
+
+// Reflector panels up to this size (with the core) stay in shared memory: at k = 16 that leaves two or
+// three CTAs an SM, at k = 32 and b = 500 it would leave one (13.9 against 11.9 ms of k_orth per FP64
+// evaluation at N = 50,000), so the wider panels go to the tile's global scratch, which L2 holds.
+constexpr size_t kPanelSmem = 70 * 1024;
+
 int launch_orth(double* Z, int n, int b, int k, int ldp, int tile_base, const int* tj, const int* need,
                 double* gscratch, int nchunk, const int* status, cudaStream_t s) {
-  if (k == 16 && b <= 32 * kOrRpl) {  // panel in registers
-    k_orth_reg<8><<<nchunk, 256, 0, s>>>(Z, n, b, ldp, tile_base, tj, need, status);
+  return panel_shape(b, [&](auto gw, auto nblk) {
+    constexpr int GW = decltype(gw)::value, NBLK = decltype(nblk)::value;
+    constexpr int kLdx = Side<GW, NBLK>::kLdx;
+    const int in_smem = (size_t)kLdx * k * 8 <= kPanelSmem;
+    const size_t sm = sizeof(PanelShared<GW, NBLK>) + (size_t)kLdx * (in_smem ? k : 8) * 8;
+    cudaFuncSetAttribute(k_orth<GW, NBLK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_orth<GW, NBLK><<<nchunk, GW * 32, sm, s>>>(Z, n, b, k, ldp, tile_base, tj, need, gscratch,
+                                                 orth_slot_doubles(b, kMaxSketch), in_smem, status);
     return (int)cudaGetLastError();
-  }
-  if (k == 32 && b <= 32 * kOrRpl) {
-    k_orth_reg<16><<<nchunk, 512, 0, s>>>(Z, n, b, ldp, tile_base, tj, need, status);
-    return (int)cudaGetLastError();
-  }
-  size_t sm = (40 + 136) * 8;
-  const int in_smem = (size_t)b * k * 8 <= 160 * 1024;
-  if (in_smem) sm += (size_t)b * k * 8;
-  cudaFuncSetAttribute(k_orth, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  // the wide levels hold few tiles, each a long chain of column steps: four times the warps per
-  // step there
-  k_orth<<<nchunk, k >= 32 ? 1024 : 256, sm, s>>>(Z, n, b, k, ldp, tile_base, tj, need, gscratch, in_smem, status);
-  return (int)cudaGetLastError();
+  });
 }
 
 int launch_resid(const double* T, int n, int b, int k, int ldp, int tile_base, const int* ti, const int* tj,
@@ -822,14 +832,20 @@ int launch_finalize(int n, int b, int k, int ldp, int cap, int margin, int tile_
                     int* need, const double* P, const double* C, const double* parts, const double* fparts,
                     int nblk, double* gscratch, double* gsv, double* U, double* V, int* rank, int last_level,
                     int nchunk, int* rlog, double* tail0, double* fro0, int* blog, int* status, cudaStream_t s) {
-  size_t sm = (40 + 136 * 3 + 8 + (k <= 64 ? 2 * (size_t)k * k : 0)) * 8;
-  const int w_in_smem = k <= 64 && (size_t)b * k * 8 <= 160 * 1024;
-  if (w_in_smem) sm += (size_t)b * k * 8;
-  cudaFuncSetAttribute(k_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_finalize<<<nchunk, k >= 32 ? 1024 : 256, sm, s>>>(n, b, k, ldp, cap, margin, tile_base, ti, tj, need, P, C, parts,
-                                                      fparts, nblk, gscratch, gsv, U, V, rank, last_level,
-                                                      w_in_smem, rlog, tail0, fro0, blog, status);
-  return (int)cudaGetLastError();
+  return panel_shape(b, [&](auto gw, auto nb) {
+    constexpr int GW = decltype(gw)::value, NBLK = decltype(nb)::value;
+    constexpr int kLdx = Side<GW, NBLK>::kLdx;
+    const size_t core = ((size_t)k * (k + 1) + 1) / 2 * 2;
+    const int in_smem = (core + (size_t)kLdx * k) * 8 <= kPanelSmem;
+    // the panel's place also holds the k x r coefficients (k <= 32)
+    const size_t pan = std::max<size_t>((size_t)kLdx * (in_smem ? k : 8), k <= 32 ? (size_t)k * k : 0);
+    const size_t sm = sizeof(PanelShared<GW, NBLK>) + (core + pan) * 8;
+    cudaFuncSetAttribute(k_finalize<GW, NBLK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_finalize<GW, NBLK><<<nchunk, GW * 32, sm, s>>>(n, b, k, ldp, cap, margin, tile_base, ti, tj, need, P, C, parts,
+                                                     fparts, nblk, gscratch, orth_slot_doubles(b, kMaxSketch), gsv, U, V,
+                                                     rank, last_level, in_smem, rlog, tail0, fro0, blog, status);
+    return (int)cudaGetLastError();
+  });
 }
 
 }  // namespace tlr

@@ -53,6 +53,7 @@ int launch_gen_offdiag(const double* xy, int n, int b, int tile_base, const int*
 int launch_sketch(const double* T, int n, int b, int k, int tile_base, const int* ti, const int* tj, const int* need,
                   const double* P, double* out, int ldp, int omega, int mode, int nchunk, const int* status,
                   cudaStream_t s);
+size_t orth_slot_doubles(int b, int kmax);  // doubles of gscratch per tile
 int launch_orth(double* Z, int n, int b, int k, int ldp, int tile_base, const int* tj, const int* need,
                 double* gscratch, int nchunk, const int* status, cudaStream_t s);
 // k = 16 and b <= 512 even: projection C = T P and its residual in one pass (parts / fparts get
