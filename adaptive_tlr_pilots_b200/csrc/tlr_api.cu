@@ -56,6 +56,7 @@ struct tlr_plan {
   // data
   double *xy = nullptr, *y = nullptr, *rhs = nullptr, *z = nullptr;
   // factor
+  double* Linv = nullptr;  // inverses of the 32 x 32 diagonal blocks of every L_kk
   double *D = nullptr, *U = nullptr, *V = nullptr, *Wd = nullptr, *Yd = nullptr;
   int *rank = nullptr, *rank0 = nullptr, *ti = nullptr, *tj = nullptr;
   // compression chunk
@@ -73,7 +74,6 @@ struct tlr_plan {
   cudaEvent_t ev_panel = nullptr, ev_diag = nullptr;
   // backward: the TLR solve for alpha runs on the side stream, one event per block row
   std::vector<cudaEvent_t> ev_alpha;
-  double* solve_work = nullptr;  // inverses of the 32 x 32 diagonal blocks, allocated at the first solve
   // results
   double *ldpart = nullptr, *qpart = nullptr, *out = nullptr;
   int* status = nullptr;
@@ -255,9 +255,9 @@ int run_factorization(tlr_plan* p) {
   cudaStream_t s = p->stream, sd = p->side;
   TRY(cuda_check(cudaMemsetAsync(p->rc_next, 0, sizeof(int) * p->nB, s), "pair counters"));
   LAUNCH(TLR_K_DIAG, tlr::launch_diag_build(p->xy, p->n, p->b, 0, p->U, p->Yd, p->rank, p->cap, p->D, p->status, s));
-  LAUNCH(TLR_K_POTRF, tlr::launch_potrf(p->D, p->n, p->b, 0, p->rhs, p->z, p->ldpart, p->qpart, p->status, s));
+  LAUNCH(TLR_K_POTRF, tlr::launch_potrf(p->D, p->Linv, p->n, p->b, 0, p->rhs, p->z, p->ldpart, p->qpart, p->status, s));
   for (int k = 0; k < p->nB; ++k) {
-    LAUNCH(TLR_K_TRSM, tlr::launch_trsm(p->D, p->n, p->b, k, p->nB, p->U, p->V, p->Wd, p->Yd, p->rank, p->cap, p->z, p->rhs,
+    LAUNCH(TLR_K_TRSM, tlr::launch_trsm(p->D, p->Linv, p->n, p->b, k, p->nB, p->U, p->V, p->Wd, p->Yd, p->rank, p->cap, p->z, p->rhs,
                                         p->prec, p->blog + p->rlog_off[p->nB], 0, 1, p->status, s));
     const bool ahead = k + 1 < p->nB;
     if (ahead) {
@@ -271,7 +271,7 @@ int run_factorization(tlr_plan* p) {
                                                 p->status, s));
       TRY(cuda_check(cudaEventRecord(p->ev_panel, s), "event"));
       TRY(cuda_check(cudaStreamWaitEvent(sd, p->ev_panel, 0), "wait"));
-      LAUNCH_ON(sd, TLR_K_POTRF, tlr::launch_potrf(p->D, p->n, p->b, k + 1, p->rhs, p->z, p->ldpart, p->qpart,
+      LAUNCH_ON(sd, TLR_K_POTRF, tlr::launch_potrf(p->D, p->Linv, p->n, p->b, k + 1, p->rhs, p->z, p->ldpart, p->qpart,
                                                    p->status, sd));
       TRY(cuda_check(cudaEventRecord(p->ev_diag, sd), "event"));
     }
@@ -730,6 +730,7 @@ int tlr_plan_create(tlr_plan** plan, int n, int b, int cap, int device, void* st
   A(dalloc(p, &p->rhs, (size_t)p->nB * B));
   A(dalloc(p, &p->z, (size_t)p->nB * B));
   A(dalloc(p, &p->D, (size_t)p->nB * B * B));
+  A(dalloc(p, &p->Linv, tlr::diag_inv_doubles(b, p->nB)));
   const size_t nt = std::max(p->ntiles, 1);
   A(dalloc(p, &p->U, nt * B * cap));
   A(dalloc(p, &p->V, nt * B * cap));
@@ -1345,7 +1346,7 @@ int dist_build(tlr_plan* p, int k, cudaStream_t st) {
 }
 int dist_potrf(tlr_plan* p, int k, cudaStream_t st) {
   if (k % p->pworld != p->prank) return 0;
-  LAUNCH_ON(st, TLR_K_POTRF, tlr::launch_potrf(p->D, p->n, p->b, k, p->rhs, p->z, p->ldpart, p->qpart, p->status,
+  LAUNCH_ON(st, TLR_K_POTRF, tlr::launch_potrf(p->D, p->Linv, p->n, p->b, k, p->rhs, p->z, p->ldpart, p->qpart, p->status,
                                                st));
   return 0;
 }
@@ -1390,12 +1391,13 @@ int tlr_dist_unpack_diag(tlr_plan* p, int k, const double* buf) {
   if (!buf) return fail(TLR_ERR_ARG, "buffer is NULL");
   if (k % p->pworld == p->prank) return 0;  // the owner keeps its own
   LAUNCH(TLR_K_FILL, tlr::launch_dist_unpack_diag(p->D, p->z, p->status, p->n, p->b, k, buf, p->stream));
+  LAUNCH(TLR_K_FILL, tlr::launch_diag_inv(p->D, p->n, p->b, k, p->Linv, p->stream));
   return 0;
 }
 
 int tlr_dist_solve_step(tlr_plan* p, int k) {
   TRY(dist_ready(p, k));
-  LAUNCH(TLR_K_TRSM, tlr::launch_trsm(p->D, p->n, p->b, k, p->nB, p->U, p->V, p->Wd, p->Yd, p->rank, p->cap, p->z,
+  LAUNCH(TLR_K_TRSM, tlr::launch_trsm(p->D, p->Linv, p->n, p->b, k, p->nB, p->U, p->V, p->Wd, p->Yd, p->rank, p->cap, p->z,
                                       p->rhs, p->prec, p->blog + p->rlog_off[p->nB], p->prank, p->pworld, p->status,
                                       p->stream));
   return 0;
@@ -1483,9 +1485,8 @@ int tlr_factor_solve(tlr_plan* p, double* x_dev, int m, int trans) {
   if (!p->factor_ok) return fail(TLR_ERR_NOT_READY, "the plan holds no completed factorization");
   if (m == 0) return 0;
   TRY(cuda_check(cudaSetDevice(p->device), "cudaSetDevice"));
-  if (!p->solve_work) TRY(dalloc(p, &p->solve_work, tlr::solve_work_doubles(p->b, p->nB)));
-  const int rc = tlr::launch_factor_solve(p->D, p->U, p->V, p->rank, p->cap, p->n, p->b, p->nB, x_dev, m, trans,
-                                          p->solve_work, p->stream);
+  const int rc = tlr::launch_factor_solve(p->D, p->Linv, p->U, p->V, p->rank, p->cap, p->n, p->b, p->nB, x_dev, m,
+                                          trans, p->stream);
   if (rc) return fail(TLR_ERR_CUDA, std::string("solve launch: ") + cudaGetErrorString((cudaError_t)rc));
   return cuda_check(cudaStreamSynchronize(p->stream), "solve");
 }

@@ -13,8 +13,8 @@
 //                     k_recompress_general below under the storage rule 'mixed'
 // Layout in HBM: diagonal tiles column-major (ld b); off-diagonal factors U, V column-major
 // (ld b, cap columns per tile); tile (i, j), i > j, has index i (i - 1) / 2 + j.
-#include "tlr_device.cuh"
 #include "tlr_kernels.h"
+#include "tlr_panel.cuh"
 
 namespace tlr {
 
@@ -110,159 +110,218 @@ __global__ void __launch_bounds__(256) k_diag_build(const double* TLR_RESTRICT x
 }
 
 // ----------------------------------------------------------------------------------------
-// Panel solve for column k: one CTA per row tile i > k.
-__global__ void __launch_bounds__(256) k_trsm(const double* TLR_RESTRICT D, int n, int b, int k, int nB,
-                                             double* TLR_RESTRICT U, double* TLR_RESTRICT V,
-                                             double* TLR_RESTRICT Wd, double* TLR_RESTRICT Y,
-                                             const int* TLR_RESTRICT rank, int cap,
-                                             const double* TLR_RESTRICT z, double* TLR_RESTRICT rhs,
-                                             int* TLR_RESTRICT prec, int* TLR_RESTRICT blog_trsm, int prank,
-                                             int pworld, const int* TLR_RESTRICT status) {
+// Panel solve for column k: one CTA per row tile i > k.  V_ik <- L_kk^{-1} V_ik runs through the tile in
+// panels of 32 rows: X_p <- inv_p X_p with the inverse of the panel's diagonal block (formed beside POTRF),
+// then the rows below lose L[., p] X_p, both on the FP64 tensor cores with a column of X as a row of the
+// tiles (lane (g, t): column g, rows 2t and 2t + 1), the factor's operands loaded ahead of the barrier.
+// Then W' = V^T [V, z_k] and [Y, -rhs update] = U W'.  Bound by the chain of panels (two barriers and two
+// short products each); measured per launch at N = 50,000, b = 500: 184 -> 110 us (the tiles of the highest ranks last longest) against a 32-step
+// substitution per panel and column in one thread.
+constexpr int kTsW = 8;     // warps
+constexpr int kTsCols = 32; // columns of V per pass (16 for tiles past 512 rows)
+
+// One pass: NCB blocks of 8 columns in xs (pitch ld, npk panels of 32 rows, zero past bk).
+template <int NCB>
+__device__ __forceinline__ void trsm_pass(const double* TLR_RESTRICT L, const double* TLR_RESTRICT inv, int b, int bk,
+                                          double* xs, int ld, double* xp) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int npk = (bk + 31) / 32;
+#pragma unroll 1
+  for (int p = 0; p < npk; ++p) {
+    const int p0 = p * 32, nrest = (npk - 1 - p) * 4;  // blocks of 8 rows below
+    auto frag = [&](double (&f)[8], int q) {           // L[p0 + 32 + 8 q + g, p0 + 4 kk + t]
+      const int r = p0 + 32 + 8 * q + g;
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) f[kk] = q < nrest && r < bk ? L[(size_t)(p0 + 4 * kk + t) * b + r] : 0.0;
+    };
+    double f[8], w[8];
+    frag(f, warp);
+    const double* ip = inv + (size_t)p * 1024;
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) w[kk] = ip[(4 * kk + t) * 32 + 8 * (warp & 3) + g];
+#pragma unroll
+    for (int i = 0; i < (NCB * 4 + kTsW - 1) / kTsW; ++i) {  // rows 8 (warp % 4) of X_p, column block cb
+      const int cb = (warp >> 2) + 2 * i;
+      if (cb < NCB) {
+        const double* xc = xs + (size_t)(8 * cb + g) * ld + p0 + t;
+        double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};
+#pragma unroll
+        for (int kk = 0; kk < 8; kk += 2) {
+          dmma884(a0[0], a0[1], xc[4 * kk], w[kk]);
+          dmma884(a1[0], a1[1], xc[4 * kk + 4], w[kk + 1]);
+        }
+        *reinterpret_cast<double2*>(xp + (8 * cb + g) * 40 + 8 * (warp & 3) + 2 * t) =
+            make_double2(a0[0] + a1[0], a0[1] + a1[1]);
+      }
+    }
+    __syncthreads();
+    for (int e = tid; e < NCB * 128; e += kTsW * 32) {  // the solved panel back to xs (not read again here)
+      const int c = e >> 4, r = 2 * (e & 15);
+      *reinterpret_cast<double2*>(xs + (size_t)c * ld + p0 + r) = *reinterpret_cast<const double2*>(xp + c * 40 + r);
+    }
+    double a[NCB][8];
+#pragma unroll
+    for (int cb = 0; cb < NCB; ++cb)
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) a[cb][kk] = -xp[(8 * cb + g) * 40 + 4 * kk + t];
+#pragma unroll 1
+    for (int q = warp; q < nrest; q += kTsW) {
+      double fn[8];  // the block after this one
+      frag(fn, q + kTsW);
+      double2 v[NCB];
+#pragma unroll
+      for (int cb = 0; cb < NCB; ++cb)
+        v[cb] = *reinterpret_cast<const double2*>(xs + (size_t)(8 * cb + g) * ld + p0 + 32 + 8 * q + 2 * t);
+      if (NCB == 1) {  // one chain would be eight products deep
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int kk = 0; kk < 8; kk += 2) {
+          dmma884(v[0].x, v[0].y, a[0][kk], f[kk]);
+          dmma884(s0, s1, a[0][kk + 1], f[kk + 1]);
+        }
+        v[0].x += s0;
+        v[0].y += s1;
+      } else {
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+#pragma unroll
+          for (int cb = 0; cb < NCB; ++cb) dmma884(v[cb].x, v[cb].y, a[cb][kk], f[kk]);
+      }
+#pragma unroll
+      for (int cb = 0; cb < NCB; ++cb)
+        *reinterpret_cast<double2*>(xs + (size_t)(8 * cb + g) * ld + p0 + 32 + 8 * q + 2 * t) = v[cb];
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) f[kk] = fn[kk];
+    }
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(kTsW * 32)
+    k_trsm(const double* TLR_RESTRICT D, const double* TLR_RESTRICT Linv, int n, int b, int k, int nB, int cols,
+           double* TLR_RESTRICT U, double* TLR_RESTRICT V, double* TLR_RESTRICT Wd, double* TLR_RESTRICT Y,
+           const int* TLR_RESTRICT rank, int cap, const double* TLR_RESTRICT z, double* TLR_RESTRICT rhs,
+           int* TLR_RESTRICT prec, int* TLR_RESTRICT blog_trsm, int prank, int pworld, const int* TLR_RESTRICT status) {
   if (*status != 0) return;
   const EvalParams& prm = *eval_params(status);
   const int round_store = prm.round_store, rmode = prm.rmode;
   const double thr_abs = prm.thr_abs;
   const int i = k + 1 + blockIdx.x;
   if (i >= nB || i % pworld != prank) return;  // block-row partition: this rank's rows only
-  const int t = tidx(i, k);
-  const int r = rank[t];
+  const int t0 = tidx(i, k);
+  const int r = rank[t0];
   if (r == 0) return;
   const int bk = min(b, n - k * b), bi = min(b, n - i * b);
   const double* L = D + (size_t)k * b * b;
-  double* Vt = V + (size_t)t * b * cap;
-  double* Ut = U + (size_t)t * b * cap;
+  const double* inv = Linv + (size_t)k * ((b + 31) / 32) * 1024;
+  double* Vt = V + (size_t)t0 * b * cap;
+  double* Ut = U + (size_t)t0 * b * cap;
   if (threadIdx.x == 0) add_work(status, 9, (double)bk * bk * r + 2.0 * bk * r * r + 4.0 * bk * r,
                                  8.0 * ((double)bk * bk * 0.5 + 2.0 * bk * r + bi * r));
-  __shared__ double L11[32][33];
-  __shared__ double dinv[32];
-  __shared__ double Xp[32][65];
-  __shared__ double zt[64];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int q0 = 0; q0 < r; q0 += 64) {
-    const int rq = min(64, r - q0);
-    for (int p0 = 0; p0 < bk; p0 += 32) {
-      const int pw = min(32, bk - p0);
-      __syncthreads();
-      for (int e = tid; e < 32 * 32; e += 256) {
-        const int a = e & 31, c = e >> 5;
-        L11[a][c] = (a < pw && c < pw && a >= c) ? L[(size_t)(p0 + c) * b + p0 + a] : 0.0;
-      }
-      if (tid < 32) dinv[tid] = tid < pw ? 1.0 / L[(size_t)(p0 + tid) * b + p0 + tid] : 0.0;
-      __syncthreads();
-      // diagonal block solve, one thread per column
-      if (tid < rq) {
-        double* vc = Vt + (size_t)(q0 + tid) * b + p0;
-        double x[32];
-#pragma unroll
-        for (int a = 0; a < 32; ++a) x[a] = (a < pw) ? vc[a] : 0.0;
-#pragma unroll
-        for (int a = 0; a < 32; ++a) {
-          if (a < pw) {
-            double s = x[a];
-#pragma unroll
-            for (int c = 0; c < a; ++c) s -= L11[a][c] * x[c];
-            x[a] = s * dinv[a];
-          }
-        }
-#pragma unroll
-        for (int a = 0; a < 32; ++a)
-          if (a < pw) { vc[a] = x[a]; Xp[a][tid] = x[a]; }
-      }
-      __syncthreads();
-      // update rows below: V[row, q] -= sum_c L[row, p0 + c] X[c, q]
-      for (int row = p0 + pw + tid; row < bk; row += 256) {
-        double l[32];
-#pragma unroll
-        for (int c = 0; c < 32; ++c) l[c] = (c < pw) ? L[(size_t)(p0 + c) * b + row] : 0.0;
-        // eight columns of V at a time: their current values are loaded together, then the dots
-        for (int q1 = 0; q1 < rq; q1 += 8) {
-          double old[8], sv[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            old[u] = q1 + u < rq ? Vt[(size_t)(q0 + q1 + u) * b + row] : 0.0;
-            sv[u] = 0.0;
-          }
-#pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            const double lc = l[c];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) sv[u] = fma(lc, Xp[c][min(q1 + u, 63)], sv[u]);
-          }
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (q1 + u < rq) Vt[(size_t)(q0 + q1 + u) * b + row] = old[u] - sv[u];
-        }
-      }
+  extern __shared__ __align__(16) double xs[];
+  __shared__ __align__(16) double xp[kTsCols * 40];
+  __shared__ double red[kTsW][64];
+  __shared__ double Ws[32 * 33];
+  __shared__ double zt[128];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int rows = (bk + 31) / 32 * 32, ld = rows + 8;
+  const bool al = (b & 1) == 0;
+  for (int q0 = 0; q0 < r; q0 += cols) {
+    const int rq = min(cols, r - q0), ncb = (rq + 7) >> 3, ncx = ncb <= 2 ? ncb : 4;
+    for (int e = tid; e < rows * 8 * ncx; e += kTsW * 32) {
+      const int a = e % rows, c = e / rows;
+      xs[(size_t)c * ld + a] = (c < rq && a < bk) ? Vt[(size_t)(q0 + c) * b + a] : 0.0;
     }
+    __syncthreads();
+    if (ncb == 1) trsm_pass<1>(L, inv, b, bk, xs, ld, xp);
+    else if (ncb == 2) trsm_pass<2>(L, inv, b, bk, xs, ld, xp);
+    else trsm_pass<4>(L, inv, b, bk, xs, ld, xp);
+    for (int e = tid; e < rows * rq; e += kTsW * 32) {
+      const int a = e % rows, c = e / rows;
+      if (a < bk) Vt[(size_t)(q0 + c) * b + a] = xs[(size_t)c * ld + a];
+    }
+    __syncthreads();
   }
-  __syncthreads();
   if (round_store) {  // storage rule 'mixed': the factor tile rounded under the full budget (17:183-184)
     __shared__ double rred[40];
-    const int bits = cta_round_pair(Ut, Vt, bi, bk, r, b, thr_abs, rred, rmode == kRankReplay ? blog_trsm[t] : 0);
+    const int bits = cta_round_pair(Ut, Vt, bi, bk, r, b, thr_abs, rred, rmode == kRankReplay ? blog_trsm[t0] : 0);
     if (tid == 0) {
-      prec[t] = bits;
-      if (rmode == kRankRecord) blog_trsm[t] = bits;
+      prec[t0] = bits;
+      if (rmode == kRankRecord) blog_trsm[t0] = bits;
     }
+    __syncthreads();
   }
-  // W = V^T V (r x r) and t = V^T z_k
+  // W' = V^T [V, z_k] (r x (r + 1)), V from shared memory when it is there whole and unrounded
+  const bool held = r <= cols && !round_store;
+  const double* Vs = held ? xs : Vt;
+  const int ldv = held ? ld : b, mv = held ? rows : bk;
   const double* zk = z + (size_t)k * b;
-  double* W = Wd + (size_t)t * cap * cap;
-  for (int e = warp; e < r * r + r; e += 8) {
-    double s = 0.0;
-    if (e < r * r) {
-      const int p = e % r, q = e / r;
-      if (p <= q) {
-        const double* vp = Vt + (size_t)p * b;
-        const double* vq = Vt + (size_t)q * b;
-        for (int a = lane; a < bk; a += 32) s += vp[a] * vq[a];
-        s = warp_sum(s);
-        if (lane == 0) { W[(size_t)q * cap + p] = s; W[(size_t)p * cap + q] = s; }
+  double* W = r <= 32 ? Ws : Wd + (size_t)t0 * cap * cap;
+  const int ldw = r <= 32 ? 33 : cap;
+  for (int vb = 0; 8 * vb <= r; ++vb)
+    for (int ub = 0; ub <= vb && 8 * ub < r; ++ub) {
+      const double* pu = Vs + (size_t)min(8 * ub + g, r - 1) * ldv;
+      const int v = 8 * vb + g;
+      const bool isz = v >= r;
+      const double* pv = isz ? zk : Vs + (size_t)v * ldv;
+      const int mz = isz ? bk : mv;
+      const bool alu = held || al, alz = isz ? al : alu;  // z_k starts on 16 bytes for even b
+      double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
+#pragma unroll 4
+      for (int row = 8 * warp; row < bk; row += 8 * kTsW) {
+        const double2 x = load2(pu, row + 2 * t, mv, alu), y = load2(pv, row + 2 * t, mz, alz);
+        dmma884(a0, a1, x.x, y.x);
+        dmma884(b0, b1, x.y, y.y);
       }
-    } else {
-      const int p = e - r * r;
-      const double* vp = Vt + (size_t)p * b;
-      for (int a = lane; a < bk; a += 32) s += vp[a] * zk[a];
-      s = warp_sum(s);
-      if (lane == 0 && p < 64) zt[p] = s;
-    }
-  }
-  __syncthreads();
-  // Y_ik = U_ik W_ik, the factor of the deferred diagonal update of tile i
-  double* Yt = Y + (size_t)t * b * cap;
-  for (int a = tid; a < bi; a += 256)
-    for (int q1 = 0; q1 < r; q1 += 8) {  // eight output columns per pass over the row of U
-      double sv[8];
+      red[warp][g * 8 + 2 * t] = a0 + b0;
+      red[warp][g * 8 + 2 * t + 1] = a1 + b1;
+      __syncthreads();
+      if (tid < 64) {
+        double s = 0.0;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) sv[u] = 0.0;
-      for (int p = 0; p < r; ++p) {
-        const double up = Ut[(size_t)p * b + a];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) sv[u] = fma(up, W[(size_t)min(q1 + u, r - 1) * cap + p], sv[u]);
+        for (int w = 0; w < kTsW; ++w) s += red[w][tid];
+        const int u = 8 * ub + (tid >> 3), c = 8 * vb + (tid & 7);
+        if (u < r && c < r) {
+          W[u * ldw + c] = s;
+          if (ub != vb) W[c * ldw + u] = s;
+        } else if (u < r && c == r) {
+          zt[u] = s;
+        }
       }
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (q1 + u < r) Yt[(size_t)(q1 + u) * b + a] = sv[u];
+      __syncthreads();
     }
+  // [Y_ik, x] = U_ik W': the factor of the deferred diagonal update of tile i, and rhs_i -= x
+  double* Yt = Y + (size_t)t0 * b * cap;
   double* ri = rhs + (size_t)i * b;
-  if (r <= 64) {
-    for (int a = tid; a < bi; a += 256) {
-      double s = 0.0;
-      for (int q = 0; q < r; ++q) s = fma(Ut[(size_t)q * b + a], zt[q], s);
-      ri[a] -= s;
-    }
-  } else {
-    // wider ranks: recompute the projections column by column (rare)
-    for (int a = tid; a < bi; a += 256) {
-      double s = 0.0;
-      for (int q = 0; q < r; ++q) {
-        double tq = 0.0;
-        const double* vq = Vt + (size_t)q * b;
-        for (int u = 0; u < bk; ++u) tq += vq[u] * zk[u];
-        s = fma(Ut[(size_t)q * b + a], tq, s);
+  const int nob = r / 8 + 1;
+  for (int blk = warp; 8 * blk < bi; blk += kTsW)
+    for (int o0 = 0; o0 < nob; o0 += 4) {
+      double acc[4][2];
+#pragma unroll
+      for (int o = 0; o < 4; ++o) acc[o][0] = acc[o][1] = 0.0;
+      const int row = 8 * blk + g;
+#pragma unroll 2
+      for (int u0 = 0; u0 < r; u0 += 4) {
+        const int u = u0 + t;
+        const double x = (u < r && row < bi) ? Ut[(size_t)u * b + row] : 0.0;
+#pragma unroll
+        for (int o = 0; o < 4; ++o)
+          if (o0 + o < nob) {
+            const int c = 8 * (o0 + o) + g;
+            dmma884(acc[o][0], acc[o][1], u < r ? (c < r ? W[u * ldw + c] : (c == r ? zt[u] : 0.0)) : 0.0, x);
+          }
       }
-      ri[a] -= s;
+#pragma unroll
+      for (int o = 0; o < 4; ++o) {
+        const int c = 8 * (o0 + o) + g;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int a = 8 * blk + 2 * t + h;
+          if (a < bi && c < r) Yt[(size_t)c * b + a] = acc[o][h];
+          else if (a < bi && c == r) ri[a] -= acc[o][h];
+        }
+      }
     }
-  }
 }
 
 // ----------------------------------------------------------------------------------------
@@ -521,12 +580,15 @@ int launch_diag_build(const double* xy, int n, int b, int k, const double* U, co
   return (int)cudaGetLastError();
 }
 
-int launch_trsm(const double* D, int n, int b, int k, int nB, double* U, double* V, double* Wd, double* Y,
-                const int* rank, int cap, const double* z, double* rhs, int* prec, int* blog_trsm, int prank,
+int launch_trsm(const double* D, const double* Linv, int n, int b, int k, int nB, double* U, double* V, double* Wd,
+                double* Y, const int* rank, int cap, const double* z, double* rhs, int* prec, int* blog_trsm, int prank,
                 int pworld, const int* status, cudaStream_t s) {
   if (nB - k - 1 <= 0) return 0;
-  k_trsm<<<nB - k - 1, 256, 0, s>>>(D, n, b, k, nB, U, V, Wd, Y, rank, cap, z, rhs, prec, blog_trsm, prank, pworld,
-                                    status);
+  const int cols = b <= 512 ? kTsCols : kTsCols / 2;
+  const size_t sm = (size_t)cols * ((b + 31) / 32 * 32 + 8) * sizeof(double);
+  cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_trsm<<<nB - k - 1, kTsW * 32, sm, s>>>(D, Linv, n, b, k, nB, cols, U, V, Wd, Y, rank, cap, z, rhs, prec, blog_trsm,
+                                           prank, pworld, status);
   return (int)cudaGetLastError();
 }
 

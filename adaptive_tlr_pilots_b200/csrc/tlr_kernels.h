@@ -73,10 +73,15 @@ int launch_finalize(int n, int b, int k, int ldp, int cap, int margin, int tile_
 // factorization
 int launch_diag_build(const double* xy, int n, int b, int k, const double* U, const double* Y, const int* rank,
                       int cap, double* D, const int* status, cudaStream_t s);
-int launch_potrf(double* D, int n, int b, int k, double* rhs, double* z, double* ldpart, double* qpart,
+// POTRF of tile k; Linv gets the inverses of its 32 x 32 diagonal blocks (block p of tile k at
+// (k np + p) 1024, np = ceil(b / 32): column-major, zero above the diagonal, padded with the identity).
+// launch_diag_inv forms them from L_kk (the same bits): a block-row rank does so for a tile it received.
+size_t diag_inv_doubles(int b, int nB);
+int launch_diag_inv(const double* D, int n, int b, int k, double* Linv, cudaStream_t s);
+int launch_potrf(double* D, double* Linv, int n, int b, int k, double* rhs, double* z, double* ldpart, double* qpart,
                  int* status, cudaStream_t s);
-int launch_trsm(const double* D, int n, int b, int k, int nB, double* U, double* V, double* Wd, double* Y,
-                const int* rank, int cap, const double* z, double* rhs, int* prec, int* blog_trsm, int prank,
+int launch_trsm(const double* D, const double* Linv, int n, int b, int k, int nB, double* U, double* V, double* Wd,
+                double* Y, const int* rank, int cap, const double* z, double* rhs, int* prec, int* blog_trsm, int prank,
                 int pworld, const int* status, cudaStream_t s);
 // every trailing pair of step k; next_pair: a counter that is zero at launch (the CTAs claim
 // pairs past the grid through it).  The general form serves the storage rule 'mixed'.
@@ -147,10 +152,8 @@ int launch_dtrace_step(const double* xy, int n, int b, int m, int nB, double sig
 int launch_grad_finish(const double* part, long nparts, double* grad, const int* status, cudaStream_t s);
 
 // solves and products with the factor (tlr_solve.cu); column-major n x m, ld n
-// work: solve_work_doubles(b, nB) doubles
-size_t solve_work_doubles(int b, int nB);
-int launch_factor_solve(const double* D, const double* U, const double* V, const int* rank, int cap, int n, int b,
-                        int nB, double* X, int m, int trans, double* work, cudaStream_t s);
+int launch_factor_solve(const double* D, const double* Linv, const double* U, const double* V, const int* rank, int cap,
+                        int n, int b, int nB, double* X, int m, int trans, cudaStream_t s);
 int launch_factor_matvec(const double* D, const double* U, const double* V, const int* rank, int cap, int n, int b,
                          int nB, const double* Z, double* Y, int m, cudaStream_t s);
 

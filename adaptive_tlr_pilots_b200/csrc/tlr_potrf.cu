@@ -112,14 +112,14 @@ __device__ __forceinline__ void panel_frag(double (&f)[8][NR], const double* P, 
 // the right-hand side; 1 to 7 the trailing pieces
 template <int G>
 __global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(256)
-    k_potrf_cluster(double* TLR_RESTRICT D, int n, int b, int k, double* TLR_RESTRICT rhs, double* TLR_RESTRICT z,
+    k_potrf_cluster(double* TLR_RESTRICT D, double* TLR_RESTRICT Linv, int n, int b, int k, double* TLR_RESTRICT rhs, double* TLR_RESTRICT z,
                     double* TLR_RESTRICT ldpart, double* TLR_RESTRICT qpart, int* TLR_RESTRICT status) {
   constexpr int NW = 8;
   cg::cluster_group cluster = cg::this_cluster();
   const int g = (int)cluster.block_rank();
   __shared__ __align__(16) double Lc[2][kPB * kPL];
   __shared__ __align__(16) double Cs[kPB * kPL];  // the 32 solved rows, then the next diagonal block
-  __shared__ double dinv[2][kPB];
+  __shared__ double dinv[2][kPB], dinv2[kPB];
   __shared__ double zp[kPB];
   __shared__ int go, fail[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fg = lane >> 2, ft = lane & 3;
@@ -158,7 +158,7 @@ __global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(256)
     const double* lc = Lc[cur];
     // ---- rows below: block 0 in every CTA, the others dealt out to the cluster; the right-hand side
     const int nrb = (m + 31) / 32;
-    static_assert(5 * G + 1 >= (G == 4 ? 8 : 32), "a row warp takes at most one block of rows");
+    static_assert(4 * G + 1 + (G - 1) >= (G == 4 ? 8 : 32), "a row warp takes at most one block, the last none");
     const bool rhs_warp = warp == NW - 1;
     const int rb = warp == 1 ? 0 : 1 + g + G * (warp - 2), r = rb * 32 + lane;
     const bool rows = warp > 0 && !rhs_warp && rb < nrb;
@@ -184,6 +184,17 @@ __global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(256)
             if (q < pw) __stcg(P + (size_t)q * b + r, row[q]);
         }
       }
+    } else if (warp == 6 && g == G - 1) {
+      // a warp without rows: the inverse of the diagonal block for the panel solves, column `lane` of it as
+      // the solution for e_lane (with the quotients 1 / L_cc, as k_diag_inv)
+      dinv2[lane] = 1.0 / lc[lane * kPL + lane];
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < kPB; ++q) row[q] = q == lane ? 1.0 : 0.0;
+      solve_row(row, lc, dinv2);
+      double* o = Linv + ((size_t)k * ((b + 31) / 32) + p0 / kPB) * 1024 + lane * 32;
+#pragma unroll
+      for (int q = 0; q < kPB; q += 2) *reinterpret_cast<double2*>(o + q) = make_double2(row[q], row[q + 1]);
     } else if (warp == 0 && g == 0) {
 #pragma unroll
       for (int j = 0; j < kPB; ++j)
@@ -318,12 +329,12 @@ __global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(256)
 
 }  // namespace
 
-int launch_potrf(double* D, int n, int b, int k, double* rhs, double* z, double* ldpart, double* qpart,
+int launch_potrf(double* D, double* Linv, int n, int b, int k, double* rhs, double* z, double* ldpart, double* qpart,
                  int* status, cudaStream_t s) {
   // four CTAs share the rows and the trailing pieces of the smaller tiles (one CTA takes 41 us at
   // b = 100 against 35: its chain and its update meet on one SM), eight those past 256 rows
-  if (b <= 256) k_potrf_cluster<4><<<4, 256, 0, s>>>(D, n, b, k, rhs, z, ldpart, qpart, status);
-  else k_potrf_cluster<8><<<8, 256, 0, s>>>(D, n, b, k, rhs, z, ldpart, qpart, status);
+  if (b <= 256) k_potrf_cluster<4><<<4, 256, 0, s>>>(D, Linv, n, b, k, rhs, z, ldpart, qpart, status);
+  else k_potrf_cluster<8><<<8, 256, 0, s>>>(D, Linv, n, b, k, rhs, z, ldpart, qpart, status);
   return (int)cudaGetLastError();
 }
 

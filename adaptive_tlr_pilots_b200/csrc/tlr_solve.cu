@@ -8,9 +8,8 @@
 // launches whatever m.  Column-major N x m operands (ld = N), in place.
 //
 // A solve is one chain through the N rows, so its time is the chain's latency (the products are
-// m N b flops, microseconds).  The inverses of the 32 x 32 diagonal blocks of every L_kk come first, all
-// at once (k_diag_inv: 640 warps at N = 20,000); a panel step is then a 32 x 32 by 32 x 8 product and
-// an update of the other rows, both on the FP64 tensor cores with the operands that do not depend on X
+// m N b flops, microseconds).  The inverses of the 32 x 32 diagonal blocks of every L_kk are kept from the
+// factorization, so a panel step is a 32 x 32 by 32 x 8 product and an update of the other rows, both on the FP64 tensor cores with the operands that do not depend on X
 // loaded ahead of the barrier.  Kriging at N = 20,000, b = 500 with 300 sites (two solves of one
 // column, one of 300): 174 -> 10 ms against the substitution with one thread per column.
 #include "tlr_device.cuh"
@@ -31,16 +30,16 @@ __device__ __forceinline__ double2 pair_at(const double* s, int row, int m, bool
   return make_double2(row < m ? s[row] : 0.0, row + 1 < m ? s[row + 1] : 0.0);
 }
 
-// inv (32 x 32, column-major, zero above the diagonal) = the inverse of diagonal block p of L_kk, padded
-// with the identity: one warp per block, lane j solves L x = e_j in registers.
-__global__ void __launch_bounds__(64) k_diag_inv(const double* TLR_RESTRICT D, int n, int b, int np,
-                                                double* TLR_RESTRICT inv, int total) {
+// The inverses of the 32 x 32 diagonal blocks of L_kk (column-major, zero above the diagonal, padded with
+// the identity): one warp per block, lane j solves L x = e_j in registers.
+__global__ void __launch_bounds__(64) k_diag_inv(const double* TLR_RESTRICT D, int n, int b, int k, int np,
+                                                double* TLR_RESTRICT inv) {
   __shared__ __align__(16) double lc[2][32 * kSPitch];
   __shared__ double dinv[2][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q = blockIdx.x * 2 + w;
-  if (q >= total) return;
-  const int k = q / np, p0 = (q - k * np) * 32;
+  if (q >= np) return;
+  const int p0 = q * 32;
   const int pw = max(0, min(32, min(b, n - k * b) - p0));
   const double* L = D + (size_t)k * b * b + (size_t)p0 * b + p0;
 #pragma unroll 8
@@ -59,7 +58,7 @@ __global__ void __launch_bounds__(64) k_diag_inv(const double* TLR_RESTRICT D, i
 #pragma unroll
     for (int j = c + 1; j < 32; ++j) x[j] = fma(-x[c], lc[w][c * kSPitch + j], x[j]);
   }
-  double* o = inv + (size_t)q * 1024 + lane * 32;
+  double* o = inv + ((size_t)k * np + q) * 1024 + lane * 32;
 #pragma unroll
   for (int r = 0; r < 32; r += 2) *reinterpret_cast<double2*>(o + r) = make_double2(x[r], x[r + 1]);
 }
@@ -292,18 +291,23 @@ __global__ void __launch_bounds__(256) k_matvec_L(const double* TLR_RESTRICT D, 
 
 }  // namespace
 
-size_t solve_work_doubles(int b, int nB) { return (size_t)nB * ((b + 31) / 32) * 1024; }
+size_t diag_inv_doubles(int b, int nB) { return (size_t)nB * ((b + 31) / 32) * 1024; }
 
-int launch_factor_solve(const double* D, const double* U, const double* V, const int* rank, int cap, int n, int b,
-                        int nB, double* X, int m, int trans, double* work, cudaStream_t s) {
-  const int np = (b + 31) / 32, total = nB * np;
+int launch_diag_inv(const double* D, int n, int b, int k, double* Linv, cudaStream_t s) {
+  const int np = (b + 31) / 32;
+  k_diag_inv<<<(np + 1) / 2, 64, 0, s>>>(D, n, b, k, np, Linv);
+  return (int)cudaGetLastError();
+}
+
+int launch_factor_solve(const double* D, const double* Linv, const double* U, const double* V, const int* rank, int cap,
+                        int n, int b, int nB, double* X, int m, int trans, cudaStream_t s) {
+  const int np = (b + 31) / 32;
   const size_t sm = (size_t)kSC * (np * 32 + 8) * sizeof(double);
   const auto tri = trans ? k_tri_solve<true> : k_tri_solve<false>;
   cudaFuncSetAttribute(tri, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_diag_inv<<<(total + 1) / 2, 64, 0, s>>>(D, n, b, np, work, total);
   for (int q = 0; q < nB; ++q) {
     const int k = trans ? nB - 1 - q : q;
-    tri<<<(m + kSC - 1) / kSC, kSW * 32, sm, s>>>(D, work, n, b, np, k, X, n, m);
+    tri<<<(m + kSC - 1) / kSC, kSW * 32, sm, s>>>(D, Linv, n, b, np, k, X, n, m);
     const int rows = trans ? k : nB - k - 1;
     if (rows > 0) {
       if (m <= 8) k_solve_update<1><<<dim3(rows, 1), kSW * 32, 0, s>>>(U, V, rank, cap, n, b, k, X, n, m, trans);
