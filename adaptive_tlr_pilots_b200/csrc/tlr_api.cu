@@ -741,12 +741,12 @@ int tlr_plan_create(tlr_plan** plan, int n, int b, int cap, int device, void* st
   A(dalloc(p, &p->ti, nt));
   A(dalloc(p, &p->tj, nt));
   // compression chunk: bounded so T + panels stay within ~4 GB
-  const size_t per_tile = (B * B + 3 * B * kMaxK + tlr::orth_slot_doubles(b, kMaxK) + 2 * (size_t)kMaxK * kMaxK) * 8;
+  const size_t per_tile = (tlr::tile_doubles(b) + 3 * B * kMaxK + tlr::orth_slot_doubles(b, kMaxK) + 2 * (size_t)kMaxK * kMaxK) * 8;
   p->chunk = (int)std::max<size_t>(1, std::min<size_t>(nt, (size_t)4 * 1024 * 1024 * 1024 / per_tile));
   p->nblk = (b + 63) / 64;
   const size_t ch = (size_t)p->chunk;
   A(dalloc(p, &p->need, ch));
-  A(dalloc(p, &p->T, ch * B * B));
+  A(dalloc(p, &p->T, ch * tlr::tile_doubles(b)));
   A(dalloc(p, &p->P, ch * B * kMaxK));
   A(dalloc(p, &p->Z, ch * B * kMaxK));
   A(dalloc(p, &p->C, ch * B * kMaxK));

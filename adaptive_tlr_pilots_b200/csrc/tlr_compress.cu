@@ -23,6 +23,7 @@
 namespace tlr {
 
 constexpr int kMaxSketch = 128;  // widest sketch level
+__host__ __device__ inline int tile_pitch(int b) { return (b + 1) & ~1; }  // 16-byte rows of the generated tiles
 
 __device__ __forceinline__ double omega_entry(uint32_t tile, uint32_t row, uint32_t col) {
   // splitmix64 (Steele, Lea, Flood 2014) on (tile, row, col): a fixed, reproducible test matrix
@@ -35,7 +36,7 @@ __device__ __forceinline__ double omega_entry(uint32_t tile, uint32_t row, uint3
 }
 
 // ----------------------------------------------------------------------------------------
-// T[c] = sigma2 * matern32(dist(S_i, S_j)), row-major with leading dimension b.
+// T[c] = sigma2 * matern32(dist(S_i, S_j)), row-major with leading dimension tile_pitch(b).
 __global__ void k_gen_offdiag(const double* TLR_RESTRICT xy, int n, int b, int tile_base,
                               const int* TLR_RESTRICT ti, const int* TLR_RESTRICT tj, double* TLR_RESTRICT T,
                               const int* TLR_RESTRICT status) {
@@ -48,218 +49,119 @@ __global__ void k_gen_offdiag(const double* TLR_RESTRICT xy, int n, int b, int t
   const int i = ti[t], j = tj[t];
   const int i0 = i * b, j0 = j * b;
   const int bi = min(b, n - i0), bj = min(b, n - j0);
-  double* Tc = T + (size_t)c * b * b;
+  const int ldt = tile_pitch(b);
+  double* Tc = T + (size_t)c * b * ldt;
   const int total = bi * bj;
   if (blockIdx.x == 0 && threadIdx.x == 0) add_work(status, 1, 0.0, 8.0 * total);
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
     const int a = e / bj, q = e - a * bj;
     const double2 pa = reinterpret_cast<const double2*>(xy)[i0 + a];
     const double2 pq = reinterpret_cast<const double2*>(xy)[j0 + q];
-    Tc[(size_t)a * b + q] = matern_cov(pa.x, pa.y, pq.x, pq.y, sigma2, inv_range, nu5);
+    Tc[(size_t)a * ldt + q] = matern_cov(pa.x, pa.y, pq.x, pq.y, sigma2, inv_range, nu5);
   }
 }
 
 // ----------------------------------------------------------------------------------------
-// Strip-wise products with a 16-column block of P held in shared memory.
-//   mode 0: Z[:, g] = T^T (T P[:, g])          (range-finder sketch)
-//   mode 1: C[:, g] = T P[:, g]                 (projection)
-// P is Omega (generated) when omega != 0.  One CTA of 256 threads per (tile, column group).
-template <int H, int ZR>
-__global__ void __launch_bounds__(256) k_sketch(const double* TLR_RESTRICT T, int n, int b, int kcols,
-                                               int tile_base, const int* TLR_RESTRICT ti,
-                                               const int* TLR_RESTRICT tj, const int* TLR_RESTRICT need,
-                                               const double* TLR_RESTRICT P, double* TLR_RESTRICT out,
-                                               int ldp, int omega, int mode, const int* TLR_RESTRICT status) {
-  if (*status != 0) return;
-  const int c = blockIdx.x, g = blockIdx.y;
-  if (!need[c]) return;
-  const int t = tile_at(status, tile_base + c);
-  const int bi = min(b, n - ti[t] * b), bj = min(b, n - tj[t] * b);
-  if (threadIdx.x == 0)
-    add_work(status, mode == 0 ? 2 : 4, (mode == 0 ? 4.0 : 2.0) * bi * bj * 16,
-             8.0 * ((double)bi * bj + (omega ? 0.0 : bj * 16.0) + (mode == 0 ? bj : bi) * 16.0));
-  extern __shared__ double smem[];
-  double* Ps = smem;                       // [bj][16]
-  double* Ts = Ps + (size_t)b * 16;        // [H][b + 1]
-  double* red = Ts + (size_t)H * (b + 1);  // [KS][H][16]
-  double* Ys = red + 256 * 4;              // [H][16]
-  const int ldt = b + 1;
-  const double* Tc = T + (size_t)c * b * b;
-  const size_t pbase = (size_t)c * b * ldp;
-
-  for (int e = threadIdx.x; e < bj * 16; e += 256) {
-    const int row = e >> 4, q = e & 15;
-    Ps[e] = omega ? omega_entry((uint32_t)t, (uint32_t)row, (uint32_t)(g * 16 + q))
-                  : P[pbase + (size_t)(g * 16 + q) * b + row];
-  }
-  constexpr int BLK = (H / 2) * 8;  // 2x2 register blocks per K slice
-  constexpr int KS = 256 / BLK;     // K slices
-  const int ks = threadIdx.x / BLK, loc = threadIdx.x % BLK;
-  const int rp = loc >> 3, cp = loc & 7;
-
-  double zacc[ZR][16];
-#pragma unroll
-  for (int m = 0; m < ZR; ++m)
-#pragma unroll
-    for (int q = 0; q < 16; ++q) zacc[m][q] = 0.0;
-
-  for (int a0 = 0; a0 < bi; a0 += H) {
-    const int hrows = min(H, bi - a0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < H * bj; e += 256) {
-      const int r = e / bj, q = e - r * bj;
-      Ts[r * ldt + q] = (r < hrows) ? Tc[(size_t)(a0 + r) * b + q] : 0.0;
-    }
-    __syncthreads();
-    // phase A: Y = T_s P (H x 16), 2x2 blocks, K split in KS interleaved slices
-    double y00 = 0.0, y01 = 0.0, y10 = 0.0, y11 = 0.0;
-    const double* t0 = Ts + (2 * rp) * ldt;
-    const double* t1 = t0 + ldt;
-    for (int q = ks; q < bj; q += KS) {
-      const double2 pv = *reinterpret_cast<const double2*>(Ps + q * 16 + 2 * cp);
-      const double a = t0[q], bb = t1[q];
-      y00 = fma(a, pv.x, y00); y01 = fma(a, pv.y, y01);
-      y10 = fma(bb, pv.x, y10); y11 = fma(bb, pv.y, y11);
-    }
-    double* rd = red + ks * (H * 16);
-    rd[(2 * rp) * 16 + 2 * cp] = y00; rd[(2 * rp) * 16 + 2 * cp + 1] = y01;
-    rd[(2 * rp + 1) * 16 + 2 * cp] = y10; rd[(2 * rp + 1) * 16 + 2 * cp + 1] = y11;
-    __syncthreads();
-    for (int e = threadIdx.x; e < H * 16; e += 256) {
-      double s = 0.0;
-#pragma unroll
-      for (int k2 = 0; k2 < KS; ++k2) s += red[k2 * (H * 16) + e];
-      Ys[e] = s;
-    }
-    __syncthreads();
-    if (mode == 1) {
-      // C rows a0.., column group g
-      for (int e = threadIdx.x; e < hrows * 16; e += 256) {
-        const int r = e >> 4, q = e & 15;
-        out[pbase + (size_t)(g * 16 + q) * b + a0 + r] = Ys[e];
-      }
-      continue;
-    }
-    // phase B: Z += T_s^T Y
-#pragma unroll
-    for (int m = 0; m < ZR; ++m) {
-      const int z = threadIdx.x + 256 * m;
-      if (z < bj) {
-        for (int r = 0; r < hrows; ++r) {
-          const double a = Ts[r * ldt + z];
-          const double2* yr = reinterpret_cast<const double2*>(Ys + r * 16);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const double2 yv = yr[q];
-            zacc[m][2 * q] = fma(a, yv.x, zacc[m][2 * q]);
-            zacc[m][2 * q + 1] = fma(a, yv.y, zacc[m][2 * q + 1]);
-          }
-        }
-      }
-    }
-  }
-  if (mode == 0) {
-#pragma unroll
-    for (int m = 0; m < ZR; ++m) {
-      const int z = threadIdx.x + 256 * m;
-      if (z < bj)
-#pragma unroll
-        for (int q = 0; q < 16; ++q) out[pbase + (size_t)(g * 16 + q) * b + z] = zacc[m][q];
-    }
-  }
-}
-
-// ----------------------------------------------------------------------------------------
-// The same two products on the FP64 tensor cores (tiles up to 512 wide, even b).
-//   One CTA of 16 warps per (tile, 16-column group); warp w owns columns [32w, 32w + 32) of T.
-//   T streams through shared memory in slabs of 16 rows, double-buffered with cp.async (the
-//   next slab's copy runs under this slab's products).  Per slab R:
-//     phase A  Y_R = T_R P: each warp multiplies its 32-column strip by its 32 rows of P (held in
-//              registers for the whole kernel) -> a 16 x 16 partial; the 16 partials are summed
-//              in a fixed order (mode 1 writes that sum: the rows R of C = T P);
+// The range finder's products on the FP64 tensor cores.  One CTA of W warps per (tile, group of 8 NT
+// columns of P); warp w owns columns [CW w, CW w + CW) of T, so a CTA covers tiles up to W CW wide.
+//   T streams through shared memory in slabs of H rows, double-buffered with cp.async (the next slab's
+//   copy runs under this slab's products).  Per slab R:
+//     phase A  Y_R = T_R P: each warp multiplies its column strip by its rows of P (held in registers
+//              for the whole kernel) -> an H x 8 NT partial; the W partials are summed in a fixed order
+//              (mode 1 writes that sum: the rows R of C = T P);
 //     phase B  Z[strip] += T_R[:, strip]^T Y_R, accumulated in registers across slabs.
-//   Every T element is read from HBM once per launch and used by both phases from shared memory.
+//   Every T element is read from HBM once per launch and group and used by both phases from shared
+//   memory.
 //   MODE 0: the sketch Z = T^T T P.  MODE 1: the projection C = T P.  MODE 2 (one 16-column group,
 //   k = 16): the projection and, in place of phase B, the residual of the slab on the tensor cores,
 //   E_R = T_R - C_R P^T (accumulator started at T_R, operand -C_R), with rho^2 = sum E^2 and
 //   ||T||^2 summed per lane in a fixed order and over the CTA in warp order into parts[c],
 //   fparts[c] (one block per tile): T leaves HBM once for both.
-constexpr int kSkW = 16;                 // warps per CTA
-constexpr int kSkH = 16;                 // rows of T per slab
-constexpr int kSkCols = 32 * kSkW;       // widest tile handled (512)
-constexpr int kSkPitch = kSkCols + 4;    // slab row pitch in doubles (conflict-free fragments)
-constexpr int kSkYp = 18;                // pitch of the per-warp partials
-constexpr int kSkYs = 17;                // pitch of the summed Y_R
+// Bound by the FP64 tensor pipe (17 cycles per m8n8k4 step and scheduler).  The shape follows the tile so
+// that no warp multiplies padding: 4, 8 or 16 warps of 32 columns up to b = 128, 256, 512; up to 1024
+// sixteen warps of 64 columns with 8 columns of P (the registers of 16 would spill), at the price of
+// reading T twice as often.  T's rows are padded to an even pitch, so odd tile sizes take it too.
+// Sketch passes of one FP64 evaluation: N = 12,000, b = 1000 24.3 -> 3.2 ms, N = 10,007, b = 250
+// 3.6 -> 1.7 ms, N = 4,000, b = 203 1.64 -> 0.68 ms, N = 1,030, b = 100 0.29 -> 0.16 ms against one
+// 512-wide shape for even b <= 512 and CUDA-core products for the others.
+template <int W, int CW, int NT, int H>
+struct SketchShape {
+  static constexpr int kCols = W * CW;
+  static constexpr int kPitch = kCols + 4;  // conflict-free fragments
+  static constexpr int kYp = 8 * NT + 2;    // pitch of the per-warp partials
+  static constexpr int kYs = 8 * NT + 1;    // pitch of the summed Y_R
+  static constexpr size_t kSmem = ((size_t)2 * H * kPitch + (size_t)W * H * kYp + (size_t)H * kYs) * sizeof(double);
+};
 
-static size_t sketch_mma_smem() {
-  return ((size_t)2 * kSkH * kSkPitch + (size_t)kSkW * kSkH * kSkYp + (size_t)kSkH * kSkYs) * sizeof(double);
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(kSkW * 32, 1)
+template <int MODE, int W, int CW, int NT, int H>
+__global__ void __launch_bounds__(W * 32, 16 / W)
     k_sketch_mma(const double* TLR_RESTRICT T, int n, int b, int tile_base, const int* TLR_RESTRICT ti,
                  const int* TLR_RESTRICT tj, const int* TLR_RESTRICT need, const double* TLR_RESTRICT P,
                  double* TLR_RESTRICT out, int ldp, int omega, double* TLR_RESTRICT parts,
                  double* TLR_RESTRICT fparts, const int* TLR_RESTRICT status) {
-  constexpr int mode = MODE == 0 ? 0 : 1;
+  using Sh = SketchShape<W, CW, NT, H>;
+  constexpr int kPitch = Sh::kPitch, kYp = Sh::kYp, kYs = Sh::kYs, kMt = H / 8;
+  static_assert(MODE != 2 || NT == 2, "the fused residual needs the whole k = 16 panel");
   if (*status != 0) return;
   const int c = blockIdx.x, grp = blockIdx.y;
   if (!need[c]) return;
   const int t = tile_at(status, tile_base + c);
   const int bi = min(b, n - ti[t] * b), bj = min(b, n - tj[t] * b);
   if (threadIdx.x == 0) {
-    add_work(status, mode == 0 ? 2 : 4, (mode == 0 ? 4.0 : 2.0) * bi * bj * 16,
-             8.0 * ((double)bi * bj + (omega ? 0.0 : bj * 16.0) + (mode == 0 ? bj : bi) * 16.0));
+    add_work(status, MODE == 0 ? 2 : 4, (MODE == 0 ? 4.0 : 2.0) * bi * bj * 8 * NT,
+             8.0 * ((double)bi * bj + (omega ? 0.0 : bj * 8.0 * NT) + (MODE == 0 ? bj : bi) * 8.0 * NT));
     if (MODE == 2) add_work(status, 5, 2.0 * bi * bj * 17, 0.0);
   }
   extern __shared__ __align__(16) double sk_smem[];
-  double* Ts = sk_smem;                                   // [2][kSkH][kSkPitch]
-  double* Yp = Ts + (size_t)2 * kSkH * kSkPitch;          // [kSkW][kSkH][kSkYp]
-  double* Ys = Yp + (size_t)kSkW * kSkH * kSkYp;          // [kSkH][kSkYs]
+  double* Ts = sk_smem;                          // [2][H][kPitch]
+  double* Yp = Ts + (size_t)2 * H * kPitch;      // [W][H][kYp]
+  double* Ys = Yp + (size_t)W * H * kYp;         // [H][kYs]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tg = lane & 3;
-  const double* Tc = T + (size_t)c * b * b;
+  const int ldt = tile_pitch(b);
+  const double* Tc = T + (size_t)c * b * ldt;
   const size_t pbase = (size_t)c * b * ldp;
-  const int col0 = warp * 32;
-  const int nslab = (bi + kSkH - 1) / kSkH;
+  const int col0 = warp * CW;
+  const int nslab = (bi + H - 1) / H;
 
-  // slab s -> stage s & 1: kSkH rows x kSkCols columns in 16-byte pieces, zero past bi / bj
+  // slab s -> stage s & 1: H rows x kCols columns in 16-byte pieces, zero past bi / bj
   auto issue = [&](int s) {
-    double* dst = Ts + (size_t)(s & 1) * kSkH * kSkPitch;
-    const int a0 = s * kSkH;
-    for (int e = tid; e < kSkH * (kSkCols / 2); e += kSkW * 32) {
-      const int r = e / (kSkCols / 2), col = 2 * (e % (kSkCols / 2));
+    double* dst = Ts + (size_t)(s & 1) * H * kPitch;
+    const int a0 = s * H;
+#pragma unroll
+    for (int e = tid; e < H * (Sh::kCols / 2); e += W * 32) {
+      const int r = e / (Sh::kCols / 2), col = 2 * (e % (Sh::kCols / 2));
       const int row = a0 + r;
       const int bytes = row < bi ? (col + 1 < bj ? 16 : (col < bj ? 8 : 0)) : 0;
-      cp_async16(dst + (size_t)r * kSkPitch + col, bytes ? Tc + (size_t)row * b + col : Tc, bytes);
+      cp_async16(dst + (size_t)r * kPitch + col, bytes ? Tc + (size_t)row * ldt + col : Tc, bytes);
     }
     cp_async_commit();
   };
   issue(0);
 
   // B fragments of P for phase A: rows col0 + 4 kk + tg, columns 8 nt + g of the group
-  double pf[8][2];
+  double pf[CW / 4][NT];
 #pragma unroll
-  for (int kk = 0; kk < 8; ++kk)
+  for (int kk = 0; kk < CW / 4; ++kk)
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-      const int row = col0 + 4 * kk + tg, q = grp * 16 + 8 * nt + g;
+    for (int nt = 0; nt < NT; ++nt) {
+      const int row = col0 + 4 * kk + tg, q = (grp * NT + nt) * 8 + g;
       pf[kk][nt] = row < bj ? (omega ? omega_entry((uint32_t)t, (uint32_t)row, (uint32_t)q)
                                      : P[pbase + (size_t)q * b + row])
                             : 0.0;
     }
-  double za[4][2][2];
+  double za[CW / 8][NT][2];
 #pragma unroll
-  for (int m = 0; m < 4; ++m)
+  for (int m = 0; m < CW / 8; ++m)
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) za[m][nt][0] = za[m][nt][1] = 0.0;
+    for (int nt = 0; nt < NT; ++nt) za[m][nt][0] = za[m][nt][1] = 0.0;
   // MODE 2: B fragments of P^T for the residual, P rows col0 + 8 j + g, columns 4 kq + tg
-  double pt[4][4];
+  double pt[4][CW / 8];
   double rho = 0.0, fro = 0.0;
   if (MODE == 2) {
 #pragma unroll
     for (int kq = 0; kq < 4; ++kq)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < CW / 8; ++j) {
         const int row = col0 + 8 * j + g;
         pt[kq][j] = row < bj ? P[pbase + (size_t)(4 * kq + tg) * b + row] : 0.0;
       }
@@ -269,67 +171,68 @@ __global__ void __launch_bounds__(kSkW * 32, 1)
     cp_async_wait_all();
     __syncthreads();  // slab s visible to all; every warp is done with slab s - 1
     if (s + 1 < nslab) issue(s + 1);
-    const double* Tsl = Ts + (size_t)(s & 1) * kSkH * kSkPitch;
-    double ya[2][2][2];
+    const double* Tsl = Ts + (size_t)(s & 1) * H * kPitch;
+    double ya[kMt][NT][2];
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
+    for (int m = 0; m < kMt; ++m)
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt) ya[m][nt][0] = ya[m][nt][1] = 0.0;
+      for (int nt = 0; nt < NT; ++nt) ya[m][nt][0] = ya[m][nt][1] = 0.0;
 #pragma unroll
-    for (int kk = 0; kk < 8; ++kk)
+    for (int kk = 0; kk < CW / 4; ++kk)
 #pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        const double a = Tsl[(size_t)(8 * m + g) * kSkPitch + col0 + 4 * kk + tg];
+      for (int m = 0; m < kMt; ++m) {
+        const double a = Tsl[(size_t)(8 * m + g) * kPitch + col0 + 4 * kk + tg];
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) dmma884(ya[m][nt][0], ya[m][nt][1], a, pf[kk][nt]);
+        for (int nt = 0; nt < NT; ++nt) dmma884(ya[m][nt][0], ya[m][nt][1], a, pf[kk][nt]);
       }
-    double* yp = Yp + (size_t)warp * kSkH * kSkYp;
+    double* yp = Yp + (size_t)warp * H * kYp;
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
+    for (int m = 0; m < kMt; ++m)
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
+      for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) yp[(8 * m + g) * kSkYp + 8 * nt + 2 * tg + h] = ya[m][nt][h];
+        for (int h = 0; h < 2; ++h) yp[(8 * m + g) * kYp + 8 * nt + 2 * tg + h] = ya[m][nt][h];
     __syncthreads();
-    if (tid < kSkH * 16) {
-      const int r = tid >> 4, q = tid & 15;
+#pragma unroll
+    for (int e = tid; e < H * 8 * NT; e += W * 32) {
+      const int r = e / (8 * NT), q = e % (8 * NT);
       double sum = 0.0;
 #pragma unroll
-      for (int w = 0; w < kSkW; ++w) sum += Yp[(size_t)w * kSkH * kSkYp + r * kSkYp + q];
-      if (mode == 1) {
-        const int row = s * kSkH + r;
-        if (row < bi) out[pbase + (size_t)(grp * 16 + q) * b + row] = sum;
+      for (int w = 0; w < W; ++w) sum += Yp[(size_t)w * H * kYp + r * kYp + q];
+      if (MODE != 0) {
+        const int row = s * H + r;
+        if (row < bi) out[pbase + (size_t)(grp * 8 * NT + q) * b + row] = sum;
       }
-      if (MODE != 1) Ys[r * kSkYs + q] = sum;
+      if (MODE != 1) Ys[r * kYs + q] = sum;
     }
     if (MODE == 1) continue;
     __syncthreads();
     if (MODE == 2) {
       // E_R[:, strip] = T_R[:, strip] - C_R P[strip, :]^T
-      double e[2][4][2];
+      double e[kMt][CW / 8][2];
 #pragma unroll
-      for (int m = 0; m < 2; ++m)
+      for (int m = 0; m < kMt; ++m)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < CW / 8; ++j)
 #pragma unroll
-          for (int h = 0; h < 2; ++h) e[m][j][h] = Tsl[(size_t)(8 * m + g) * kSkPitch + col0 + 8 * j + 2 * tg + h];
+          for (int h = 0; h < 2; ++h) e[m][j][h] = Tsl[(size_t)(8 * m + g) * kPitch + col0 + 8 * j + 2 * tg + h];
 #pragma unroll
       for (int kq = 0; kq < 4; ++kq)
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
-          const double a = -Ys[(8 * m + g) * kSkYs + 4 * kq + tg];
+        for (int m = 0; m < kMt; ++m) {
+          const double a = -Ys[(8 * m + g) * kYs + 4 * kq + tg];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) dmma884(e[m][j][0], e[m][j][1], a, pt[kq][j]);
+          for (int j = 0; j < CW / 8; ++j) dmma884(e[m][j][0], e[m][j][1], a, pt[kq][j]);
         }
 #pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        const bool rin = s * kSkH + 8 * m + g < bi;
+      for (int m = 0; m < kMt; ++m) {
+        const bool rin = s * H + 8 * m + g < bi;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < CW / 8; ++j)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             if (rin && col0 + 8 * j + 2 * tg + h < bj) {
-              const double tv = Tsl[(size_t)(8 * m + g) * kSkPitch + col0 + 8 * j + 2 * tg + h];
+              const double tv = Tsl[(size_t)(8 * m + g) * kPitch + col0 + 8 * j + 2 * tg + h];
               rho = fma(e[m][j][h], e[m][j][h], rho);
               fro = fma(tv, tv, fro);
             }
@@ -339,15 +242,15 @@ __global__ void __launch_bounds__(kSkW * 32, 1)
     }
     if constexpr (MODE == 0) {  // the sketch's second product; the other modes left above
 #pragma unroll
-      for (int kq = 0; kq < kSkH / 4; ++kq) {
-        double bf[2];
+      for (int kq = 0; kq < H / 4; ++kq) {
+        double bf[NT];
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) bf[nt] = Ys[(4 * kq + tg) * kSkYs + 8 * nt + g];
+        for (int nt = 0; nt < NT; ++nt) bf[nt] = Ys[(4 * kq + tg) * kYs + 8 * nt + g];
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          const double a = Tsl[(size_t)(4 * kq + tg) * kSkPitch + col0 + 8 * m + g];
+        for (int m = 0; m < CW / 8; ++m) {
+          const double a = Tsl[(size_t)(4 * kq + tg) * kPitch + col0 + 8 * m + g];
 #pragma unroll
-          for (int nt = 0; nt < 2; ++nt) dmma884(za[m][nt][0], za[m][nt][1], a, bf[nt]);
+          for (int nt = 0; nt < NT; ++nt) dmma884(za[m][nt][0], za[m][nt][1], a, bf[nt]);
         }
       }
     }
@@ -358,14 +261,14 @@ __global__ void __launch_bounds__(kSkW * 32, 1)
     __syncthreads();
     if (lane == 0) {
       Yp[warp] = rho;
-      Yp[kSkW + warp] = fro;
+      Yp[W + warp] = fro;
     }
     __syncthreads();
     if (tid == 0) {
       double a = 0.0, f = 0.0;
-      for (int w = 0; w < kSkW; ++w) {
+      for (int w = 0; w < W; ++w) {
         a += Yp[w];
-        f += Yp[kSkW + w];
+        f += Yp[W + w];
       }
       parts[c] = a;
       fparts[c] = f;
@@ -373,13 +276,14 @@ __global__ void __launch_bounds__(kSkW * 32, 1)
   }
   if (MODE == 0) {
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
+    for (int m = 0; m < CW / 8; ++m) {
       const int col = col0 + 8 * m + g;
       if (col < bj)
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
+        for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-          for (int h = 0; h < 2; ++h) out[pbase + (size_t)(grp * 16 + 8 * nt + 2 * tg + h) * b + col] = za[m][nt][h];
+          for (int h = 0; h < 2; ++h)
+            out[pbase + (size_t)((grp * NT + nt) * 8 + 2 * tg + h) * b + col] = za[m][nt][h];
     }
   }
 }
@@ -532,7 +436,8 @@ __global__ void __launch_bounds__(256) k_resid(const double* TLR_RESTRICT T, int
     const int r = e % 64, q = e / 64;
     Pb[r * (k + 1) + q] = (r < qn) ? P[pbase + (size_t)q * b + q0 + r] : 0.0;
   }
-  const double* Tc = T + (size_t)c * b * b;
+  const int ldt = tile_pitch(b);
+  const double* Tc = T + (size_t)c * b * ldt;
   double acc = 0.0, facc = 0.0;
   const int col = threadIdx.x & 63, rsub = threadIdx.x >> 6;  // 4 row lanes x 64 columns
   for (int a0 = 0; a0 < bi; a0 += 16) {
@@ -550,7 +455,7 @@ __global__ void __launch_bounds__(256) k_resid(const double* TLR_RESTRICT T, int
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int r = rsub + 4 * u;
-        tv[u] = r < hrows ? Tc[(size_t)(a0 + r) * b + q0 + col] : 0.0;
+        tv[u] = r < hrows ? Tc[(size_t)(a0 + r) * ldt + q0 + col] : 0.0;
         sv[u] = tv[u];
       }
       const double* pr = Pb + col * (k + 1);
@@ -738,47 +643,51 @@ int launch_gen_offdiag(const double* xy, int n, int b, int tile_base, const int*
   return (int)cudaGetLastError();
 }
 
-static size_t sketch_smem(int b, int H) { return ((size_t)b * 16 + (size_t)H * (b + 1) + 256 * 4 + H * 16) * 8; }
+template <int MODE, int W, int CW, int NT, int H>
+static int run_sketch(int nchunk, int k, const double* T, int n, int b, int tile_base, const int* ti, const int* tj,
+                      const int* need, const double* P, double* out, int ldp, int omega, double* parts, double* fparts,
+                      const int* status, cudaStream_t s) {
+  constexpr size_t sm = SketchShape<W, CW, NT, H>::kSmem;
+  cudaFuncSetAttribute(k_sketch_mma<MODE, W, CW, NT, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_sketch_mma<MODE, W, CW, NT, H><<<dim3((unsigned)nchunk, (unsigned)(k / (8 * NT))), W * 32, sm, s>>>(
+      T, n, b, tile_base, ti, tj, need, P, out, ldp, omega, parts, fparts, status);
+  return (int)cudaGetLastError();
+}
 
 int launch_sketch(const double* T, int n, int b, int k, int tile_base, const int* ti, const int* tj,
                   const int* need, const double* P, double* out, int ldp, int omega, int mode, int nchunk,
                   const int* status, cudaStream_t s) {
-  dim3 grid((unsigned)nchunk, (unsigned)(k / 16));
-  if (b <= kSkCols && b % 2 == 0) {  // 16-byte aligned rows: the tensor-core form
-    const size_t sm = sketch_mma_smem();
-    if (mode == 0) {
-      cudaFuncSetAttribute(k_sketch_mma<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_sketch_mma<0><<<grid, kSkW * 32, sm, s>>>(T, n, b, tile_base, ti, tj, need, P, out, ldp, omega, nullptr,
-                                                  nullptr, status);
-    } else {
-      cudaFuncSetAttribute(k_sketch_mma<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_sketch_mma<1><<<grid, kSkW * 32, sm, s>>>(T, n, b, tile_base, ti, tj, need, P, out, ldp, omega, nullptr,
-                                                  nullptr, status);
-    }
-  } else if (b <= 512) {
-    const size_t sm = sketch_smem(b, 16);
-    cudaFuncSetAttribute(k_sketch<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_sketch<16, 2><<<grid, 256, sm, s>>>(T, n, b, k, tile_base, ti, tj, need, P, out, ldp, omega, mode, status);
-  } else {
-    const size_t sm = sketch_smem(b, 8);
-    cudaFuncSetAttribute(k_sketch<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_sketch<8, 4><<<grid, 256, sm, s>>>(T, n, b, k, tile_base, ti, tj, need, P, out, ldp, omega, mode, status);
-  }
-  return (int)cudaGetLastError();
+  auto run = [&](auto m) {
+    constexpr int M = decltype(m)::value;
+    if (b <= 128)
+      return run_sketch<M, 4, 32, 2, 16>(nchunk, k, T, n, b, tile_base, ti, tj, need, P, out, ldp, omega, nullptr, nullptr,
+                                         status, s);
+    if (b <= 256)
+      return run_sketch<M, 8, 32, 2, 16>(nchunk, k, T, n, b, tile_base, ti, tj, need, P, out, ldp, omega, nullptr, nullptr,
+                                         status, s);
+    if (b <= 512)
+      return run_sketch<M, 16, 32, 2, 16>(nchunk, k, T, n, b, tile_base, ti, tj, need, P, out, ldp, omega, nullptr,
+                                          nullptr, status, s);
+    return run_sketch<M, 16, 64, 1, 8>(nchunk, k, T, n, b, tile_base, ti, tj, need, P, out, ldp, omega, nullptr, nullptr,
+                                       status, s);
+  };
+  return mode == 0 ? run(std::integral_constant<int, 0>{}) : run(std::integral_constant<int, 1>{});
 }
 
-bool project_resid_fused(int b, int k) { return k == 16 && b <= kSkCols && b % 2 == 0; }
+bool project_resid_fused(int b, int k) { return k == 16 && b <= 512; }
 
 int launch_project_resid(const double* T, int n, int b, int tile_base, const int* ti, const int* tj,
                          const int* need, const double* P, double* C, int ldp, double* parts, double* fparts,
                          int nchunk, const int* status, cudaStream_t s) {
   if (!project_resid_fused(b, 16)) return (int)cudaErrorInvalidValue;
-  const size_t sm = sketch_mma_smem();
-  cudaFuncSetAttribute(k_sketch_mma<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_sketch_mma<2><<<dim3((unsigned)nchunk, 1), kSkW * 32, sm, s>>>(T, n, b, tile_base, ti, tj, need, P, C, ldp, 0,
-                                                                   parts, fparts, status);
-  return (int)cudaGetLastError();
+  if (b <= 128)
+    return run_sketch<2, 4, 32, 2, 16>(nchunk, 16, T, n, b, tile_base, ti, tj, need, P, C, ldp, 0, parts, fparts, status, s);
+  if (b <= 256)
+    return run_sketch<2, 8, 32, 2, 16>(nchunk, 16, T, n, b, tile_base, ti, tj, need, P, C, ldp, 0, parts, fparts, status, s);
+  return run_sketch<2, 16, 32, 2, 16>(nchunk, 16, T, n, b, tile_base, ti, tj, need, P, C, ldp, 0, parts, fparts, status, s);
 }
+
+size_t tile_doubles(int b) { return (size_t)b * tile_pitch(b); }
 
 // The CTA shape of the panel kernels for a tile size: calls f with (warps, row blocks per warp)
 template <class F>

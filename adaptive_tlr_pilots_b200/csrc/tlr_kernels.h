@@ -48,6 +48,7 @@ int launch_gather_sites(const double* xy_in, const double* y_in, const long long
                         double* y_out, cudaStream_t s);
 
 // initial compression
+size_t tile_doubles(int b);  // doubles of one generated tile T (row-major, even pitch)
 int launch_gen_offdiag(const double* xy, int n, int b, int tile_base, const int* ti, const int* tj, double* T,
                        int nchunk, const int* status, cudaStream_t s);
 int launch_sketch(const double* T, int n, int b, int k, int tile_base, const int* ti, const int* tj, const int* need,
@@ -56,7 +57,7 @@ int launch_sketch(const double* T, int n, int b, int k, int tile_base, const int
 size_t orth_slot_doubles(int b, int kmax);  // doubles of gscratch per tile
 int launch_orth(double* Z, int n, int b, int k, int ldp, int tile_base, const int* tj, const int* need,
                 double* gscratch, int nchunk, const int* status, cudaStream_t s);
-// k = 16 and b <= 512 even: projection C = T P and its residual in one pass (parts / fparts get
+// k = 16 and b <= 512: projection C = T P and its residual in one pass (parts / fparts get
 // one block per tile)
 bool project_resid_fused(int b, int k);
 int launch_project_resid(const double* T, int n, int b, int tile_base, const int* ti, const int* tj,
