@@ -757,7 +757,7 @@ int tlr_plan_create(tlr_plan** plan, int n, int b, int cap, int device, void* st
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   p->nsm = nsm;
-  p->nslots = nsm * tlr::rc_blocks_per_sm(b);  // resident recompression CTAs
+  p->nslots = nsm * tlr::rc_blocks_per_sm(b, cap);  // resident recompression CTAs
   p->nslots_general = nsm * tlr::rc_general_blocks_per_sm();
   p->slot_doubles = std::max(tlr::rc_slot_doubles(b, cap), tlr::rc_general_slot_doubles(b, cap));
   A(dalloc(p, &p->rcs, (size_t)std::max(p->nslots, p->nslots_general) * p->slot_doubles));

@@ -522,7 +522,8 @@ __global__ void __launch_bounds__(GW * 32, 16 / GW)
       else jacobi_warp<2, 16>(M, ldm, k);
     }
   } else {
-    jacobi_group<GT>(M, ldm, k, nn, mx, flag, tid, 1);
+    if (k <= 64) jacobi_group<GT, 8, 8, true>(M, ldm, k, nn, mx, flag, tid, 1);
+    else jacobi_group<GT, 8, 16, true>(M, ldm, k, nn, mx, flag, tid, 1);
   }
   sd.sync();
   for (int q0 = 0; q0 < k; q0 += GT / 4) {  // singular values: the row norms

@@ -86,7 +86,7 @@ int launch_trsm(const double* D, const double* Linv, int n, int b, int k, int nB
                 int pworld, const int* status, cudaStream_t s);
 // every trailing pair of step k; next_pair: a counter that is zero at launch (the CTAs claim
 // pairs past the grid through it).  The general form serves the storage rule 'mixed'.
-int rc_blocks_per_sm(int b);  // k_recompress CTAs resident per SM
+int rc_blocks_per_sm(int b, int cap);  // k_recompress CTAs resident per SM
 size_t rc_slot_doubles(int b, int cap);
 int launch_recompress(int n, int b, int k, int nB, double* U, double* V, int* rank, int cap, double* scratch,
                       size_t slot_doubles, int nslots, int* next_pair, int* rlog_step, int prank, int pworld,

@@ -381,30 +381,58 @@ __device__ __noinline__ void warp_core_r(double* M, int ldm, int s, double* buf)
   __syncwarp();
 }
 
-// The same by a whole group (s > 32): a thread per column.
-template <int GT>
+// The same by a whole group (s > 32): the rows of a column split over up to four adjacent lanes.
+template <int GT, bool SHARED>
 __device__ __noinline__ void group_core_r(double* M, int ldm, int s, int tg, int bar) {
+  if (SHARED) __builtin_assume(__isShared(M));
+  const int nsp = s <= GT / 4 ? 4 : s <= GT / 2 ? 2 : 1, sp = tg % nsp;
   for (int c = 0; c < s - 1; ++c) {
     double sg[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int r0 = c + 1; r0 < s; r0 += 4)
+    for (int r0 = c + 1 + sp; r0 < s; r0 += 8 * nsp) {
+      double x[8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const double x = r0 + u < s ? M[(r0 + u) * ldm + c] : 0.0;
-        sg[u] = fma(x, x, sg[u]);
-      }
-    const double sig2 = (sg[0] + sg[1]) + (sg[2] + sg[3]);
+      for (int u = 0; u < 8; ++u) x[u] = r0 + u * nsp < s ? M[(r0 + u * nsp) * ldm + c] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) sg[u & 3] = fma(x[u], x[u], sg[u & 3]);
+    }
+    double sig2 = (sg[0] + sg[1]) + (sg[2] + sg[3]);
+    for (int o = 1; o < nsp; o <<= 1) sig2 += __shfl_xor_sync(0xffffffffu, sig2, o);
     const Reflector rf = reflector(M[c * ldm + c], sig2);
-    for (int j = c + 1 + tg; j < s; j += GT) {
-      double d0 = 0.0, d1 = 0.0;
-      int r = c + 1;
-      for (; r + 1 < s; r += 2) {
-        d0 = fma(M[r * ldm + c], M[r * ldm + j], d0);
-        d1 = fma(M[(r + 1) * ldm + c], M[(r + 1) * ldm + j], d1);
+    const int step = GT / nsp;
+    for (int j0 = c + 1; j0 < s; j0 += step) {  // the same trip count in every thread (shuffles)
+      const int j = j0 + tg / nsp, jc = min(j, s - 1);
+      double d[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int r0 = c + 1 + sp; r0 < s; r0 += 8 * nsp) {
+        double x[8], y[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const bool in = r0 + u * nsp < s;
+          x[u] = in ? M[(r0 + u * nsp) * ldm + c] : 0.0;
+          y[u] = in ? M[(r0 + u * nsp) * ldm + jc] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) d[u & 3] = fma(x[u], y[u], d[u & 3]);
       }
-      if (r < s) d0 = fma(M[r * ldm + c], M[r * ldm + j], d0);
-      const double w = rf.kappa * fma(rf.d, M[c * ldm + j], d0 + d1);
-      for (int q = c + 1; q < s; ++q) M[q * ldm + j] = fma(-w, M[q * ldm + c], M[q * ldm + j]);
-      M[c * ldm + j] = fma(-w, rf.d, M[c * ldm + j]);
+      double dt = (d[0] + d[1]) + (d[2] + d[3]);
+      for (int o = 1; o < nsp; o <<= 1) dt += __shfl_xor_sync(0xffffffffu, dt, o);
+      const double mj = M[c * ldm + jc], w = rf.kappa * fma(rf.d, mj, dt);
+      __syncwarp();
+      if (j < s) {
+        // eight rows at a time: their loads come ahead of the stores, which the compiler could not reorder
+        for (int q0 = c + 1 + sp; q0 < s; q0 += 8 * nsp) {
+          double xc[8], xj[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const int q = min(q0 + u * nsp, s - 1);
+            xc[u] = M[q * ldm + c];
+            xj[u] = M[q * ldm + j];
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (q0 + u * nsp < s) M[(q0 + u * nsp) * ldm + j] = fma(-w, xc[u], xj[u]);
+        }
+        if (sp == 0) M[c * ldm + j] = fma(-w, rf.d, mj);
+      }
     }
     bar_sync<GT>(bar);
     if (tg == 0) M[c * ldm + c] = rf.beta;
@@ -519,11 +547,21 @@ __device__ __noinline__ void jacobi_warp(double* M, int ldm, int s) {
   }
 }
 
-// Larger orders by a whole group of GT threads: eight lanes per pair, the rows in M (shared or global).
-template <int GT>
-__device__ __noinline__ void jacobi_group(double* M, int ldm, int s, double* nn, unsigned long long* mx, int* flag, int tg, int bar) {
-  const int h = tg & 7, sub = tg >> 3;
-  constexpr int nsub = GT / 8;
+// Larger orders by a whole group of GT threads, the rows in M (shared or global): LP lanes per pair, RL
+// elements a lane in registers (s <= LP RL where they are to hold it all: lanes past s still take FP64 slots,
+// so the caller picks RL by s).
+template <int GT, int LP, int RL, bool SHARED>
+__device__ __noinline__ void jacobi_group(double* M, int ldm, int s, double* nn, unsigned long long* mx, int* flag, int tg,
+                                          int bar) {
+  if (SHARED) __builtin_assume(__isShared(M));
+  __builtin_assume(__isShared(nn));
+  const int h = tg % LP, sub = tg / LP;
+  constexpr int nsub = GT / LP;
+  auto sum = [&](double a) {
+#pragma unroll
+    for (int o = LP / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
+  };
   const int np = (s + 1) & ~1, npairs = np / 2, iters = (npairs + nsub - 1) / nsub;
   const double tol = (double)s * 2.220446049250313e-16, tol2 = tol * tol;
   if (tg == 0) {
@@ -536,10 +574,8 @@ __device__ __noinline__ void jacobi_group(double* M, int ldm, int s, double* nn,
       const int c = c0 + sub;
       double a = 0.0;
       if (c < s)
-        for (int e = h; e < s; e += 8) a = fma(M[c * ldm + e], M[c * ldm + e], a);
-      a += __shfl_xor_sync(0xffffffffu, a, 4);
-      a += __shfl_xor_sync(0xffffffffu, a, 2);
-      a += __shfl_xor_sync(0xffffffffu, a, 1);
+        for (int e = h; e < s; e += LP) a = fma(M[c * ldm + e], M[c * ldm + e], a);
+      a = sum(a);
       if (c < s && h == 0) {
         nn[c] = a;
         atomicMax(&mx[sweep & 1], (unsigned long long)__double_as_longlong(a));
@@ -565,17 +601,31 @@ __device__ __noinline__ void jacobi_group(double* M, int ldm, int s, double* nn,
         const int p = act ? min(a, b) : 0, q = act ? max(a, b) : 0;
         double* mp = M + p * ldm;
         double* mq = M + q * ldm;
-        double apq = 0.0;
-#pragma unroll 8
-        for (int e = h; e < s; e += 8) apq = fma(mp[e], mq[e], apq);
-        apq += __shfl_xor_sync(0xffffffffu, apq, 4);
-        apq += __shfl_xor_sync(0xffffffffu, apq, 2);
-        apq += __shfl_xor_sync(0xffffffffu, apq, 1);
+        // the pair's elements in registers between the product and the rotation (RL a lane; past that only
+        // the first RL stay, the others are read again)
+        double vx[RL], vy[RL], d[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int u = 0; u < RL; ++u) {
+          const int e = h + u * LP;
+          vx[u] = e < s ? mp[e] : 0.0;
+          vy[u] = e < s ? mq[e] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < RL; ++u) d[u & 3] = fma(vx[u], vy[u], d[u & 3]);
+        for (int e = h + RL * LP; e < s; e += LP) d[0] = fma(mp[e], mq[e], d[0]);
+        const double apq = sum((d[0] + d[1]) + (d[2] + d[3]));
         const double app = nn[p], aqq = nn[q];
         const Rotation r = rotation(app, aqq, apq, tol2, floor2);
         if (act && r.rot) {
-#pragma unroll 4
-          for (int e = h; e < s; e += 8) {
+#pragma unroll
+          for (int u = 0; u < RL; ++u) {
+            const int e = h + u * LP;
+            if (e < s) {
+              mp[e] = r.cs * fma(-r.tn, vy[u], vx[u]);
+              mq[e] = r.cs * fma(r.tn, vx[u], vy[u]);
+            }
+          }
+          for (int e = h + RL * LP; e < s; e += LP) {
             const double x = mp[e], y = mq[e];
             mp[e] = r.cs * fma(-r.tn, y, x);
             mq[e] = r.cs * fma(r.tn, x, y);

@@ -54,14 +54,19 @@ long rc_npairs(int k, int nB, int prank, int pworld) {
   return rc_pairs_before(ii0 < mB ? (mB - 1 - ii0) / pworld + 1 : 0, ii0, pworld);
 }
 
-// Pair qq of the rank's trailing pairs: rows ii (i = k + 1 + ii, i % pworld == prank) hold ii pairs each
-// (rows 0..m-1 of the rank C(m) = m ii0 + pworld m (m - 1) / 2); pp = its index among all trailing pairs.
-__device__ __forceinline__ void rc_decode(long qq, long ii0, int pworld, int k, int& i, int& j, long& pp) {
+// Pair qq of the rank's trailing pairs (i, j); pp = its index among all trailing pairs in the order of the
+// rank map (row ii, then jj).  On one rank the pairs come by distance from the diagonal, i - j = 1 first: the
+// ranks fall with it, so the longest pairs start first.  On a block-row partition rows ii (i = k + 1 + ii,
+// i % pworld == prank) hold ii pairs each (rows 0..m-1 of the rank C(m) = m ii0 + pworld m (m - 1) / 2).
+__device__ __forceinline__ void rc_decode(long qq, long npairs, long ii0, int pworld, int k, int mB, int& i, int& j,
+                                          long& pp) {
+  if (pworld == 1) qq = npairs - 1 - qq;
   const double hb = (double)ii0 - 0.5 * pworld;
   long m = (long)((-hb + sqrt(hb * hb + 2.0 * pworld * (double)qq)) / pworld);
   while (m > 0 && rc_pairs_before(m, ii0, pworld) > qq) --m;
   while (rc_pairs_before(m + 1, ii0, pworld) <= qq) ++m;
-  const int ii = (int)(ii0 + m * pworld), jj = (int)(qq - rc_pairs_before(m, ii0, pworld));
+  int ii = (int)(ii0 + m * pworld), jj = (int)(qq - rc_pairs_before(m, ii0, pworld));
+  if (pworld == 1) ii = mB - ii + jj;  // group ii holds the ii pairs at distance mB - ii
   pp = (long)ii * (ii - 1) / 2 + jj;
   i = k + 1 + ii;
   j = k + 1 + jj;
@@ -106,10 +111,11 @@ struct RcPair {
   int i, j, r1, ri, rj;
 };
 
-template <int GW, int NBLK>
+template <int GW, int NBLK, int XU>
 struct RcShared {
   static constexpr int kLdx = Side<GW, NBLK>::kLdx;
-  static constexpr int kXu = 8 * kLdx > kSmall ? 8 * kLdx : kSmall;
+  static constexpr int kXu0 = 8 * kLdx > kSmall ? 8 * kLdx : kSmall;
+  static constexpr int kXu = XU > kXu0 ? XU : kXu0;
   double xu[kXu];                      // U panel for its QR, product parts; then M, GU, GV, Gb
   double xv[8 * kLdx];                 // V panel: reflectors, then Q3 (directly after xu)
   double redv[kRu * GW * 64];          // product parts of the V side
@@ -129,7 +135,7 @@ struct RcShared {
 
 }  // namespace
 
-template <int GW, int NBLK, int MINB>
+template <int GW, int NBLK, int MINB, int XU>
 __global__ void __launch_bounds__(GW * 64, MINB)
     k_recompress(int n, int b, int k, int nB, double* TLR_RESTRICT U, double* TLR_RESTRICT V, int* TLR_RESTRICT rank,
                  int cap, double* TLR_RESTRICT scratch, size_t slot_doubles, int* TLR_RESTRICT next_pair,
@@ -138,7 +144,7 @@ __global__ void __launch_bounds__(GW * 64, MINB)
   using S = Side<GW, NBLK>;
   constexpr int GT = S::GT, LDX = S::kLdx;
   extern __shared__ __align__(16) unsigned char rc_raw[];
-  auto& sm = *reinterpret_cast<RcShared<GW, NBLK>*>(rc_raw);
+  auto& sm = *reinterpret_cast<RcShared<GW, NBLK, XU>*>(rc_raw);
   const EvalParams& prm = *eval_params(status);
   const int rule_fixed = prm.rule_fixed, rmode = prm.rmode;
   const double thr_rel = prm.thr_rel, thr_abs = prm.thr_abs;
@@ -163,7 +169,7 @@ __global__ void __launch_bounds__(GW * 64, MINB)
   auto fetch = [&](long qq, RcPair& out) {
     for (; qq < npairs; qq = (long)gridDim.x + atomicAdd(next_pair, 1)) {
       RcPair p;
-      rc_decode(qq, ii0, pworld, k, p.i, p.j, p.pp);
+      rc_decode(qq, npairs, ii0, pworld, k, nB - k - 1, p.i, p.j, p.pp);
       p.ri = rank[tidx(p.i, k)];
       p.rj = rank[tidx(p.j, k)];
       if (p.ri == 0 || p.rj == 0) continue;
@@ -249,16 +255,42 @@ __global__ void __launch_bounds__(GW * 64, MINB)
 
     const int ldm = s | 1;
     // the core lies over xu (wide pairs: over xu and xv, whose panel is in the scratch slot)
-    double* M = s * ldm <= RcShared<GW, NBLK>::kXu + 8 * LDX ? sm.xu : ws.m;
-    double* GU = fast ? sm.xu + kFs * (kFs + 1) : ws.gu;
-    double* GV = fast ? GU + (kFs + kFlong) * kLdg : ws.gv;
-    double* Gb = fast ? GV + kFs * kLdg : ws.gb;
-    const int ldg = fast ? kLdg : round8(cap);
+    double* M = s * ldm <= RcShared<GW, NBLK, XU>::kXu + 8 * LDX ? sm.xu : ws.m;
 
     // ---- stage 0: the side's panel, block by block: projection, earlier reflector blocks, QR.
     // Stage 1 (V side): Q3 = the QR's Q, a block of columns at a time from the last, then once more
     // against V_ij.  Both are a list of steps x <- x - src coef with coef from the products src^T x, and
     // share one copy of the code.
+    // core M = diag + [C; R2] [D; R3]^T
+    const double *cu = fast ? sm.cr[0] : ws.cru, *cv = fast ? sm.cr[1] : ws.crv;
+    auto form_core = [&](int first, int step) {
+      for (int e = first; e < s * s; e += step) {
+        const int a = e / s, c = e - a * s;
+        const double *ca = cu + (size_t)a * ldq, *cc = cv + (size_t)c * ldq;
+        double a0 = (a == c && a < r1) ? sm.n1[a] * sm.nvv[a] : 0.0, a1 = 0.0;
+        for (int v = 0; v < q; v += 2) {
+          a0 = fma(ca[v], cc[v], a0);
+          if (v + 1 < q) a1 = fma(ca[v + 1], cc[v + 1], a1);
+        }
+        M[a * ldm + c] = a0 + a1;
+      }
+    };
+    // orders past 32: the U group forms the core and its R while the V group forms Q3, then both rotate
+    auto large_core = [&]() {
+      const bool near = M == sm.xu;
+      if (side == 0) {
+        form_core(sd.tg, GT);
+        sd.sync();
+        if (near) group_core_r<GT, true>(M, ldm, s, sd.tg, sd.bar);
+        else group_core_r<GT, false>(M, ldm, s, sd.tg, sd.bar);
+      }
+      bar_sync<2 * GT>(5);
+      constexpr int kLp = MINB == 1 ? 4 : 8;  // one turn per round while the registers hold the rows
+      if (!near) jacobi_group<2 * GT, 8, 16, false>(M, ldm, s, sm.sig, sm.mx, sm.flag, tid, 6);
+      else if (s <= 64) jacobi_group<2 * GT, 8, 8, true>(M, ldm, s, sm.sig, sm.mx, sm.flag, tid, 6);
+      else if (s <= 96) jacobi_group<2 * GT, kLp, 96 / kLp, true>(M, ldm, s, sm.sig, sm.mx, sm.flag, tid, 6);
+      else jacobi_group<2 * GT, kLp, 128 / kLp, true>(M, ldm, s, sm.sig, sm.mx, sm.flag, tid, 6);
+    };
     const bool prod = side == 0 ? short_v : !short_v;  // this side's panel is -P W
 #pragma unroll 1
     for (int stage = 0; stage <= side; ++stage) {
@@ -351,41 +383,31 @@ __global__ void __launch_bounds__(GW * 64, MINB)
     }
 
     if (side == 1) {
+      if (s > 32) large_core();
       bar_sync<2 * GT>(4);  // the rank and the coefficients are in place
     } else {
       bar_sync<2 * GT>(3);
-      // ---- core M = diag + [C; R2] [D; R3]^T, its R, the SVD and the rank
-      const double* cv = fast ? sm.cr[1] : ws.crv;
-      for (int e = sd.tg; e < s * s; e += GT) {
-        const int a = e / s, c = e - a * s;
-        const double *ca = cr + (size_t)a * ldq, *cc = cv + (size_t)c * ldq;
-        double a0 = (a == c && a < r1) ? sm.n1[a] * sm.nvv[a] : 0.0, a1 = 0.0;
-        for (int v = 0; v < q; v += 2) {
-          a0 = fma(ca[v], cc[v], a0);
-          if (v + 1 < q) a1 = fma(ca[v + 1], cc[v + 1], a1);
-        }
-        M[a * ldm + c] = a0 + a1;
-      }
-      sd.sync();
-      if (s <= 32) {
-        if (sd.gw == 0) {
-          if (s <= 8) warp_core_r<8>(M, ldm, s, sm.srt);
-          else if (s <= 16) warp_core_r<16>(M, ldm, s, sm.srt);
-          else if (s <= 24) warp_core_r<24>(M, ldm, s, sm.srt);
-          else warp_core_r<32>(M, ldm, s, sm.srt);
-        }
+      // ---- the core, its R, the SVD and the rank
+      if (s > 32) {
+        large_core();
       } else {
-        group_core_r<GT>(M, ldm, s, sd.tg, sd.bar);
-      }
-      sd.sync();
-      if (s <= 32) {
+        form_core(sd.tg, GT);
+        sd.sync();
         if (sd.gw == 0) {
-          if (s <= 8) jacobi_warp<4, 2>(M, ldm, s);
-          else if (s <= 16) jacobi_warp<4, 4>(M, ldm, s);
-          else jacobi_warp<2, 16>(M, ldm, s);
+          if (s <= 8) {
+            warp_core_r<8>(M, ldm, s, sm.srt);
+            jacobi_warp<4, 2>(M, ldm, s);
+          } else if (s <= 16) {
+            warp_core_r<16>(M, ldm, s, sm.srt);
+            jacobi_warp<4, 4>(M, ldm, s);
+          } else if (s <= 24) {
+            warp_core_r<24>(M, ldm, s, sm.srt);
+            jacobi_warp<2, 16>(M, ldm, s);
+          } else {
+            warp_core_r<32>(M, ldm, s, sm.srt);
+            jacobi_warp<2, 16>(M, ldm, s);
+          }
         }
-      } else {
-        jacobi_group<GT>(M, ldm, s, sm.sig, sm.mx, sm.flag, sd.tg, sd.bar);
       }
       sd.sync();
       for (int c0 = 0; c0 < s; c0 += 8 * GW) {  // singular values: the row norms; sig = their reciprocals
@@ -466,6 +488,12 @@ __global__ void __launch_bounds__(GW * 64, MINB)
     // when X = -U_ik W
     const int rn = sm.rsel;
     if (rn < 0) return;
+    // their arrays: behind the core in shared memory where they fit, else in the scratch slot
+    const int ldg = fast ? kLdg : round8(rn), core = fast ? kFs * (kFs + 1) : (s * ldm + 1) & ~1;
+    const bool near = fast || (M == sm.xu && core + (r1 + ri + s + q) * ldg <= RcShared<GW, NBLK, XU>::kXu + 8 * LDX);
+    double* GU = near ? sm.xu + core : ws.gu;
+    double* GV = near ? GU + (fast ? kFs + kFlong : r1 + ri) * ldg : ws.gv;
+    double* Gb = near ? GV + (fast ? kFs : s) * ldg : ws.gb;
     for (int e = sd.tg; e < s * rn; e += GT) {
       const int kk = e / rn, c = e - kk * rn;
       const int pc = sm.perm[c];
@@ -476,7 +504,7 @@ __global__ void __launch_bounds__(GW * 64, MINB)
       } else if (kk < r1) {
         GU[kk * ldg + c] = vc[kk] * inv * sm.nvv[kk];
       } else {
-        const double* dv = (fast ? sm.cr[1] : ws.crv) + (kk - r1);
+        const double* dv = cv + (kk - r1);
         double a0 = 0.0, a1 = 0.0;
         for (int a = 0; a < s; a += 2) {
           a0 = fma(dv[(size_t)a * ldq], vc[a], a0);
@@ -510,6 +538,7 @@ __global__ void __launch_bounds__(GW * 64, MINB)
       if (rn <= 8) sd.template output<1>(out, b, rn, Q1, r1, co, src2, ld2, n2, m2, co + r1 * ldg, ldg);
       else if (rn <= 16) sd.template output<2>(out, b, rn, Q1, r1, co, src2, ld2, n2, m2, co + r1 * ldg, ldg);
       else if (rn <= 32) sd.template output<4>(out, b, rn, Q1, r1, co, src2, ld2, n2, m2, co + r1 * ldg, ldg);
+      else if (rn <= 64) sd.template output<8>(out, b, rn, Q1, r1, co, src2, ld2, n2, m2, co + r1 * ldg, ldg);
       else sd.template output<16>(out, b, rn, Q1, r1, co, src2, ld2, n2, m2, co + r1 * ldg, ldg);
     }
     if (tid == 0) rank[tij] = rn;
@@ -519,32 +548,46 @@ __global__ void __launch_bounds__(GW * 64, MINB)
 
 namespace {
 
-template <int GW, int NBLK, int MINB>
+template <int GW, int NBLK, int MINB, int XU = 0>
 struct RcShape {
   static constexpr int kPerSm = MINB;
   static size_t slot(int cap) { return wide_slot<Side<GW, NBLK>::kLdx>(nullptr, cap, nullptr); }
   static int launch(int grid, int n, int b, int k, int nB, double* U, double* V, int* rank, int cap, double* scratch,
                     size_t slot_doubles, int* next_pair, int* rlog, int prank, int pworld, long npairs, int* status,
                     cudaStream_t s) {
-    const size_t sm = sizeof(RcShared<GW, NBLK>);
-    cudaFuncSetAttribute(k_recompress<GW, NBLK, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_recompress<GW, NBLK, MINB><<<grid, GW * 64, sm, s>>>(n, b, k, nB, U, V, rank, cap, scratch, slot_doubles, next_pair,
+    const size_t sm = sizeof(RcShared<GW, NBLK, XU>);
+    cudaFuncSetAttribute(k_recompress<GW, NBLK, MINB, XU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_recompress<GW, NBLK, MINB, XU><<<grid, GW * 64, sm, s>>>(n, b, k, nB, U, V, rank, cap, scratch, slot_doubles, next_pair,
                                                            rlog, prank, pworld, npairs, status);
     return (int)cudaGetLastError();
   }
 };
-using Rc128 = RcShape<4, 4, 2>;
-using Rc256 = RcShape<4, 8, 2>;
-using Rc512 = RcShape<4, 16, 2>;
-using Rc1024 = RcShape<8, 16, 1>;
+constexpr int kTallXu = 18496;  // doubles of xu that hold, with xv, a core of order 150
+// calls f with the shape for a tile size and rank capacity
+template <class F>
+auto rc_shape(int b, int cap, F f) {
+  // past the default capacity a plan has met ranks above 64: cores that do not fit beside a second CTA's
+  // shared memory are then what a step waits for (1.8 ms each through L2), so one CTA keeps the SM
+  // (recompression at N = 20,000, range 0.1, ranks to 65: 62 -> 53 ms)
+  if (cap > 64) {
+    if (b <= 128) return f(RcShape<4, 4, 1, kTallXu>{});
+    if (b <= 256) return f(RcShape<4, 8, 1, kTallXu>{});
+    if (b <= 512) return f(RcShape<4, 16, 1, kTallXu>{});
+    return f(RcShape<8, 16, 1>{});
+  }
+  if (b <= 128) return f(RcShape<4, 4, 2>{});
+  if (b <= 256) return f(RcShape<4, 8, 2>{});
+  if (b <= 512) return f(RcShape<4, 16, 2>{});
+  return f(RcShape<8, 16, 1>{});
+}
 
 }  // namespace
 
-int rc_blocks_per_sm(int b) {
-  return b <= 128 ? Rc128::kPerSm : b <= 256 ? Rc256::kPerSm : b <= 512 ? Rc512::kPerSm : Rc1024::kPerSm;
+int rc_blocks_per_sm(int b, int cap) {
+  return rc_shape(b, cap, [](auto shape) { return decltype(shape)::kPerSm; });
 }
 size_t rc_slot_doubles(int b, int cap) {
-  return b <= 128 ? Rc128::slot(cap) : b <= 256 ? Rc256::slot(cap) : b <= 512 ? Rc512::slot(cap) : Rc1024::slot(cap);
+  return rc_shape(b, cap, [&](auto shape) { return shape.slot(cap); });
 }
 
 int launch_recompress(int n, int b, int k, int nB, double* U, double* V, int* rank, int cap, double* scratch,
@@ -553,14 +596,10 @@ int launch_recompress(int n, int b, int k, int nB, double* U, double* V, int* ra
   const long npairs = rc_npairs(k, nB, prank, pworld);
   if (npairs <= 0) return 0;
   const int grid = (int)std::min<long>(npairs, nslots);
-  auto run = [&](auto shape) {
+  return rc_shape(b, cap, [&](auto shape) {
     return shape.launch(grid, n, b, k, nB, U, V, rank, cap, scratch, slot_doubles, next_pair, rlog_step, prank, pworld,
                         npairs, status, s);
-  };
-  if (b <= 128) return run(Rc128{});
-  if (b <= 256) return run(Rc256{});
-  if (b <= 512) return run(Rc512{});
-  return run(Rc1024{});
+  });
 }
 
 }  // namespace tlr
