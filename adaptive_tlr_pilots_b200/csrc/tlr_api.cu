@@ -468,10 +468,9 @@ int run_backward(tlr_plan* p, double sigma2, double inv_range, double eta) {
   const size_t oVp = o; o += B * Rmax;
   const size_t oAl = o; o += (size_t)nB * B;
   const size_t oWk = o; o += B + (size_t)std::max(Rmax, 1);
-  const int nb32 = (b + 31) / 32;
   std::vector<size_t> part_off(nB);
   size_t nparts = 0;
-  for (int m = 0; m < nB; ++m) { part_off[m] = nparts; nparts += (size_t)(nB - m) * nb32 * nb32; }
+  for (int m = 0; m < nB; ++m) { part_off[m] = nparts; nparts += (size_t)(nB - m) * tlr::dtrace_parts(b); }
   const size_t oPart = o; o += 3 * nparts;
   const size_t oGrad = o; o += 4;
   TRY(grow(&p->bw, &p->bw_doubles, o));

@@ -29,79 +29,100 @@ namespace tlr {
 
 // ----------------------------------------------------------------------------------------
 // Batched FP64 GEMM  C = alpha op(A) op(B) + beta C on the FP64 tensor cores (mma m8n8k4, exact
-// FP64 fused multiply-adds).  64 x 64 output tiles, 256 threads: warp w owns rows 32 (w & 1) and
-// columns 16 (w >> 1) of the tile (4 x 2 fragments of 8 x 8).  K advances in slices of 16 through
-// shared memory, double-buffered: the next slice is loaded into registers while the tensor cores
-// work on the current one.  A job may scatter its output columns: column n then goes to ccol[n]
-// (leading rows contiguous) instead of C + n ldc.
-constexpr int kDgP = 72;  // slice row pitch in doubles (fragment reads hit every bank pair twice)
+// FP64 fused multiply-adds).  WM x WN warps of 32 x 8 NJ outputs each (NJ = 4: a k step of four reads eight
+// fragments for sixteen products), K in slices of 16 through three stages of shared memory filled by
+// cp.async (16 bytes where the operand's rows allow, else 8).  A slice keeps the operand's own order:
+// [k][m] when the m index is contiguous in memory, [m][k] when k is; both pitches put a fragment's lanes
+// in distinct banks.  A job may scatter its output columns: column n then goes to ccol[n] (leading rows
+// contiguous) instead of C + n ldc.
+// 128 x 64 tiles (two CTAs an SM) where the launch has two waves of them, 64 x 32 (four warps) where it
+// has not: one 500 x 500 x 500 product is 32 of the large tiles.  Bound by the FP64 tensor pipe (17 cycles
+// a step and scheduler); the backward pass's products at N = 50,000, b = 500: 104 -> 71 ms against 64 x 64
+// tiles staged through registers.
+constexpr int kDgK = 16, kDgStages = 3, kDgPk = kDgK + 4;
+template <int WM, int WN, int NJ>
+struct DgShape {
+  static constexpr int kM = 32 * WM, kN = 8 * NJ * WN, kT = 32 * WM * WN;
+  static constexpr int kPm = kM + 4, kPn = kN + 4;                  // pitches of [k][m], [k][n]; kDgPk of [.][k]
+  static constexpr int kA = kM * kDgPk, kB = kN * kDgPk;            // doubles per stage (the larger layout)
+  static constexpr size_t kSmem = (size_t)kDgStages * (kA + kB) * sizeof(double);
+  static_assert(kA >= kDgK * kPm && kB >= kDgK * kPn, "stage sizes");
+};
+using DgLarge = DgShape<4, 2, 4>;
+using DgSmall = DgShape<2, 2, 2>;
 
-__global__ void __launch_bounds__(256, 3) k_dgemm_batched(const GemmJob* TLR_RESTRICT jobs,
-                                                      const int* TLR_RESTRICT status, int kind) {
-  if (*status != 0) return;
-  const GemmJob jb = jobs[blockIdx.z];
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  if (m0 >= jb.M || n0 >= jb.N) return;
-  __shared__ double As[2][16][kDgP];
-  __shared__ double Bs[2][16][kDgP];
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, int src_bytes) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes) : "memory");
+}
+
+// One operand's slice to shared memory: `rows` x 16 (rows: the m or n index, r0 + row below nr), element
+// (row, k) at src[row ld + k] when kcont, else src[k ld + row].
+template <int ROWS, int THREADS>
+__device__ __forceinline__ void dg_slice(double* dst, const double* src, int ld, bool kcont, bool vec, int r0, int nr,
+                                         int k0, int nk) {
+  constexpr int P = ROWS + 4;
+#pragma unroll
+  for (int e = threadIdx.x; e < ROWS * kDgK / 2; e += THREADS) {
+    const int row = kcont ? e / (kDgK / 2) : 2 * (e % (ROWS / 2)), k = kcont ? 2 * (e % (kDgK / 2)) : e / (ROWS / 2);
+    const int gr = r0 + row, gk = k0 + k;
+    double* d = dst + (kcont ? row * kDgPk + k : k * P + row);
+    const double* g = src + (kcont ? (size_t)gr * ld + gk : (size_t)gk * ld + gr);
+    const int have = gr >= nr || gk >= nk ? 0 : min(2, kcont ? nk - gk : nr - gr);  // elements inside
+    if (vec) {
+      cp_async16(d, have ? g : src, 8 * have);
+    } else {
+      cp_async8(d, have > 0 ? g : src, have > 0 ? 8 : 0);
+      cp_async8(d + 1, have > 1 ? g + 1 : src, have > 1 ? 8 : 0);
+    }
+  }
+}
+
+template <int WM, int WN, int NJ, bool TA, bool TB>
+__device__ __forceinline__ void dgemm_tile(const GemmJob& jb, int m0, int n0, double* sm) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int wm0 = (warp & 1) * 32, wn0 = (warp >> 1) * 16;
-  double ra[4], rb[4];
-  // slice k0 -> registers, coalesced along whichever index is contiguous in memory
-  auto load = [&](int k0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + 256 * q;
-      const int kk = jb.transA ? (e & 15) : (e >> 6), mm = jb.transA ? (e >> 4) : (e & 63);
-      const int gm = m0 + mm, gk = k0 + kk;
-      ra[q] = (gm < jb.M && gk < jb.K) ? (jb.transA ? jb.A[(size_t)gm * jb.lda + gk] : jb.A[(size_t)gk * jb.lda + gm])
-                                       : 0.0;
-      const int kb = jb.transB ? (e >> 6) : (e & 15), nn = jb.transB ? (e & 63) : (e >> 4);
-      const int gn = n0 + nn, gkb = k0 + kb;
-      rb[q] = (gn < jb.N && gkb < jb.K) ? (jb.transB ? jb.B[(size_t)gkb * jb.ldb + gn] : jb.B[(size_t)gn * jb.ldb + gkb])
-                                        : 0.0;
-    }
-  };
-  auto store = [&](int buf) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + 256 * q;
-      const int kk = jb.transA ? (e & 15) : (e >> 6), mm = jb.transA ? (e >> 4) : (e & 63);
-      As[buf][kk][mm] = ra[q];
-      const int kb = jb.transB ? (e >> 6) : (e & 15), nn = jb.transB ? (e & 63) : (e >> 4);
-      Bs[buf][kb][nn] = rb[q];
-    }
-  };
-  double acc[4][2][2];
+  using S = DgShape<WM, WN, NJ>;
+  const int wm0 = (warp % WM) * 32, wn0 = (warp / WM) * 8 * NJ;
+  const bool va = ((reinterpret_cast<size_t>(jb.A) | ((size_t)jb.lda * 8)) & 15) == 0;
+  const bool vb = ((reinterpret_cast<size_t>(jb.B) | ((size_t)jb.ldb * 8)) & 15) == 0;
+  double acc[4][NJ][2];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  if (jb.K > 0) {
-    load(0);
-    store(0);
-  }
-  __syncthreads();
-  for (int k0 = 0, buf = 0; k0 < jb.K; k0 += 16, buf ^= 1) {
-    const bool more = k0 + 16 < jb.K;
-    if (more) load(k0 + 16);
+    for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int nk = (jb.K + kDgK - 1) / kDgK;
+  auto issue = [&](int s) {
+    if (s < nk) {
+      double* st = sm + (size_t)(s % kDgStages) * (S::kA + S::kB);
+      dg_slice<S::kM, S::kT>(st, jb.A, jb.lda, TA, va, m0, jb.M, s * kDgK, jb.K);
+      dg_slice<S::kN, S::kT>(st + S::kA, jb.B, jb.ldb, !TB, vb, n0, jb.N, s * kDgK, jb.K);
+    }
+    cp_async_commit();  // one group per slice, empty past the end
+  };
+  for (int s = 0; s < kDgStages - 1; ++s) issue(s);
+  for (int s = 0; s < nk; ++s) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kDgStages - 2) : "memory");
+    __syncthreads();  // slice s is here, and every warp is done with the stage that the next copy fills
+    issue(s + kDgStages - 1);
+    const double* As = sm + (size_t)(s % kDgStages) * (S::kA + S::kB);
+    const double* Bs = As + S::kA;
 #pragma unroll
-    for (int kq = 0; kq < 4; ++kq) {
-      double a[4], bv[2];
+    for (int kq = 0; kq < kDgK / 4; ++kq) {
+      double a[4], b[NJ];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[buf][4 * kq + t][wm0 + 8 * i + g];
+      for (int i = 0; i < 4; ++i)
+        a[i] = TA ? As[(wm0 + 8 * i + g) * kDgPk + 4 * kq + t] : As[(4 * kq + t) * S::kPm + wm0 + 8 * i + g];
 #pragma unroll
-      for (int j = 0; j < 2; ++j) bv[j] = Bs[buf][4 * kq + t][wn0 + 8 * j + g];
+      for (int j = 0; j < NJ; ++j)
+        b[j] = TB ? Bs[(4 * kq + t) * S::kPn + wn0 + 8 * j + g] : Bs[(wn0 + 8 * j + g) * kDgPk + 4 * kq + t];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 2; ++j) dmma884(acc[i][j][0], acc[i][j][1], a[i], bv[j]);
+        for (int j = 0; j < NJ; ++j) dmma884(acc[i][j][0], acc[i][j][1], a[i], b[j]);
     }
-    if (more) store(buf ^ 1);
-    __syncthreads();
   }
 #pragma unroll
-  for (int j = 0; j < 2; ++j)
+  for (int j = 0; j < NJ; ++j)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int gn = n0 + wn0 + 8 * j + 2 * t + h;
@@ -115,8 +136,27 @@ __global__ void __launch_bounds__(256, 3) k_dgemm_batched(const GemmJob* TLR_RES
         cc[gm] = (jb.beta == 0.0) ? v : fma(jb.beta, cc[gm], v);
       }
     }
-  if (tid == 0) {
-    const int mt = min(64, jb.M - m0), nt = min(64, jb.N - n0);
+}
+
+template <int WM, int WN, int NJ>
+__global__ void __launch_bounds__(32 * WM * WN, 16 / (WM * WN)) k_dgemm_batched(const GemmJob* TLR_RESTRICT jobs,
+                                                                                 const int* TLR_RESTRICT status,
+                                                                                 int kind) {
+  if (*status != 0) return;
+  using S = DgShape<WM, WN, NJ>;
+  const GemmJob jb = jobs[blockIdx.z];
+  const int m0 = blockIdx.y * S::kM, n0 = blockIdx.x * S::kN;
+  if (m0 >= jb.M || n0 >= jb.N) return;
+  extern __shared__ __align__(16) double dg_smem[];
+  if (jb.transA) {
+    if (jb.transB) dgemm_tile<WM, WN, NJ, true, true>(jb, m0, n0, dg_smem);
+    else dgemm_tile<WM, WN, NJ, true, false>(jb, m0, n0, dg_smem);
+  } else {
+    if (jb.transB) dgemm_tile<WM, WN, NJ, false, true>(jb, m0, n0, dg_smem);
+    else dgemm_tile<WM, WN, NJ, false, false>(jb, m0, n0, dg_smem);
+  }
+  if (threadIdx.x == 0) {
+    const int mt = min(S::kM, jb.M - m0), nt = min(S::kN, jb.N - n0);
     add_work(status, kind, 2.0 * jb.K * mt * nt, 8.0 * ((double)mt * nt + (double)(mt + nt) * jb.K));
   }
 }
@@ -124,8 +164,17 @@ __global__ void __launch_bounds__(256, 3) k_dgemm_batched(const GemmJob* TLR_RES
 int launch_dgemm_batched(const GemmJob* jobs, int njobs, int max_m, int max_n, const int* status, int kind,
                          cudaStream_t s) {
   if (njobs <= 0) return 0;
-  dim3 grid((unsigned)((max_n + 63) / 64), (unsigned)((max_m + 63) / 64), (unsigned)njobs);
-  k_dgemm_batched<<<grid, 256, 0, s>>>(jobs, status, kind);
+  auto blocks = [](int n, int per) { return (unsigned)((n + per - 1) / per); };
+  const long large = (long)blocks(max_n, DgLarge::kN) * blocks(max_m, DgLarge::kM) * njobs;
+  if (large >= 4 * 148) {  // two waves of two CTAs an SM
+    cudaFuncSetAttribute(k_dgemm_batched<4, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DgLarge::kSmem);
+    k_dgemm_batched<4, 2, 4><<<dim3(blocks(max_n, DgLarge::kN), blocks(max_m, DgLarge::kM), (unsigned)njobs), DgLarge::kT,
+                               DgLarge::kSmem, s>>>(jobs, status, kind);
+  } else {
+    cudaFuncSetAttribute(k_dgemm_batched<2, 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DgSmall::kSmem);
+    k_dgemm_batched<2, 2, 2><<<dim3(blocks(max_n, DgSmall::kN), blocks(max_m, DgSmall::kM), (unsigned)njobs), DgSmall::kT,
+                               DgSmall::kSmem, s>>>(jobs, status, kind);
+  }
   return (int)cudaGetLastError();
 }
 
@@ -308,77 +357,91 @@ int launch_alpha_step(int n, int b, int m, int nB, const double* U, const double
 
 // ----------------------------------------------------------------------------------------
 // Contraction of dSigma (regenerated) with Sbar = 1/2 (alpha_i alpha_m^T - Z_im) over the tiles
-// (i, m), i >= m, of block column m; weight 2 for off-diagonal tiles.  One CTA per 32 x 32 block;
-// partial sums [3] per CTA into part (fixed slots: deterministic final reduction).
+// (i, m), i >= m, of block column m; weight 2 for off-diagonal tiles.  One CTA per 128 x 32 block, sixteen
+// entries a thread (a column's rows, so Z is read along its columns), then one reduction of the three sums;
+// partial sums [3] per CTA into part (fixed slots: deterministic final reduction).  Bound by the FP64
+// square root and exponential of every entry; N = 50,000: 11.9 -> 9.5 ms per evaluation against four
+// entries a thread and three block sums.
+constexpr int kDtRows = 128, kDtCols = 32;
+
+int dtrace_parts(int b) { return ((b + kDtRows - 1) / kDtRows) * ((b + kDtCols - 1) / kDtCols); }
+
 __global__ void __launch_bounds__(256) k_dtrace_step(const double* TLR_RESTRICT xy, int n, int b, int m, int nB,
                                                     double sigma2, double inv_range, int nu5, double eta,
                                                     const double* TLR_RESTRICT Zbuf,
                                                     const double* TLR_RESTRICT alpha, double* TLR_RESTRICT part,
                                                     const int* TLR_RESTRICT status) {
   if (*status != 0) return;
-  const int nb32 = (b + 31) / 32;
-  const int per_tile = nb32 * nb32;
+  const int ncb = (b + kDtCols - 1) / kDtCols, per_tile = ((b + kDtRows - 1) / kDtRows) * ncb;
   const int i = m + blockIdx.x / per_tile;
   const int blk = blockIdx.x % per_tile;
-  const int rb = blk / nb32, cb = blk % nb32;
+  const int r0 = (blk / ncb) * kDtRows, c0 = (blk % ncb) * kDtCols;
   double* out = part + (size_t)blockIdx.x * 3;
   const int bi = min(b, n - i * b), bm = min(b, n - m * b);
-  const int r0 = rb * 32, c0 = cb * 32;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-  if (r0 < bi && c0 < bm) {
-    const double* Z = Zbuf + (size_t)(i - m) * b * b;  // Z_im, column-major, ld b
-    const double2* p2 = reinterpret_cast<const double2*>(xy);
-    const double* ai = alpha + (size_t)i * b;
-    const double* am = alpha + (size_t)m * b;
-    const int cl = tid & 31, rl = tid >> 5;
-    const int c = c0 + cl;
-    if (c < bm) {
-      const double2 pc = p2[(size_t)m * b + c];
-      const double amc = am[c];
-      for (int q = 0; q < 4; ++q) {
-        const int a = r0 + rl + 8 * q;
-        if (a >= bi) continue;
-        const double2 pa = p2[(size_t)i * b + a];
-        const double dx = pa.x - pc.x, dy = pa.y - pc.y;
-        // dk/d sigma2 = k; dk/d range = sigma2 x^2 e^{-x} / range (nu 3/2) or
-        // sigma2 x^2 (1 + x) e^{-x} / (3 range) (nu 5/2)
-        const double h = sqrt(fmax(dx * dx + dy * dy, 0.0));
-        const double x = (nu5 ? kSqrt5 : kSqrt3) * h * inv_range;
-        const double e = exp(-x);
-        const double sbar = 0.5 * (ai[a] * amc - Z[(size_t)c * b + a]);
-        double ds = (nu5 ? 1.0 + x + x * x / 3.0 : 1.0 + x) * e;
-        const double dr = nu5 ? sigma2 * x * x * (1.0 + x) / 3.0 * e * inv_range : sigma2 * x * x * e * inv_range;
-        double de = 0.0;
-        if (i == m && a == c) {
-          ds += eta;
-          de = sigma2;
-        }
-        g0 = fma(ds, sbar, g0);
-        g1 = fma(dr, sbar, g1);
-        g2 = fma(de, sbar, g2);
+  const double* Z = Zbuf + (size_t)(i - m) * b * b;  // Z_im, column-major, ld b
+  const double2* p2 = reinterpret_cast<const double2*>(xy);
+  // thread: rows r0 + lane + 32 u (u < 4), columns c0 + warp + 8 q (q < 4)
+  double2 pa[4];
+  double aa[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int a = min(r0 + lane + 32 * u, bi - 1);
+    pa[u] = p2[(size_t)i * b + a];
+    aa[u] = alpha[(size_t)i * b + a];
+  }
+  const double cx = nu5 ? kSqrt5 : kSqrt3;
+#pragma unroll
+  for (int q = 0; q < kDtCols / 8; ++q) {
+    const int c = c0 + warp + 8 * q;
+    if (c >= bm) continue;
+    const double2 pc = p2[(size_t)m * b + c];
+    const double amc = alpha[(size_t)m * b + c];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int a = r0 + lane + 32 * u;
+      if (a >= bi) continue;
+      const double dx = pa[u].x - pc.x, dy = pa[u].y - pc.y;
+      // dk/d sigma2 = k; dk/d range = sigma2 x^2 e^{-x} / range (nu 3/2) or
+      // sigma2 x^2 (1 + x) e^{-x} / (3 range) (nu 5/2)
+      const double h = sqrt(fmax(dx * dx + dy * dy, 0.0));
+      const double x = cx * h * inv_range;
+      const double e = exp(-x);
+      const double sbar = 0.5 * (aa[u] * amc - Z[(size_t)c * b + a]);
+      double ds = (nu5 ? 1.0 + x + x * x / 3.0 : 1.0 + x) * e;
+      const double dr = nu5 ? sigma2 * x * x * (1.0 + x) / 3.0 * e * inv_range : sigma2 * x * x * e * inv_range;
+      if (i == m && a == c) {
+        ds += eta;
+        g2 = fma(sigma2, sbar, g2);
       }
+      g0 = fma(ds, sbar, g0);
+      g1 = fma(dr, sbar, g1);
     }
   }
-  __shared__ double red[40];
-  const double w = (i == m) ? 1.0 : 2.0;
-  g0 = block_sum(g0, red);
-  g1 = block_sum(g1, red);
-  g2 = block_sum(g2, red);
-  if (tid == 0) {
-    out[0] = w * g0;
-    out[1] = w * g1;
-    out[2] = w * g2;
+  __shared__ double red[3][8];
+  g0 = warp_sum(g0);
+  g1 = warp_sum(g1);
+  g2 = warp_sum(g2);
+  if (lane == 0) {
+    red[0][warp] = g0;
+    red[1][warp] = g1;
+    red[2][warp] = g2;
+  }
+  __syncthreads();
+  if (tid < 3) {
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s += red[tid][w];
+    out[tid] = (i == m ? 1.0 : 2.0) * s;
   }
 }
 
 int launch_dtrace_step(const double* xy, int n, int b, int m, int nB, double sigma2, double inv_range, int nu5,
                        double eta, const double* Zbuf, const double* alpha, double* part, const int* status,
                        cudaStream_t s) {
-  const int nb32 = (b + 31) / 32;
-  const int ntile = nB - m;
-  k_dtrace_step<<<ntile * nb32 * nb32, 256, 0, s>>>(xy, n, b, m, nB, sigma2, inv_range, nu5, eta, Zbuf, alpha, part,
-                                                    status);
+  k_dtrace_step<<<(nB - m) * dtrace_parts(b), 256, 0, s>>>(xy, n, b, m, nB, sigma2, inv_range, nu5, eta, Zbuf, alpha,
+                                                           part, status);
   return (int)cudaGetLastError();
 }
 

@@ -147,6 +147,7 @@ int launch_copy_cols(const CopyJob* jobs, int njobs, const int* status, cudaStre
 int launch_alpha_step(int n, int b, int m, int nB, const double* U, const double* V, const int* rank, int cap,
                       const double* Li, const double* z, double* alpha, double* work, const int* status,
                       cudaStream_t s);
+int dtrace_parts(int b);  // partial sums (of three) per tile
 int launch_dtrace_step(const double* xy, int n, int b, int m, int nB, double sigma2, double inv_range, int nu5,
                        double eta, const double* Zbuf, const double* alpha, double* part, const int* status,
                        cudaStream_t s);
