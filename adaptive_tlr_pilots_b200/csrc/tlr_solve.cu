@@ -8,10 +8,14 @@
 // launches whatever m.  Column-major N x m operands (ld = N), in place.
 //
 // A solve is one chain through the N rows, so its time is the chain's latency (the products are
-// m N b flops, microseconds).  The inverses of the 32 x 32 diagonal blocks of every L_kk are kept from the
-// factorization, so a panel step is a 32 x 32 by 32 x 8 product and an update of the other rows, both on the FP64 tensor cores with the operands that do not depend on X
-// loaded ahead of the barrier.  Kriging at N = 20,000, b = 500 with 300 sites (two solves of one
-// column, one of 300): 174 -> 10 ms against the substitution with one thread per column.
+// m N b flops, microseconds).  The inverses of the 32 x 32 diagonal blocks of every L_kk are kept from
+// the factorization, so a panel step is a 32 x 32 by 32 x 8 product and an update of the other rows,
+// both on the FP64 tensor cores.  What is left is the wait for L: a panel's first row blocks and its
+// inverse do not depend on X and are loaded while the panel before it updates, and the coupling
+// kernel keeps eight row blocks of a column (four with several column blocks) in flight per warp.
+// Per launch at b = 500, one column: diagonal solve 49 -> 44 us, coupling 26 -> 8.4 us with these loads
+// ahead.  Kriging at N = 20,000, b = 500 with 300 sites (two solves of one column, one of 300):
+// 174 ms with one thread per column by substitution, 10.1 with the inverses, 7.5 with the loads ahead.
 #include "tlr_device.cuh"
 #include "tlr_kernels.h"
 
@@ -83,29 +87,34 @@ __global__ void __launch_bounds__(kSW * 32) k_tri_solve(const double* TLR_RESTRI
     xs[c * ld + r] = (c < nc && r < bk) ? X[(size_t)(c0 + c) * ldx + (size_t)k * b + r] : 0.0;
   }
   __syncthreads();
+  // row blocks of 8 that panel pi leaves to be solved, the next panel's first
+  auto rest = [&](int pi) { return (npk - 1 - pi) * 4; };
+  auto row0 = [&](int p0, int q) { return TRANS ? p0 - 8 - 8 * q : p0 + 32 + 8 * q; };
+  // L[row r0 + g, p0 + 4 kk + t] (or its transpose) for block q of panel pi, zero past the tile's last row
+  auto frag = [&](double (&f)[8], int pi, int q) {
+    const int p0 = (TRANS ? npk - 1 - pi : pi) * 32, r = row0(p0, q) + g;
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) {
+      const int c = p0 + 4 * kk + t;
+      f[kk] = q < rest(pi) && r < bk && c < bk ? (TRANS ? L[(size_t)r * b + c] : L[(size_t)c * b + r]) : 0.0;
+    }
+  };
+  // inv[row 8 (warp % 4) + g][col 4 kk + t] of panel pi, or inv^T
+  auto invfrag = [&](double (&w)[8], int pi) {
+    const double* ip = inv + (size_t)(TRANS ? npk - 1 - pi : pi) * 1024;
+    const int i = 8 * (warp & 3) + g;
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) w[kk] = TRANS ? ip[i * 32 + 4 * kk + t] : ip[(4 * kk + t) * 32 + i];
+  };
+  double f0[8], f1[8], w[8];
+  invfrag(w, 0);
+  frag(f0, 0, warp);
+  frag(f1, 0, warp + kSW);
+#pragma unroll 1
   for (int pi = 0; pi < npk; ++pi) {
-    const int p = TRANS ? npk - 1 - pi : pi, p0 = p * 32;
-    // row blocks of 8 that are still to be solved, the next panel's first
-    const int nrest = TRANS ? p * 4 : (npk - 1 - p) * 4;
-    auto row0 = [&](int q) { return TRANS ? p0 - 8 - 8 * q : p0 + 32 + 8 * q; };
-    // L[row r0 + g, p0 + 4 kk + t] (or its transpose), zero past the tile's last row
-    auto frag = [&](double (&f)[8], int q) {
-      const int r = row0(q) + g;
-#pragma unroll
-      for (int kk = 0; kk < 8; ++kk) {
-        const int c = p0 + 4 * kk + t;
-        f[kk] = q < nrest && r < bk && c < bk ? (TRANS ? L[(size_t)r * b + c] : L[(size_t)c * b + r]) : 0.0;
-      }
-    };
-    double f0[8], f1[8];
-    frag(f0, warp);
-    frag(f1, warp + kSW);
+    const int p0 = (TRANS ? npk - 1 - pi : pi) * 32, nrest = rest(pi);
     if (warp < 4) {  // rows 8 warp .. of X_p
-      const double* ip = inv + (size_t)p * 1024;
-      double w[8], a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};
-#pragma unroll
-      for (int kk = 0; kk < 8; ++kk)  // inv[row 8 warp + g][col 4 kk + t], or inv^T
-        w[kk] = TRANS ? ip[(8 * warp + g) * 32 + 4 * kk + t] : ip[(4 * kk + t) * 32 + 8 * warp + g];
+      double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};
 #pragma unroll
       for (int kk = 0; kk < 8; kk += 2) {
         dmma884(a0[0], a0[1], xs[g * ld + p0 + 4 * kk + t], w[kk]);
@@ -114,6 +123,7 @@ __global__ void __launch_bounds__(kSW * 32) k_tri_solve(const double* TLR_RESTRI
       *reinterpret_cast<double2*>(xp + g * 40 + 8 * warp + 2 * t) = make_double2(a0[0] + a1[0], a0[1] + a1[1]);
     }
     __syncthreads();
+    if (pi + 1 < npk) invfrag(w, pi + 1);  // the next panel's operands come while this one updates
     if (tid < 128) {  // the solved panel back to xs (read again at the end only)
       const int c = tid >> 4, r = 2 * (tid & 15);
       *reinterpret_cast<double2*>(xs + c * ld + p0 + r) = *reinterpret_cast<const double2*>(xp + c * 40 + r);
@@ -121,22 +131,26 @@ __global__ void __launch_bounds__(kSW * 32) k_tri_solve(const double* TLR_RESTRI
     double a[8];
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) a[kk] = -xp[g * 40 + 4 * kk + t];
-    for (int q = warp; q < nrest; q += 2 * kSW) {
-      double g0[8], g1[8];  // the pair after this one
-      frag(g0, q + 2 * kSW);
-      frag(g1, q + 3 * kSW);
+#pragma unroll 1
+    for (int q = warp;; q += 2 * kSW) {
+      const bool more = q + 2 * kSW < nrest;
+      double g0[8], g1[8];  // the pair after this one, or the next panel's first
+      if (more || pi + 1 < npk) {
+        frag(g0, more ? pi : pi + 1, more ? q + 2 * kSW : warp);
+        frag(g1, more ? pi : pi + 1, more ? q + 3 * kSW : warp + kSW);
+      }
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         if (q + u * kSW < nrest) {
-          double2* xr = reinterpret_cast<double2*>(xs + g * ld + row0(q + u * kSW) + 2 * t);
-          double2 v = *xr;
+          double2* xr = reinterpret_cast<double2*>(xs + g * ld + row0(p0, q + u * kSW) + 2 * t);
+          double2 x = *xr;
           double s0 = 0.0, s1 = 0.0;
 #pragma unroll
           for (int kk = 0; kk < 8; kk += 2) {
-            dmma884(v.x, v.y, a[kk], u ? f1[kk] : f0[kk]);
+            dmma884(x.x, x.y, a[kk], u ? f1[kk] : f0[kk]);
             dmma884(s0, s1, a[kk + 1], u ? f1[kk + 1] : f0[kk + 1]);
           }
-          *xr = make_double2(v.x + s0, v.y + s1);
+          *xr = make_double2(x.x + s0, x.y + s1);
         }
       }
 #pragma unroll
@@ -144,6 +158,7 @@ __global__ void __launch_bounds__(kSW * 32) k_tri_solve(const double* TLR_RESTRI
         f0[kk] = g0[kk];
         f1[kk] = g1[kk];
       }
+      if (!more) break;
     }
     __syncthreads();
   }
@@ -175,22 +190,29 @@ __global__ void __launch_bounds__(kSW * 32) k_solve_update(const double* TLR_RES
   // 16-byte row pairs of the factor and of X (whose base comes from the caller)
   const bool alp = (b & 1) == 0, alx = alp && (ldx & 1) == 0 && (reinterpret_cast<size_t>(X) & 15) == 0;
   const double* xk = X + (size_t)k * b;
+  constexpr int kRb = NC == 1 ? 8 : 4;  // row blocks whose loads are in flight together
   for (int u0 = 0; u0 < r; u0 += 8) {
     const double* pc = P + (size_t)min(u0 + g, r - 1) * b;
     double acc[NC][2];
 #pragma unroll
     for (int c = 0; c < NC; ++c) acc[c][0] = acc[c][1] = 0.0;
-#pragma unroll 2
-    for (int row = 8 * warp; row < bk; row += 8 * kSW) {
-      const double2 a = pair_at(pc, row + 2 * t, bk, alp);
-      double2 x[NC];
+#pragma unroll 1
+    for (int row = 8 * warp; row < bk; row += 8 * kSW * kRb) {
+      double2 a[kRb], x[kRb][NC];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) x[c] = pair_at(xk + (size_t)min(c0 + 8 * c + g, m - 1) * ldx, row + 2 * t, bk, alx);
+      for (int p = 0; p < kRb; ++p) {
+        const int rr = row + 8 * kSW * p + 2 * t;
+        a[p] = pair_at(pc, rr, bk, alp);
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        dmma884(acc[c][0], acc[c][1], a.x, x[c].x);
-        dmma884(acc[c][0], acc[c][1], a.y, x[c].y);
+        for (int c = 0; c < NC; ++c) x[p][c] = pair_at(xk + (size_t)min(c0 + 8 * c + g, m - 1) * ldx, rr, bk, alx);
       }
+#pragma unroll
+      for (int p = 0; p < kRb; ++p)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          dmma884(acc[c][0], acc[c][1], a[p].x, x[p][c].x);
+          dmma884(acc[c][0], acc[c][1], a[p].y, x[p][c].y);
+        }
     }
     // the upper warps hand their parts to the lower ones, whose sums are added below
     for (int half = 1; half >= 0; --half) {
@@ -213,31 +235,45 @@ __global__ void __launch_bounds__(kSW * 32) k_solve_update(const double* TLR_RES
     __syncthreads();
   }
   double* xo = X + (size_t)o * b;
-#pragma unroll 2
-  for (int row = 8 * warp; row < bo; row += 8 * kSW) {
-    double acc[NC][2];
+#pragma unroll 1
+  for (int row = 8 * warp; row < bo; row += 8 * kSW * kRb) {
+    double acc[kRb][NC][2];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const double2 v = pair_at(xo + (size_t)min(c0 + 8 * c + g, m - 1) * ldx, row + 2 * t, bo, alx);
-      acc[c][0] = v.x;
-      acc[c][1] = v.y;
-    }
+    for (int p = 0; p < kRb; ++p)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const double2 v =
+            pair_at(xo + (size_t)min(c0 + 8 * c + g, m - 1) * ldx, row + 8 * kSW * p + 2 * t, bo, alx);
+        acc[p][c][0] = v.x;
+        acc[p][c][1] = v.y;
+      }
+#pragma unroll 2
     for (int q0 = 0; q0 < r; q0 += 4) {
       const int u = q0 + t;
-      const double e = (u < r && row + g < bo) ? E[(size_t)u * b + row + g] : 0.0;
+      const double* ec = E + (size_t)min(u, r - 1) * b + g;
+      double e[kRb];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) dmma884(acc[c][0], acc[c][1], u < r ? -T[u][8 * c + g] : 0.0, e);
-    }
+      for (int p = 0; p < kRb; ++p) e[p] = row + 8 * kSW * p + g < bo ? ec[row + 8 * kSW * p] : 0.0;
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      if (c0 + 8 * c + g >= m) continue;
-      double* d = xo + (size_t)(c0 + 8 * c + g) * ldx + row + 2 * t;
-      if (alx && row + 2 * t + 1 < bo) *reinterpret_cast<double2*>(d) = make_double2(acc[c][0], acc[c][1]);
-      else {
-        if (row + 2 * t < bo) d[0] = acc[c][0];
-        if (row + 2 * t + 1 < bo) d[1] = acc[c][1];
+      for (int c = 0; c < NC; ++c) {
+        const double a = u < r ? -T[u][8 * c + g] : 0.0;
+#pragma unroll
+        for (int p = 0; p < kRb; ++p) dmma884(acc[p][c][0], acc[p][c][1], a, e[p]);
       }
     }
+#pragma unroll
+    for (int p = 0; p < kRb; ++p)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        if (c0 + 8 * c + g >= m) continue;
+        const int rr = row + 8 * kSW * p + 2 * t;
+        double* d = xo + (size_t)(c0 + 8 * c + g) * ldx + rr;
+        if (alx && rr + 1 < bo) *reinterpret_cast<double2*>(d) = make_double2(acc[p][c][0], acc[p][c][1]);
+        else {
+          if (rr < bo) d[0] = acc[p][c][0];
+          if (rr + 1 < bo) d[1] = acc[p][c][1];
+        }
+      }
   }
 }
 
