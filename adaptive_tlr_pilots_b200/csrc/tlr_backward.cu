@@ -290,16 +290,7 @@ __global__ void __cluster_dims__(kAC, 1, 1) __launch_bounds__(256)
   const int bm = min(b, n - m * b);
   double* rhs = work;      // b
   double* tq = work + b;   // sum_{i>m} r_im
-  if (tid == 0) {
-    int o = 0;
-    for (int i = m + 1; i < nB; ++i) {
-      off[i - m - 1] = o;
-      o += rank[i * (i - 1) / 2 + m];
-    }
-    off[nB - m - 1] = o;
-  }
-  __syncthreads();
-  const int R = off[nB - m - 1];
+  const int R = block_offsets(off, nB - m - 1, [&](int q) { return rank[(m + 1 + q) * (m + q) / 2 + m]; });
   const int nw = kAC * 8, gw = g * 8 + warp;
   for (int e = gw; e < R; e += nw) {
     int lo = 0, hi = nB - m - 1;  // off[lo] <= e < off[lo + 1]

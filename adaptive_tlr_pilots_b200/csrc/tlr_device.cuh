@@ -43,6 +43,33 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// Exclusive prefix sums of f(0), ..., f(count - 1) into the shared off[0 .. count]; returns the total.
+// Every thread of the block calls it: the values (ranks of a block row or column) are read by all threads
+// at once instead of one after another.
+template <class F>
+__device__ __forceinline__ int block_offsets(int* off, int count, F f) {
+  for (int i = threadIdx.x; i < count; i += blockDim.x) off[i] = f(i);
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int carry = 0;
+    for (int i0 = 0; i0 < count; i0 += 32) {
+      const int v = i0 + lane < count ? off[i0 + lane] : 0;
+      int x = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int w = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += w;
+      }
+      if (i0 + lane < count) off[i0 + lane] = carry + x - v;
+      carry += __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (lane == 0) off[count] = carry;
+  }
+  __syncthreads();
+  return off[count];
+}
+
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));

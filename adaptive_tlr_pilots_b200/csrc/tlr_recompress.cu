@@ -179,10 +179,11 @@ __global__ void __launch_bounds__(GW * 64, MINB)
     }
     out.i = -1;
   };
-  if (blockIdx.x == 0 && tid == 0) {  // the panel column k is read once per step
-    double by = 0.0;
-    for (int i = k + 1; i < nB; ++i) by += 8.0 * 2.0 * b * rank[tidx(i, k)];
-    add_work(status, 10, 0.0, by);
+  if (blockIdx.x == 0 && tid < 32) {  // the panel column k is read once per step
+    int sum = 0;
+    for (int i = k + 1 + tid; i < nB; i += 32) sum += rank[tidx(i, k)];
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (tid == 0) add_work(status, 10, 0.0, 16.0 * b * sum);
   }
   if (tid == GT) fetch(blockIdx.x, sm.pair[0]);
   __syncthreads();
