@@ -135,83 +135,98 @@ __global__ void __launch_bounds__(256, 2) k_diag_build(const double* TLR_RESTRIC
 // then the rows below lose L[., p] X_p, both on the FP64 tensor cores with a column of X as a row of the
 // tiles (lane (g, t): column g, rows 2t and 2t + 1), the factor's operands loaded ahead of the barrier.
 // Then W' = V^T [V, z_k] and [Y, -rhs update] = U W'.  Bound by the chain of panels (two barriers and two
-// short products each); measured per launch at N = 50,000, b = 500: 184 -> 110 us (the tiles of the highest ranks last longest) against a 32-step
-// substitution per panel and column in one thread.
-constexpr int kTsW = 8;     // warps
+// short products each) and, per SM, by reading L from L2.  Sixteen warps, so that the products with U,
+// whose loads wait on L2, have twice the warps in flight.  Per launch at N = 50,000, b = 500: 184 us with a
+// 32-step substitution per panel and column in one thread, 110 with the inverses and eight warps,
+// 90 now; ranks up to 65 at N = 20,000: 15.5 -> 11.1 ms per evaluation against eight warps.
+constexpr int kTsW = 16;    // warps
+constexpr int kTsPitch = 36; // of the solved panel
 constexpr int kTsCols = 32; // columns of V per pass (16 for tiles past 512 rows)
 
-// One pass: NCB blocks of 8 columns in xs (pitch ld, npk panels of 32 rows, zero past bk).
+// One pass: NCB blocks of 8 columns in xs (pitch ld, npk panels of 32 rows, zero past bk).  L is read in
+// blocks of 16 rows, whole 128-byte lines of a column: the lane's two rows 2 g and 2 g + 1 are row g of two
+// products, so that its results are rows 4 t .. 4 t + 3.
 template <int NCB>
 __device__ __forceinline__ void trsm_pass(const double* TLR_RESTRICT L, const double* TLR_RESTRICT inv, int b, int bk,
                                           double* xs, int ld, double* xp) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int npk = (bk + 31) / 32;
-#pragma unroll 1
-  for (int p = 0; p < npk; ++p) {
-    const int p0 = p * 32, nrest = (npk - 1 - p) * 4;  // blocks of 8 rows below
-    auto frag = [&](double (&f)[8], int q) {           // L[p0 + 32 + 8 q + g, p0 + 4 kk + t]
-      const int r = p0 + 32 + 8 * q + g;
+  const bool al = (b & 1) == 0;
+  auto frag = [&](double2 (&f)[8], int p, int q) {  // rows 32 p + 32 + 16 q + 2 g (+ 1), columns 32 p + 4 kk + t
+    const int r = 32 * p + 32 + 16 * q + 2 * g;
+    const bool in = q < 2 * (npk - 1 - p) && r < bk;
+    const double* src = L + (size_t)(32 * p + t) * b + r;
 #pragma unroll
-      for (int kk = 0; kk < 8; ++kk) f[kk] = q < nrest && r < bk ? L[(size_t)(p0 + 4 * kk + t) * b + r] : 0.0;
-    };
-    double f[8], w[8];
-    frag(f, warp);
-    const double* ip = inv + (size_t)p * 1024;
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk) w[kk] = ip[(4 * kk + t) * 32 + 8 * (warp & 3) + g];
-#pragma unroll
-    for (int i = 0; i < (NCB * 4 + kTsW - 1) / kTsW; ++i) {  // rows 8 (warp % 4) of X_p, column block cb
-      const int cb = (warp >> 2) + 2 * i;
-      if (cb < NCB) {
-        const double* xc = xs + (size_t)(8 * cb + g) * ld + p0 + t;
-        double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};
-#pragma unroll
-        for (int kk = 0; kk < 8; kk += 2) {
-          dmma884(a0[0], a0[1], xc[4 * kk], w[kk]);
-          dmma884(a1[0], a1[1], xc[4 * kk + 4], w[kk + 1]);
-        }
-        *reinterpret_cast<double2*>(xp + (8 * cb + g) * 40 + 8 * (warp & 3) + 2 * t) =
-            make_double2(a0[0] + a1[0], a0[1] + a1[1]);
+    for (int kk = 0; kk < 8; ++kk, src += 4 * (size_t)b) {
+      f[kk] = make_double2(0.0, 0.0);
+      if (in) {
+        if (al) f[kk] = *reinterpret_cast<const double2*>(src);
+        else f[kk] = make_double2(src[0], r + 1 < bk ? src[1] : 0.0);
       }
     }
+  };
+  auto invfrag = [&](double (&w)[8], int p) {
+    if ((warp >> 2) >= NCB) return;
+    const double* ip = inv + (size_t)p * 1024 + 8 * (warp & 3) + g;
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) w[kk] = ip[(4 * kk + t) * 32];
+  };
+  double2 f[8];
+  double w[8];
+  invfrag(w, 0);
+  frag(f, 0, warp);
+#pragma unroll 1
+  for (int p = 0; p < npk; ++p) {
+    const int p0 = p * 32, nrest = 2 * (npk - 1 - p);  // blocks of 16 rows below
+    if ((warp >> 2) < NCB) {  // rows 8 (warp % 4) .. of X_p, column block warp / 4
+      const int cb = warp >> 2;
+      const double* xc = xs + (size_t)(8 * cb + g) * ld + p0 + t;
+      double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};
+#pragma unroll
+      for (int kk = 0; kk < 8; kk += 2) {
+        dmma884(a0[0], a0[1], xc[4 * kk], w[kk]);
+        dmma884(a1[0], a1[1], xc[4 * kk + 4], w[kk + 1]);
+      }
+      *reinterpret_cast<double2*>(xp + (8 * cb + g) * kTsPitch + 8 * (warp & 3) + 2 * t) =
+          make_double2(a0[0] + a1[0], a0[1] + a1[1]);
+    }
     __syncthreads();
+    if (p + 1 < npk) invfrag(w, p + 1);  // comes while this panel updates
     for (int e = tid; e < NCB * 128; e += kTsW * 32) {  // the solved panel back to xs (not read again here)
       const int c = e >> 4, r = 2 * (e & 15);
-      *reinterpret_cast<double2*>(xs + (size_t)c * ld + p0 + r) = *reinterpret_cast<const double2*>(xp + c * 40 + r);
+      *reinterpret_cast<double2*>(xs + (size_t)c * ld + p0 + r) =
+          *reinterpret_cast<const double2*>(xp + c * kTsPitch + r);
     }
-    double a[NCB][8];
-#pragma unroll
-    for (int cb = 0; cb < NCB; ++cb)
-#pragma unroll
-      for (int kk = 0; kk < 8; ++kk) a[cb][kk] = -xp[(8 * cb + g) * 40 + 4 * kk + t];
 #pragma unroll 1
-    for (int q = warp; q < nrest; q += kTsW) {
-      double fn[8];  // the block after this one
-      frag(fn, q + kTsW);
-      double2 v[NCB];
+    for (int q = warp; p + 1 < npk; q += kTsW) {
+      const bool more = q + kTsW < nrest;
+      double2 fn[8];  // the block after this one, or the next panel's first
+      frag(fn, more ? p : p + 1, more ? q + kTsW : warp);
+      if (q < nrest) {
+        double2* xr = reinterpret_cast<double2*>(xs + (size_t)g * ld + p0 + 32 + 16 * q + 4 * t);
+        double2 v[NCB][2];
 #pragma unroll
-      for (int cb = 0; cb < NCB; ++cb)
-        v[cb] = *reinterpret_cast<const double2*>(xs + (size_t)(8 * cb + g) * ld + p0 + 32 + 8 * q + 2 * t);
-      if (NCB == 1) {  // one chain would be eight products deep
-        double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-        for (int kk = 0; kk < 8; kk += 2) {
-          dmma884(v[0].x, v[0].y, a[0][kk], f[kk]);
-          dmma884(s0, s1, a[0][kk + 1], f[kk + 1]);
+        for (int cb = 0; cb < NCB; ++cb) {
+          v[cb][0] = xr[cb * 4 * ld];
+          v[cb][1] = xr[cb * 4 * ld + 1];
         }
-        v[0].x += s0;
-        v[0].y += s1;
-      } else {
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
 #pragma unroll
-          for (int cb = 0; cb < NCB; ++cb) dmma884(v[cb].x, v[cb].y, a[cb][kk], f[kk]);
+          for (int cb = 0; cb < NCB; ++cb) {
+            const double a = -xp[(8 * cb + g) * kTsPitch + 4 * kk + t];
+            dmma884(v[cb][0].x, v[cb][1].x, a, f[kk].x);
+            dmma884(v[cb][0].y, v[cb][1].y, a, f[kk].y);
+          }
+#pragma unroll
+        for (int cb = 0; cb < NCB; ++cb) {
+          xr[cb * 4 * ld] = v[cb][0];
+          xr[cb * 4 * ld + 1] = v[cb][1];
+        }
       }
 #pragma unroll
-      for (int cb = 0; cb < NCB; ++cb)
-        *reinterpret_cast<double2*>(xs + (size_t)(8 * cb + g) * ld + p0 + 32 + 8 * q + 2 * t) = v[cb];
-#pragma unroll
       for (int kk = 0; kk < 8; ++kk) f[kk] = fn[kk];
+      if (!more) break;
     }
     __syncthreads();
   }
@@ -239,12 +254,12 @@ __global__ void __launch_bounds__(kTsW * 32)
   if (threadIdx.x == 0) add_work(status, 9, (double)bk * bk * r + 2.0 * bk * r * r + 4.0 * bk * r,
                                  8.0 * ((double)bk * bk * 0.5 + 2.0 * bk * r + bi * r));
   extern __shared__ __align__(16) double xs[];
-  __shared__ __align__(16) double xp[kTsCols * 40];
+  __shared__ __align__(16) double xp[kTsCols * kTsPitch];
   __shared__ double red[kTsW][64];
   __shared__ double Ws[32 * 33];
   __shared__ double zt[128];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int rows = (bk + 31) / 32 * 32, ld = rows + 8;
+  const int rows = (bk + 31) / 32 * 32, ld = rows + 4;
   const bool al = (b & 1) == 0;
   for (int q0 = 0; q0 < r; q0 += cols) {
     const int rq = min(cols, r - q0), ncb = (rq + 7) >> 3, ncx = ncb <= 2 ? ncb : 4;
@@ -606,7 +621,7 @@ int launch_trsm(const double* D, const double* Linv, int n, int b, int k, int nB
                 int pworld, const int* status, cudaStream_t s) {
   if (nB - k - 1 <= 0) return 0;
   const int cols = b <= 512 ? kTsCols : kTsCols / 2;
-  const size_t sm = (size_t)cols * ((b + 31) / 32 * 32 + 8) * sizeof(double);
+  const size_t sm = (size_t)cols * ((b + 31) / 32 * 32 + 4) * sizeof(double);
   cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   k_trsm<<<nB - k - 1, kTsW * 32, sm, s>>>(D, Linv, n, b, k, nB, cols, U, V, Wd, Y, rank, cap, z, rhs, prec, blog_trsm,
                                            prank, pworld, status);

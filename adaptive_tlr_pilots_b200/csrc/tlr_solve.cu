@@ -10,12 +10,12 @@
 // A solve is one chain through the N rows, so its time is the chain's latency (the products are
 // m N b flops, microseconds).  The inverses of the 32 x 32 diagonal blocks of every L_kk are kept from
 // the factorization, so a panel step is a 32 x 32 by 32 x 8 product and an update of the other rows,
-// both on the FP64 tensor cores.  What is left is the wait for L: a panel's first row blocks and its
-// inverse do not depend on X and are loaded while the panel before it updates, and the coupling
-// kernel keeps eight row blocks of a column (four with several column blocks) in flight per warp.
-// Per launch at b = 500, one column: diagonal solve 49 -> 44 us, coupling 26 -> 8.4 us with these loads
-// ahead.  Kriging at N = 20,000, b = 500 with 300 sites (two solves of one column, one of 300):
-// 174 ms with one thread per column by substitution, 10.1 with the inverses, 7.5 with the loads ahead.
+// both on the FP64 tensor cores.  What is left is the wait for L: the registers of a row block are
+// loaded with the next panel's as soon as they are used (16-byte loads, whole lines of a column), and the
+// coupling kernel keeps eight row blocks of a column (four with several column blocks) in flight per warp.
+// Per launch at b = 500, one column: diagonal solve 49 -> 33 us (L) and 43 -> 37 us (L^T), coupling
+// 26 -> 8.4 us against loads next to their use.  Kriging at N = 20,000, b = 500 with 300 sites (two solves
+// of one column, one of 300): 174 ms with one thread per column by substitution, 6.6 ms now.
 #include "tlr_device.cuh"
 #include "tlr_kernels.h"
 
@@ -79,37 +79,86 @@ __global__ void __launch_bounds__(kSW * 32) k_tri_solve(const double* TLR_RESTRI
   const double* L = D + (size_t)k * b * b;
   inv += (size_t)k * np * 1024;
   extern __shared__ __align__(16) double xs[];  // kSC columns, pitch ld: disjoint banks for the fragments
-  __shared__ __align__(16) double xp[kSC * 40];
-  const int ld = npk * 32 + 8;
+  constexpr int kXpPitch = TRANS ? 40 : 36;  // likewise
+  __shared__ __align__(16) double xp[kSC * kXpPitch];
+  const int ld = npk * 32 + (TRANS ? 8 : 4);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   for (int e = tid; e < npk * 32 * kSC; e += kSW * 32) {
     const int r = e % (npk * 32), c = e / (npk * 32);
     xs[c * ld + r] = (c < nc && r < bk) ? X[(size_t)(c0 + c) * ldx + (size_t)k * b + r] : 0.0;
   }
   __syncthreads();
-  // row blocks of 8 that panel pi leaves to be solved, the next panel's first
-  auto rest = [&](int pi) { return (npk - 1 - pi) * 4; };
-  auto row0 = [&](int p0, int q) { return TRANS ? p0 - 8 - 8 * q : p0 + 32 + 8 * q; };
-  // L[row r0 + g, p0 + 4 kk + t] (or its transpose) for block q of panel pi, zero past the tile's last row
-  auto frag = [&](double (&f)[8], int pi, int q) {
-    const int p0 = (TRANS ? npk - 1 - pi : pi) * 32, r = row0(p0, q) + g;
+  const bool al = (b & 1) == 0;
+  // row blocks of 16 that panel pi leaves to be solved, the next panel's first
+  auto rest = [&](int pi) { return (npk - 1 - pi) * 2; };
+  auto row0 = [&](int p0, int q) { return TRANS ? p0 - 16 - 16 * q : p0 + 32 + 16 * q; };
+  // Block q of panel pi, zero past the tile's last row.  L: rows r0 + 2 g (+ 1) of column p0 + 4 kk + t, row g of
+  // two products.  L^T: columns r0 + g and r0 + 8 + g, rows p0 + 8 kk + 2 t (+ 1), the t of two steps.
+  auto frag = [&](double2 (&f)[8], int pi, int q) {
+    const int p0 = (TRANS ? npk - 1 - pi : pi) * 32, r0 = row0(p0, q);
+    if (q >= rest(pi)) return;
+    const double* src = L + (size_t)(TRANS ? r0 + g : p0 + t) * b + (TRANS ? p0 : r0 + 2 * g) + (TRANS ? 2 * t : 0);
+    const size_t sb = b;
+    if (al && (TRANS ? p0 + 32 : r0 + 16) <= bk) {  // no branch or predicate per load
 #pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-      const int c = p0 + 4 * kk + t;
-      f[kk] = q < rest(pi) && r < bk && c < bk ? (TRANS ? L[(size_t)r * b + c] : L[(size_t)c * b + r]) : 0.0;
+      for (int kk = 0; kk < 8; ++kk)
+        f[kk] = *reinterpret_cast<const double2*>(src + (TRANS ? 8 * sb * (kk >> 2) + 8 * (kk & 3) : 4 * sb * kk));
+    } else {
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) {
+        const int row = TRANS ? p0 + 8 * (kk & 3) + 2 * t : r0 + 2 * g;
+        const double* e = src + (TRANS ? 8 * sb * (kk >> 2) + 8 * (kk & 3) : 4 * sb * kk);
+        f[kk].x = row < bk ? e[0] : 0.0;
+        f[kk].y = row + 1 < bk ? e[1] : 0.0;
+      }
     }
   };
   // inv[row 8 (warp % 4) + g][col 4 kk + t] of panel pi, or inv^T
   auto invfrag = [&](double (&w)[8], int pi) {
+    if (warp >= 4) return;
     const double* ip = inv + (size_t)(TRANS ? npk - 1 - pi : pi) * 1024;
     const int i = 8 * (warp & 3) + g;
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) w[kk] = TRANS ? ip[i * 32 + 4 * kk + t] : ip[(4 * kk + t) * 32 + i];
   };
-  double f0[8], f1[8], w[8];
+  auto update = [&](const double2 (&f)[8], int pi, int q) {
+    const int r0 = row0((TRANS ? npk - 1 - pi : pi) * 32, q);
+    const double* xc = xp + g * kXpPitch;
+    if (TRANS) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        double2* xr = reinterpret_cast<double2*>(xs + g * ld + r0 + 8 * h + 2 * t);
+        double2 x = *xr;
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          const double2 a = *reinterpret_cast<const double2*>(xc + 8 * kk + 2 * t);
+          dmma884(x.x, x.y, -a.x, f[4 * h + kk].x);
+          dmma884(s0, s1, -a.y, f[4 * h + kk].y);
+        }
+        *xr = make_double2(x.x + s0, x.y + s1);
+      }
+    } else {
+      double2* xr = reinterpret_cast<double2*>(xs + g * ld + r0 + 4 * t);
+      double2 v0 = xr[0], v1 = xr[1];
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) {
+        const double a = -xc[4 * kk + t];
+        dmma884(v0.x, v1.x, a, f[kk].x);
+        dmma884(v0.y, v1.y, a, f[kk].y);
+      }
+      xr[0] = v0;
+      xr[1] = v1;
+    }
+  };
+  // The registers of a block are loaded with the next panel's as soon as they are used: a load has the
+  // rest of the panel and the next panel's solve to come in.
+  constexpr int kHeld = 4;  // blocks per warp: tiles of 512 rows
+  double2 f[kHeld][8];
+  double w[8];
   invfrag(w, 0);
-  frag(f0, 0, warp);
-  frag(f1, 0, warp + kSW);
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u) frag(f[u], 0, warp + u * kSW);
 #pragma unroll 1
   for (int pi = 0; pi < npk; ++pi) {
     const int p0 = (TRANS ? npk - 1 - pi : pi) * 32, nrest = rest(pi);
@@ -120,45 +169,26 @@ __global__ void __launch_bounds__(kSW * 32) k_tri_solve(const double* TLR_RESTRI
         dmma884(a0[0], a0[1], xs[g * ld + p0 + 4 * kk + t], w[kk]);
         dmma884(a1[0], a1[1], xs[g * ld + p0 + 4 * kk + 4 + t], w[kk + 1]);
       }
-      *reinterpret_cast<double2*>(xp + g * 40 + 8 * warp + 2 * t) = make_double2(a0[0] + a1[0], a0[1] + a1[1]);
+      *reinterpret_cast<double2*>(xp + g * kXpPitch + 8 * warp + 2 * t) = make_double2(a0[0] + a1[0], a0[1] + a1[1]);
     }
+    if (pi + 1 < npk) invfrag(w, pi + 1);
     __syncthreads();
-    if (pi + 1 < npk) invfrag(w, pi + 1);  // the next panel's operands come while this one updates
     if (tid < 128) {  // the solved panel back to xs (read again at the end only)
       const int c = tid >> 4, r = 2 * (tid & 15);
-      *reinterpret_cast<double2*>(xs + c * ld + p0 + r) = *reinterpret_cast<const double2*>(xp + c * 40 + r);
+      *reinterpret_cast<double2*>(xs + c * ld + p0 + r) = *reinterpret_cast<const double2*>(xp + c * kXpPitch + r);
     }
-    double a[8];
 #pragma unroll
-    for (int kk = 0; kk < 8; ++kk) a[kk] = -xp[g * 40 + 4 * kk + t];
+    for (int u = 0; u < kHeld; ++u) {
+      const int q = warp + u * kSW;
+      if (q < nrest) update(f[u], pi, q);
+      if (u == 0) {
 #pragma unroll 1
-    for (int q = warp;; q += 2 * kSW) {
-      const bool more = q + 2 * kSW < nrest;
-      double g0[8], g1[8];  // the pair after this one, or the next panel's first
-      if (more || pi + 1 < npk) {
-        frag(g0, more ? pi : pi + 1, more ? q + 2 * kSW : warp);
-        frag(g1, more ? pi : pi + 1, more ? q + 3 * kSW : warp + kSW);
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        if (q + u * kSW < nrest) {
-          double2* xr = reinterpret_cast<double2*>(xs + g * ld + row0(p0, q + u * kSW) + 2 * t);
-          double2 x = *xr;
-          double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-          for (int kk = 0; kk < 8; kk += 2) {
-            dmma884(x.x, x.y, a[kk], u ? f1[kk] : f0[kk]);
-            dmma884(s0, s1, a[kk + 1], u ? f1[kk + 1] : f0[kk + 1]);
-          }
-          *xr = make_double2(x.x + s0, x.y + s1);
+        for (int e = warp + kHeld * kSW; e < nrest; e += kSW) {  // tiles past 512 rows
+          frag(f[0], pi, e);
+          update(f[0], pi, e);
         }
       }
-#pragma unroll
-      for (int kk = 0; kk < 8; ++kk) {
-        f0[kk] = g0[kk];
-        f1[kk] = g1[kk];
-      }
-      if (!more) break;
+      frag(f[u], pi + 1, q);  // nothing past the last panel
     }
     __syncthreads();
   }
