@@ -27,6 +27,10 @@
 // Panels wider than 8 columns go through the same steps block by block (blocked Householder: the
 // reflector blocks are applied as I - V T V^T), with the arrays that do not fit in shared memory in
 // the CTA's slot of global scratch (L2).
+//
+// Recompression per FP64 evaluation, against one group of 256 threads per pair with a column at a time in
+// shared memory: N = 1,030, b = 100 3.7 -> 0.77 ms; N = 10,007, b = 250 17.9 -> 4.7; N = 50,000, b = 500
+// 138 -> 44.7; N = 20,000, b = 500, range 0.1 (ranks to 65) 382 -> 53.
 #include "tlr_kernels.h"
 #include "tlr_panel.cuh"
 
@@ -564,9 +568,11 @@ struct RcShape {
   }
 };
 constexpr int kTallXu = 18496;  // doubles of xu that hold, with xv, a core of order 150
-// calls f with the shape for a tile size and rank capacity
+constexpr int kFewPairs = 148;  // one per SM
+// calls f with the shape for a tile size, a rank capacity and whether the step has at most kFewPairs pairs
+// (all shapes of a tile size have the same rows, so the same scratch slots)
 template <class F>
-auto rc_shape(int b, int cap, F f) {
+auto rc_shape(int b, int cap, bool few, F f) {
   // past the default capacity a plan has met ranks above 64: cores that do not fit beside a second CTA's
   // shared memory are then what a step waits for (1.8 ms each through L2), so one CTA keeps the SM
   // (recompression at N = 20,000, range 0.1, ranks to 65: 62 -> 53 ms)
@@ -575,6 +581,14 @@ auto rc_shape(int b, int cap, F f) {
     if (b <= 256) return f(RcShape<4, 8, 1, kTallXu>{});
     if (b <= 512) return f(RcShape<4, 16, 1, kTallXu>{});
     return f(RcShape<8, 16, 1>{});
+  }
+  // No second CTA to share the SM with: all its registers to one (255 a thread, no spills).  Recompression
+  // per evaluation: N = 1,030, b = 100 0.83 -> 0.77 ms, N = 4,000, b = 250 1.93 -> 1.68, N = 4,000, b = 203
+  // 2.94 -> 2.56; sixteen warps in its place 0.83, 1.84, 2.78.
+  if (few) {
+    if (b <= 128) return f(RcShape<4, 4, 1>{});
+    if (b <= 256) return f(RcShape<4, 8, 1>{});
+    if (b <= 512) return f(RcShape<4, 16, 1>{});
   }
   if (b <= 128) return f(RcShape<4, 4, 2>{});
   if (b <= 256) return f(RcShape<4, 8, 2>{});
@@ -585,10 +599,10 @@ auto rc_shape(int b, int cap, F f) {
 }  // namespace
 
 int rc_blocks_per_sm(int b, int cap) {
-  return rc_shape(b, cap, [](auto shape) { return decltype(shape)::kPerSm; });
+  return rc_shape(b, cap, false, [](auto shape) { return decltype(shape)::kPerSm; });
 }
 size_t rc_slot_doubles(int b, int cap) {
-  return rc_shape(b, cap, [&](auto shape) { return shape.slot(cap); });
+  return rc_shape(b, cap, false, [&](auto shape) { return shape.slot(cap); });
 }
 
 int launch_recompress(int n, int b, int k, int nB, double* U, double* V, int* rank, int cap, double* scratch,
@@ -597,7 +611,8 @@ int launch_recompress(int n, int b, int k, int nB, double* U, double* V, int* ra
   const long npairs = rc_npairs(k, nB, prank, pworld);
   if (npairs <= 0) return 0;
   const int grid = (int)std::min<long>(npairs, nslots);
-  return rc_shape(b, cap, [&](auto shape) {
+  const long m = nB - k - 1;  // all ranks' pairs, so that a partitioned step takes the same shape
+  return rc_shape(b, cap, m * (m - 1) / 2 <= kFewPairs, [&](auto shape) {
     return shape.launch(grid, n, b, k, nB, U, V, rank, cap, scratch, slot_doubles, next_pair, rlog_step, prank, pworld,
                         npairs, status, s);
   });

@@ -2,7 +2,8 @@
 in the diagonal factorization and the panel solve (31, 32, 33), the cluster sizes of the diagonal
 factorization (256, 257), the column budget of the panel solve (512 and above), the sketch's row tiles
 (319, 320, 321), odd tile sizes (unpaired loads), ranks past 32 in the panel solve and past 64 in the
-recompression (the plan's columns grow), and a last tile of a few sites.
+recompression (the plan's columns grow), steps with more and with fewer pairs than SMs, and a last tile of a
+few sites.
 
 Against the NumPy oracle: identical ranks; log-likelihood within 1e-9 relative (FP64 rounding times the
 conditioning that the parity fixtures show, 1e-10, and a margin of ten).  The GEMM at its larger tile
@@ -26,6 +27,8 @@ CASES = [  # (n, b, theta, rule, value)
     (770, 256, (1.0, 0.1, 0.005), "fixed", 1e-6),
     (775, 257, (1.0, 0.1, 0.005), "fixed", 1e-6),
     (2400, 600, (1.0, 0.05, 0.002), "fixed", 1e-6),
+    (2080, 100, (1.0, 0.3, 0.05), "adaptive", 0.9),   # 190, 171, ... pairs: both sides of one per SM
+    (3990, 200, (1.0, 0.2, 0.05), "adaptive", 0.9),
 ]
 
 
