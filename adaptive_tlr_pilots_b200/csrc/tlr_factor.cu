@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(256, 2) k_diag_build(const double* TLR_RESTRIC
 // short products each) and, per SM, by reading L from L2.  Sixteen warps, so that the products with U,
 // whose loads wait on L2, have twice the warps in flight.  Per launch at N = 50,000, b = 500: 184 us with a
 // 32-step substitution per panel and column in one thread, 110 with the inverses and eight warps,
-// 90 now; ranks up to 65 at N = 20,000: 15.5 -> 11.1 ms per evaluation against eight warps.
+// 90 now; ranks up to 65 at N = 20,000: 15.5 -> 10.7 ms per evaluation against eight warps.
 constexpr int kTsW = 16;    // warps
 constexpr int kTsPitch = 36; // of the solved panel
 constexpr int kTsCols = 32; // columns of V per pass (16 for tiles past 512 rows)
@@ -203,25 +203,19 @@ __device__ __forceinline__ void trsm_pass(const double* TLR_RESTRICT L, const do
       double2 fn[8];  // the block after this one, or the next panel's first
       frag(fn, more ? p : p + 1, more ? q + kTsW : warp);
       if (q < nrest) {
-        double2* xr = reinterpret_cast<double2*>(xs + (size_t)g * ld + p0 + 32 + 16 * q + 4 * t);
-        double2 v[NCB][2];
-#pragma unroll
+#pragma unroll 1  // the blocks at once would spill (11.1 against 10.7 ms)
         for (int cb = 0; cb < NCB; ++cb) {
-          v[cb][0] = xr[cb * 4 * ld];
-          v[cb][1] = xr[cb * 4 * ld + 1];
-        }
+          double2* xr = reinterpret_cast<double2*>(xs + (size_t)(8 * cb + g) * ld + p0 + 32 + 16 * q + 4 * t);
+          const double* xc = xp + (8 * cb + g) * kTsPitch + t;
+          double2 v0 = xr[0], v1 = xr[1];
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-#pragma unroll
-          for (int cb = 0; cb < NCB; ++cb) {
-            const double a = -xp[(8 * cb + g) * kTsPitch + 4 * kk + t];
-            dmma884(v[cb][0].x, v[cb][1].x, a, f[kk].x);
-            dmma884(v[cb][0].y, v[cb][1].y, a, f[kk].y);
+          for (int kk = 0; kk < 8; ++kk) {
+            const double a = -xc[4 * kk];
+            dmma884(v0.x, v1.x, a, f[kk].x);
+            dmma884(v0.y, v1.y, a, f[kk].y);
           }
-#pragma unroll
-        for (int cb = 0; cb < NCB; ++cb) {
-          xr[cb * 4 * ld] = v[cb][0];
-          xr[cb * 4 * ld + 1] = v[cb][1];
+          xr[0] = v0;
+          xr[1] = v1;
         }
       }
 #pragma unroll
