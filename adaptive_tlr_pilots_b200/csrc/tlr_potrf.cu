@@ -128,20 +128,22 @@ __global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(256)
   if (tid == 0) go = (g == 0) ? (*status == 0) : 0;
   cluster.sync();
   const int ok = *cluster.map_shared_rank(&go, 0);
-  cluster.sync();  // rank 0's shared memory stays valid until every CTA has read it
-  if (!ok) return;
   const int bk = min(b, n - k * b);
   double* A = D + (size_t)k * b * b;
-  double* rk = rhs + (size_t)k * b;
-  const bool al = (b & 1) == 0;
-  if (g == 0 && tid == 0) add_work(status, 8, (double)bk * bk * bk / 3.0 + (double)bk * bk, 8.0 * bk * bk);
   double row[kPB];  // warp 0: the current diagonal block; row warps: a row below it
-  double ldacc = 0.0, qacc = 0.0;
-  if (warp == 0) {
+  if (warp == 0) {  // every CTA reads the first diagonal block: CTA 0 writes L_11 over it past the barrier
     const int pw = min(kPB, bk);
 #pragma unroll
     for (int j = 0; j < kPB; ++j)
       row[j] = (lane < pw && j <= lane) ? __ldcg(A + (size_t)j * b + lane) : (j == lane ? 1.0 : 0.0);
+  }
+  cluster.sync();  // and rank 0's shared memory stays valid until every CTA has read it
+  if (!ok) return;
+  double* rk = rhs + (size_t)k * b;
+  const bool al = (b & 1) == 0;
+  if (g == 0 && tid == 0) add_work(status, 8, (double)bk * bk * bk / 3.0 + (double)bk * bk, 8.0 * bk * bk);
+  double ldacc = 0.0, qacc = 0.0;
+  if (warp == 0) {
     const int bad = factor_block(row, Lc[0], dinv[0]);
     if (lane == 0) fail[0] = bad;
   }
