@@ -10,7 +10,10 @@
 // else is kept off it:
 //   * every CTA keeps the chain to itself: warp 1 solves the 32 rows below the diagonal block, warp 0
 //     updates the next diagonal block with them and factors it (redundantly: identical inputs give
-//     identical results, so no broadcast, and a non-positive pivot stops every CTA at the same panel);
+//     identical results, so no broadcast, and a non-positive pivot stops every CTA at the same panel).
+//     The inputs are identical because CTA 0 writes what every CTA has read (the first diagonal block,
+//     those 32 rows) only past a cluster barrier that follows the reads; within the panel the solved
+//     rows come from each CTA's own copy in shared memory;
 //   * the other rows are dealt out to the cluster and solved by substitution in registers, a thread
 //     per row, with the tile's right-hand side as one more row (z_p); then rhs_rows -= X z_p (the fused
 //     forward solve);
@@ -118,7 +121,8 @@ __global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(256)
   cg::cluster_group cluster = cg::this_cluster();
   const int g = (int)cluster.block_rank();
   __shared__ __align__(16) double Lc[2][kPB * kPL];
-  __shared__ __align__(16) double Cs[kPB * kPL];  // the 32 solved rows, then the next diagonal block
+  __shared__ __align__(16) double X0[kPB * kPL];  // the 32 solved rows below the diagonal block
+  __shared__ __align__(16) double Cs[kPB * kPL];  // the next diagonal block
   __shared__ double dinv[2][kPB], dinv2[kPB];
   __shared__ double zp[kPB];
   __shared__ int go, fail[2];
@@ -178,9 +182,8 @@ __global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(256)
       } else {
         if (warp == 1) {
 #pragma unroll
-          for (int q = 0; q < kPB; ++q) Cs[q * kPL + lane] = row[q];
-        }
-        if (act && (warp > 1 || g == 0)) {
+          for (int q = 0; q < kPB; ++q) X0[q * kPL + lane] = row[q];  // to the tile past the barrier
+        } else if (act) {
 #pragma unroll
           for (int q = 0; q < kPB; ++q)
             if (q < pw) __stcg(P + (size_t)q * b + r, row[q]);
@@ -233,7 +236,7 @@ __global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(256)
             acc[nj][mi][h] = (q < pn && c <= q) ? __ldcg(T + (size_t)c * b + q) : 0.0;
           }
       double f[8][4];
-      panel_frag<4>(f, Cs, kPL, kPB, 0);
+      panel_frag<4>(f, X0, kPL, kPB, 0);
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk)
 #pragma unroll
@@ -290,7 +293,8 @@ __global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(256)
         if (!waited) cluster.barrier_wait();  // the panel is final
         waited = true;
         double fa[8][2], fb[8][4];
-        panel_frag<2>(fa, P, b, m, c0);
+        if (cb == 0) panel_frag<2>(fa, X0, kPL, kPB, c0);
+        else panel_frag<2>(fa, P, b, m, c0);
         panel_frag<4>(fb, P, b, m, r0);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
@@ -316,6 +320,11 @@ __global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(256)
           }
       }
       if (!waited) cluster.barrier_wait();
+      if (rhs_warp && g == 0 && lane < m) {  // every CTA has read these rows
+#pragma unroll
+        for (int q = 0; q < kPB; ++q)
+          if (q < pw) __stcg(P + (size_t)q * b + lane, X0[q * kPL + lane]);
+      }
     }
     cluster.sync();  // the trailing matrix and the next diagonal block's factor are in place
   }

@@ -49,7 +49,7 @@ def exe(tmp_path_factory):
     return host_cuda.build(tmp_path_factory.mktemp("potrf"), MAIN)
 
 
-@pytest.mark.parametrize("G,b", [(4, 30), (8, 32)])
+@pytest.mark.parametrize("G,b", [(4, 30), (8, 32), (4, 70), (4, 129), (8, 161)])
 def test_cluster_order_leaves_the_bits(exe, G, b):
     first = host_cuda.run(exe, G, b, 1, 0, 0)
     assert first.startswith("0 "), first[:200]
