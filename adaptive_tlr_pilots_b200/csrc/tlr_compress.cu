@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(GW * 32, 16 / GW) k_orth(double* TLR_RESTRICT 
                                                           int tile_base, const int* TLR_RESTRICT tj,
                                                           const int* TLR_RESTRICT need, double* TLR_RESTRICT gscratch,
                                                           size_t slot, int in_smem, const int* TLR_RESTRICT status) {
-  if (*status != 0) return;
+  if (cta_failed(status)) return;
   const int c = blockIdx.x;
   if (!need[c]) return;
   constexpr int kLdx = Side<GW, NBLK>::kLdx;
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(GW * 32, 16 / GW)
                int nblk, double* TLR_RESTRICT gscratch, size_t slot, double* TLR_RESTRICT gsv, double* TLR_RESTRICT Uo,
                double* TLR_RESTRICT Vo, int* TLR_RESTRICT rank, int last_level, int in_smem, int* TLR_RESTRICT rlog,
                double* TLR_RESTRICT tail0, double* TLR_RESTRICT fro0, int* TLR_RESTRICT blog, int* TLR_RESTRICT status) {
-  if (*status != 0) return;
+  if (cta_failed(status)) return;
   const EvalParams& prm = *eval_params(status);
   const int rule_fixed = prm.rule_fixed, rmode = prm.rmode, round_store = prm.round_store;
   const double thr_rel = prm.thr_rel, thr_abs = prm.thr_abs;

@@ -92,6 +92,11 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   return red[32];
 }
 
+// Whether the evaluation has failed, with one answer for the whole CTA.  The status word may be written while a
+// CTA's threads read it (POTRF beside the recompression, other CTAs of the same launch); a kernel whose
+// barriers count all its threads, or whose threads wait for what one of them claims, must leave as a whole.
+__device__ __forceinline__ bool cta_failed(const int* status) { return __syncthreads_or(*status != 0) != 0; }
+
 // ---------------------------------------------------------------- work counters
 // The plan's control block: int status, three ints of padding, then [flops, bytes] doubles per
 // kernel kind (algorithmic counts, accumulated by the kernels for the roofline report).

@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(kGcT, kGcBlocks)
                          int* TLR_RESTRICT rank, int cap, double* TLR_RESTRICT scratch, size_t slot_doubles,
                          int* TLR_RESTRICT next_pair, int* TLR_RESTRICT rlog, int* TLR_RESTRICT blog,
                          int* TLR_RESTRICT status) {
-  if (*status != 0) return;
+  if (cta_failed(status)) return;
   const EvalParams& prm = *eval_params(status);
   const int rule_fixed = prm.rule_fixed, rmode = prm.rmode;
   const double thr_rel = prm.thr_rel, thr_abs = prm.thr_abs;

@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(GW * 64, MINB)
     k_recompress(int n, int b, int k, int nB, double* TLR_RESTRICT U, double* TLR_RESTRICT V, int* TLR_RESTRICT rank,
                  int cap, double* TLR_RESTRICT scratch, size_t slot_doubles, int* TLR_RESTRICT next_pair,
                  int* TLR_RESTRICT rlog, int prank, int pworld, long npairs, int* TLR_RESTRICT status) {
-  if (*status != 0) return;
+  if (cta_failed(status)) return;
   using S = Side<GW, NBLK>;
   constexpr int GT = S::GT, LDX = S::kLdx;
   extern __shared__ __align__(16) unsigned char rc_raw[];

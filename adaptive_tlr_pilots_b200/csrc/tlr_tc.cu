@@ -207,7 +207,7 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
 __global__ void __launch_bounds__(kTcThreads, 2) k_gemm_tc3(const GemmJob* TLR_RESTRICT jobs,
                                                  const TcOperands* TLR_RESTRICT ops, int* TLR_RESTRICT status,
                                                  int kind) {
-  if (*status != 0) return;
+  if (cta_failed(status)) return;
   const GemmJob jb = jobs[blockIdx.z];
   const int m0 = blockIdx.y * kTcM, n0 = blockIdx.x * kTcN;
   if (m0 >= jb.M || n0 >= jb.N) return;
