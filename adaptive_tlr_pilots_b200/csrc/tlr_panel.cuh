@@ -615,6 +615,7 @@ __device__ __noinline__ void jacobi_group(double* M, int ldm, int s, double* nn,
         for (int e = h + RL * LP; e < s; e += LP) d[0] = fma(mp[e], mq[e], d[0]);
         const double apq = sum((d[0] + d[1]) + (d[2] + d[3]));
         const double app = nn[p], aqq = nn[q];
+        __syncwarp();  // every lane of the pair has the norms that lane h = 0 replaces below
         const Rotation r = rotation(app, aqq, apq, tol2, floor2);
         if (act && r.rot) {
 #pragma unroll

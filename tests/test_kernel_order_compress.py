@@ -1,7 +1,7 @@
 """k_orth and k_finalize on the host (emu/cuda_emu.h) under every order of their threads: two covariance tiles (one
-ragged) at sketch widths with the reflectors in shared memory and in global scratch, and with the
-core in one warp.  The bits do not depend on the order; the basis is orthonormal and the pair meets the rule;
-and a status word that another CTA sets while a CTA's threads read it ends the CTA as a whole."""
+ragged) at sketch widths with the reflectors in shared memory and in global scratch, and with cores
+of one warp and of the whole CTA.  The bits do not depend on the order; the basis is orthonormal and the pair
+meets the rule; and a status word that another CTA sets while a CTA's threads read it ends the CTA as a whole."""
 import pytest
 
 import host_cuda
@@ -121,7 +121,7 @@ def _check(out):
     assert 0 < int(w[5]) <= int(w[6]) < 16
 
 
-@pytest.mark.parametrize("b,k,in_smem", [(24, 16, 1), (33, 32, 1), (70, 32, 0)])
+@pytest.mark.parametrize("b,k,in_smem", [(24, 16, 1), (33, 32, 1), (70, 32, 0), (40, 64, 0), (70, 64, 0)])
 def test_thread_order_leaves_the_bits(exe, b, k, in_smem):
     first = host_cuda.run(exe, b, k, in_smem, 1, 1, 0, 0, -1, -1)
     _check(first)

@@ -1,5 +1,5 @@
 """k_recompress and k_recompress_general on the host (emu/cuda_emu.h) under every order of their threads: one
-factorization step of three trailing pairs, with panels of one block of columns and of several.  The bits do
+factorization step of three trailing pairs, with panels of one block of columns and of several, and cores past order 32.  The bits do
 not depend on the order; the updated tile is U V^T - U_ik V_ik^T V_jk U_jk^T up to the rule's threshold; and a
 status word that another kernel sets while a CTA's threads read it ends the CTA as a whole."""
 import pytest
@@ -128,8 +128,8 @@ def exe(tmp_path_factory):
     return host_cuda.build(tmp_path_factory.mktemp("recompress"), MAIN)
 
 
-# (kernel, b, rank, cap): narrow panels; ragged odd tiles; two panel blocks
-@pytest.mark.parametrize("general,b,rank,cap", [(0, 24, 5, 64), (0, 33, 8, 64), (0, 40, 13, 64), (1, 24, 5, 64)])
+# (kernel, b, rank, cap): narrow panels; ragged odd tiles; two panel blocks; cores past order 32
+@pytest.mark.parametrize("general,b,rank,cap", [(0, 24, 5, 64), (0, 33, 8, 64), (0, 40, 13, 64), (0, 48, 22, 64), (1, 24, 5, 64)])
 def test_thread_order_leaves_the_bits(exe, general, b, rank, cap):
     first = host_cuda.run(exe, general, b, rank, cap, 1, 0, 0, -1)
     assert first.startswith("error ") and float(first.split()[1]) <= 1e-7, first[:200]
