@@ -12,6 +12,18 @@ constexpr int kRu = 3;  // blocks of 8 columns per reduction of a product
 // H = I - kappa v v^T, v = (d; the entries below), H maps the column to beta at the pivot (the dlarfg
 // sign).  v is left unscaled, kappa = 1 / (nrm (nrm + |alpha|)), so one division follows the square
 // root (an FP64 step costs about 23 cycles of latency here, a square root 120, a division 77).
+// The squared norm alpha^2 + sig2 has to lie within 2^-500 .. 2^500: past that kappa and the products with v
+// would leave the range of a double (kappa is infinite for norms below 7e-155, and the columns of T^T T P
+// are squares of a tile's entries).  A column outside is first multiplied by column_lift, a power of two, which
+// changes no bit of the reflector; beta is divided by it.
+__device__ __forceinline__ double column_lift(double norm2) {
+  constexpr int kLow = (1023 - 500) << 20, kHigh = (1023 + 500) << 20;  // high words of 2^-500, 2^500
+  if ((unsigned)(__double2hiint(norm2) - kLow) <= (unsigned)(kHigh - kLow) || norm2 == 0.0) return 1.0;
+  return norm2 < 1.0 ? 0x1p500 : 0x1p-500;
+}
+__device__ __forceinline__ double unlift(double lift, double v) {
+  return lift == 1.0 ? v : v * (lift > 1.0 ? 0x1p-500 : 0x1p500);
+}
 struct Reflector {
   double beta, d, kappa;
 };
@@ -236,8 +248,9 @@ struct Side {
     // one body for every column (the code of a pair runs once per pair, so its size is instruction
     // fetches): the current column is y[.][0], the panel rotates by one column a step, and position j
     // holds column (j + c) mod 8
+    double lift = 1.0;
 #pragma unroll 1
-    for (int c = 0; c < nc; ++c) {
+    for (int c = 0, step = 0; c < nc; ++step) {
       const int piv = r0 + c, live = 8 - c;  // positions from `live` on: finished reflectors
       double p[8], xc[kRpt];
 #pragma unroll
@@ -267,7 +280,7 @@ struct Side {
       }
       q1 += __shfl_xor_sync(0xffffffffu, q1, 2);
       q1 += __shfl_xor_sync(0xffffffffu, q1, 1);
-      double* rb = qred + (c & 1) * (8 * GW + 8);
+      double* rb = qred + (step & 1) * (8 * GW + 8);
       if ((lane & 3) == 0) rb[gw * 8 + (lane >> 4) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = q1;
       if (tg == piv) {
 #pragma unroll
@@ -284,6 +297,15 @@ struct Side {
       for (int w = 1; w < GW; ++w)
 #pragma unroll
         for (int j = 0; j < 8; ++j) s[j] += rb[w * 8 + j];
+      if (lift == 1.0) {
+        lift = column_lift(fma(pv[0], pv[0], s[0]));
+        if (lift != 1.0) {  // the same in every thread: the rows from the pivot on, and the sums once more
+#pragma unroll
+          for (int i = 0; i < kRpt; ++i)
+            if (tg + GT * i >= piv) y[i][0] *= lift;
+          continue;
+        }
+      }
       const Reflector rf = reflector(pv[0], s[0]);
 #pragma unroll
       for (int j = 1; j < 8; ++j) {
@@ -301,11 +323,13 @@ struct Side {
 #pragma unroll
       for (int i = 0; i < kRpt; ++i) {
         double y0 = y[i][0];
-        if (i == 0 && tg == piv) y0 = rf.beta;
+        if (i == 0 && tg == piv) y0 = unlift(lift, rf.beta);
 #pragma unroll
         for (int j = 0; j < 7; ++j) y[i][j] = y[i][j + 1];
         y[i][7] = y0;
       }
+      lift = 1.0;
+      ++c;
     }
     if (tg < nrow) {
 #pragma unroll
@@ -359,21 +383,32 @@ __device__ __noinline__ void warp_core_r(double* M, int ldm, int s, double* buf)
       for (int i = 0; i < NR; i += 2) *reinterpret_cast<double2*>(xb + i) = make_double2(m[i], m[i + 1]);
     }
     __syncwarp();
-    double x[NR], sa[4] = {0.0, 0.0, 0.0, 0.0}, da[4] = {0.0, 0.0, 0.0, 0.0};
+    double x[NR], sig2, dt, lift = 1.0;
 #pragma unroll
     for (int i = 0; i < NR; i += 2) {
       const double2 v = *reinterpret_cast<const double2*>(xb + i);
       x[i] = v.x;
       x[i + 1] = v.y;
     }
+#pragma unroll 1
+    for (;;) {
+      double sa[4] = {0.0, 0.0, 0.0, 0.0}, da[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for (int i = 1; i < NR; ++i) {
-      sa[i & 3] = fma(x[i], x[i], sa[i & 3]);
-      da[i & 3] = fma(x[i], m[i], da[i & 3]);
+      for (int i = 1; i < NR; ++i) {
+        sa[i & 3] = fma(x[i], x[i], sa[i & 3]);
+        da[i & 3] = fma(x[i], m[i], da[i & 3]);
+      }
+      sig2 = (sa[0] + sa[1]) + (sa[2] + sa[3]);
+      dt = (da[0] + da[1]) + (da[2] + da[3]);
+      if (lift != 1.0) break;
+      lift = column_lift(fma(x[0], x[0], sig2));
+      if (lift == 1.0) break;
+#pragma unroll
+      for (int i = 0; i < NR; ++i) x[i] *= lift;
     }
-    const Reflector rf = reflector(x[0], (sa[0] + sa[1]) + (sa[2] + sa[3]));
-    const double w = rf.kappa * fma(rf.d, m[0], (da[0] + da[1]) + (da[2] + da[3]));
-    if (j < s) M[c * ldm + j] = j < c ? 0.0 : (j == c ? rf.beta : fma(-w, rf.d, m[0]));
+    const Reflector rf = reflector(x[0], sig2);
+    const double w = rf.kappa * fma(rf.d, m[0], dt);
+    if (j < s) M[c * ldm + j] = j < c ? 0.0 : (j == c ? unlift(lift, rf.beta) : fma(-w, rf.d, m[0]));
 #pragma unroll
     for (int i = 1; i < NR; ++i) m[i - 1] = fma(-w, x[i], m[i]);
     m[NR - 1] = 0.0;
@@ -387,17 +422,28 @@ __device__ __noinline__ void group_core_r(double* M, int ldm, int s, int tg, int
   if (SHARED) __builtin_assume(__isShared(M));
   const int nsp = s <= GT / 4 ? 4 : s <= GT / 2 ? 2 : 1, sp = tg % nsp;
   for (int c = 0; c < s - 1; ++c) {
-    double sg[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int r0 = c + 1 + sp; r0 < s; r0 += 8 * nsp) {
-      double x[8];
+    double sig2, alpha = M[c * ldm + c], lift = 1.0;
+#pragma unroll 1
+    for (;;) {
+      double sg[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int r0 = c + 1 + sp; r0 < s; r0 += 8 * nsp) {
+        double x[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) x[u] = r0 + u * nsp < s ? M[(r0 + u * nsp) * ldm + c] : 0.0;
+        for (int u = 0; u < 8; ++u) x[u] = r0 + u * nsp < s ? M[(r0 + u * nsp) * ldm + c] : 0.0;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) sg[u & 3] = fma(x[u], x[u], sg[u & 3]);
+        for (int u = 0; u < 8; ++u) sg[u & 3] = fma(x[u], x[u], sg[u & 3]);
+      }
+      sig2 = (sg[0] + sg[1]) + (sg[2] + sg[3]);
+      for (int o = 1; o < nsp; o <<= 1) sig2 += __shfl_xor_sync(0xffffffffu, sig2, o);
+      if (lift != 1.0) break;
+      lift = column_lift(fma(alpha, alpha, sig2));
+      if (lift == 1.0) break;
+      bar_sync<GT>(bar);  // the same in every thread: the column below the pivot is the reflector's alone
+      for (int r = c + 1 + tg; r < s; r += GT) M[r * ldm + c] *= lift;
+      alpha *= lift;
+      bar_sync<GT>(bar);
     }
-    double sig2 = (sg[0] + sg[1]) + (sg[2] + sg[3]);
-    for (int o = 1; o < nsp; o <<= 1) sig2 += __shfl_xor_sync(0xffffffffu, sig2, o);
-    const Reflector rf = reflector(M[c * ldm + c], sig2);
+    const Reflector rf = reflector(alpha, sig2);
     const int step = GT / nsp;
     for (int j0 = c + 1; j0 < s; j0 += step) {  // the same trip count in every thread (shuffles)
       const int j = j0 + tg / nsp, jc = min(j, s - 1);
@@ -435,7 +481,7 @@ __device__ __noinline__ void group_core_r(double* M, int ldm, int s, int tg, int
       }
     }
     bar_sync<GT>(bar);
-    if (tg == 0) M[c * ldm + c] = rf.beta;
+    if (tg == 0) M[c * ldm + c] = unlift(lift, rf.beta);
   }
   bar_sync<GT>(bar);
   for (int e = tg; e < s * s; e += GT) {

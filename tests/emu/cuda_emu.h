@@ -377,6 +377,7 @@ inline long long __double_as_longlong(double x) {
   memcpy(&r, &x, 8);
   return r;
 }
+inline int __double2hiint(double x) { return (int)(__double_as_longlong(x) >> 32); }
 inline double __longlong_as_double(long long x) {
   double r;
   memcpy(&r, &x, 8);

@@ -98,7 +98,8 @@ int main(int argc, char** argv) {
         for (int q = 0; q < rank[c]; ++q) e -= U[((size_t)c * cap + q) * b + a] / scale * V[((size_t)c * cap + q) * b + w];
         e2 += e * e;
       }
-    worst = std::max(worst, sqrt(e2) * scale / fro[c]);
+    worst = std::max(worst, sqrt(e2) * (scale / fro[c]));
+    if (!(e2 >= 0.0)) worst = 9.0;
   }
   printf("error %.17g orth %.17g ranks %d %d\n", worst, orth, rank[0], rank[1]);
   for (int c = 0; c < nc; ++c)
@@ -133,3 +134,11 @@ def test_thread_order_leaves_the_bits(exe, b, k, in_smem):
 @pytest.mark.parametrize("orth,finalize", [(32, -1), (96, -1), (-1, 32), (-1, 96), (-1, 160)])
 def test_status_set_while_a_cta_reads_it(exe, thread, orth, finalize):
     assert host_cuda.run(exe, 24, 16, 1, 1, 1, 0, thread, orth, finalize, timeout=60) == "status 3\n"
+
+
+@pytest.mark.parametrize("k,in_smem", [(16, 1), (32, 1), (64, 0)])
+@pytest.mark.parametrize("scale", [1e-62, 1e-68, 1e-72, 1e70])
+def test_tiles_of_any_size(exe, k, in_smem, scale):
+    """The columns of T^T T P are squares of the tile's entries, and their norms are squared once more: the basis
+    and the pair are those of a tile of ordinary size."""
+    _check(host_cuda.run(exe, 48, k, in_smem, scale, 1, 0, 0, -1, -1))

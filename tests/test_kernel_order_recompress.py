@@ -12,7 +12,7 @@ MAIN = r"""
 #include "tlr_factor.cu"
 #undef tidx
 using namespace tlr;
-// usage: main general b rank cap seed cta_order thread_order flip_after
+// usage: main general b rank cap seed cta_order thread_order flip_after [fall scale]
 int main(int argc, char** argv) {
   const int general = atoi(argv[1]), b = atoi(argv[2]), r = atoi(argv[3]), cap = atoi(argv[4]);
   emu::Config cfg;
@@ -21,6 +21,7 @@ int main(int argc, char** argv) {
   cfg.thread = (emu::Order)atoi(argv[7]);
   cfg.flip_after = atoi(argv[8]);
   cfg.flip_value = 3;
+  const double fall = argc > 9 ? atof(argv[9]) : 0.6, scale = argc > 10 ? atof(argv[10]) : 1.0;
   const int nB = 4, n = 3 * b + b / 2, ntiles = 6;  // the last tile is ragged
   std::vector<char> ctl(kControlBytes, 0);
   int* status = reinterpret_cast<int*>(ctl.data());
@@ -34,33 +35,33 @@ int main(int argc, char** argv) {
   std::vector<double> U((size_t)ntiles * b * cap, 0.0), V(U);
   std::vector<int> rank(ntiles);
   // orthogonal columns of falling norm in U, orthonormal ones in V
-  auto columns = [&](double* X, int rows, int cols, double fall) {
-    double s = 1.0;
-    for (int c = 0; c < cols; ++c, s *= fall) {
+  auto columns = [&](double* X, int rows, int cols, double s, double fall) {
+    for (int c = 0; c < cols; ++c) {
       double* x = X + (size_t)c * b;
       for (int a = 0; a < rows; ++a) x[a] = u(rng);
-      for (int pass = 0; pass < 2; ++pass)
-        for (int d = 0; d < c; ++d) {
+      for (int pass = 0; pass < 3; ++pass) {
+        for (int d = 0; d < c && pass < 2; ++d) {
           const double* y = X + (size_t)d * b;
-          double dot = 0.0, nn = 0.0;
-          for (int a = 0; a < rows; ++a) {
-            dot += x[a] * y[a];
-            nn += y[a] * y[a];
-          }
-          for (int a = 0; a < rows; ++a) x[a] -= dot / nn * y[a];
+          double dot = 0.0;
+          for (int a = 0; a < rows; ++a) dot += x[a] * y[a];
+          for (int a = 0; a < rows; ++a) x[a] -= dot * y[a];
         }
-      double nn = 0.0;
-      for (int a = 0; a < rows; ++a) nn += x[a] * x[a];
-      for (int a = 0; a < rows; ++a) x[a] *= s / sqrt(nn);
+        double nn = 0.0;
+        for (int a = 0; a < rows; ++a) nn += x[a] * x[a];
+        for (int a = 0; a < rows; ++a) x[a] /= sqrt(nn);
+      }
     }
+    for (int c = 0; c < cols; ++c, s *= fall)
+      for (int a = 0; a < rows; ++a) X[(size_t)c * b + a] *= s;
   };
   auto id = [](int i, int j) { return i * (i - 1) / 2 + j; };
   for (int i = 1; i < nB; ++i)
     for (int j = 0; j < i; ++j) {
-      const int t = id(i, j), rt = std::min(std::max(r - (i - j), 1), i == 3 ? b / 2 : b);
+      const int t = id(i, j), rt = std::min(r - (i + j) % 3, i == 3 ? b / 2 : b);
       rank[t] = rt;
-      columns(&U[(size_t)t * b * cap], i == 3 ? b / 2 : b, rt, 0.6);
-      columns(&V[(size_t)t * b * cap], b, rt, 1.0);
+      // scaled: the updated tiles and the factor of their update that is not U_ik's side
+      columns(&U[(size_t)t * b * cap], i == 3 ? b / 2 : b, rt, j > 0 || i == 1 ? scale : 1.0, j > 0 || i == 1 ? fall : 0.6);
+      columns(&V[(size_t)t * b * cap], b, rt, 1.0, 1.0);
     }
   auto tile = [&](const std::vector<double>& A, const std::vector<double>& B, int t, int rt) {
     std::vector<double> M((size_t)b * b, 0.0);
@@ -105,13 +106,14 @@ int main(int argc, char** argv) {
   }
   double worst = 0.0;
   for (auto& [t, M] : want) {
+    if (scale != 1.0 && t != id(2, 1) && t != id(3, 1)) continue;  // U_jk of j = 2 is of ordinary size
     const auto G = tile(U, V, t, rank[t]);
     double e = 0.0, f = 0.0;
     for (size_t q = 0; q < M.size(); ++q) {
-      e += (G[q] - M[q]) * (G[q] - M[q]);
-      f += M[q] * M[q];
+      e += (G[q] - M[q]) / scale * ((G[q] - M[q]) / scale);
+      f += M[q] / scale * (M[q] / scale);
     }
-    worst = std::max(worst, sqrt(e / f));
+    worst = std::max(worst, e >= 0.0 ? sqrt(e / f) : 9.0);
   }
   printf("error %.17g\n", worst);
   for (int t = 0; t < ntiles; ++t) {
@@ -142,3 +144,10 @@ def test_thread_order_leaves_the_bits(exe, general, b, rank, cap):
 @pytest.mark.parametrize("after", [64, 128, 224])
 def test_status_set_while_a_cta_reads_it(exe, general, thread, after):
     assert host_cuda.run(exe, general, 24, 5, 64, 1, 0, thread, after, timeout=60) == "status 3\n"
+
+
+@pytest.mark.parametrize("b,rank,fall,scale", [(24, 6, 1e-20, 1e-75), (40, 14, 1e-8, 1e-60), (48, 23, 3e-5, 1e-60)])
+def test_columns_far_below_the_first(exe, b, rank, fall, scale):
+    """Columns down to 1e-155, whose squared norms are below the smallest double that has a reciprocal."""
+    out = host_cuda.run(exe, 0, b, rank, 64, 1, 0, 0, -1, fall, scale)
+    assert out.startswith("error ") and float(out.split()[1]) <= 1e-7, out[:200]
