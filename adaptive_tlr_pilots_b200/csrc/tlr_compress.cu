@@ -23,6 +23,7 @@
 namespace tlr {
 
 constexpr int kMaxSketch = 128;  // widest sketch level
+constexpr double kCoreFloor = 1e-200;  // of the squared row norms in the Jacobi SVD
 __host__ __device__ inline int tile_pitch(int b) { return (b + 1) & ~1; }  // 16-byte rows of the generated tiles
 
 __device__ __forceinline__ double omega_entry(uint32_t tile, uint32_t row, uint32_t col) {
@@ -518,12 +519,12 @@ __global__ void __launch_bounds__(GW * 32, 16 / GW)
   sd.sync();
   if (k <= 32) {
     if (warp == 0) {
-      if (k <= 16) jacobi_warp<4, 4>(M, ldm, k);
-      else jacobi_warp<2, 16>(M, ldm, k);
+      if (k <= 16) jacobi_warp<4, 4>(M, ldm, k, kCoreFloor);
+      else jacobi_warp<2, 16>(M, ldm, k, kCoreFloor);
     }
   } else {
-    if (k <= 64) jacobi_group<GT, 8, 8, true>(M, ldm, k, nn, mx, flag, tid, 1);
-    else jacobi_group<GT, 8, 16, true>(M, ldm, k, nn, mx, flag, tid, 1);
+    if (k <= 64) jacobi_group<GT, 8, 8, true>(M, ldm, k, kCoreFloor, nn, mx, flag, tid, 1);
+    else jacobi_group<GT, 8, 16, true>(M, ldm, k, kCoreFloor, nn, mx, flag, tid, 1);
   }
   sd.sync();
   for (int q0 = 0; q0 < k; q0 += GT / 4) {  // singular values: the row norms

@@ -492,8 +492,10 @@ __device__ __noinline__ void group_core_r(double* M, int ldm, int s, int tg, int
 }
 
 // One-sided Jacobi on the rows of the s x s row-major M: on return the rows are mutually orthogonal.
-// Round-robin ordering.  A pair (p, q) is rotated unless |cos| <= s eps, or a row lies below 1e-14 of the
-// largest norm (the rounding noise of the projections).  The squared row norms are fresh at the start
+// Round-robin ordering.  A pair (p, q) is rotated unless |cos| <= s eps, or a row's squared norm lies below
+// floor_rel times the largest: 1e-28 in the recompression (the rounding noise of the projections), 1e-200 in the
+// initial compression, whose small rows carry right vectors that have to be orthonormal as well (what is
+// left out there only keeps the angle's quotients within the range of a double).  The squared row norms are fresh at the start
 // of a sweep and updated by the rotation formulas.  A sweep in which every cos and every tan stayed
 // below 3e-9 is the last: what it leaves is of the order of their squares.
 //
@@ -529,7 +531,7 @@ __device__ __forceinline__ Rotation rotation(double app, double aqq, double apq,
 // the rows move between the lane groups by shuffles after every round (the circle method), so a round
 // is one chain without shared memory or barriers: 450 cycles at LP = 4, RL = 4, 710 at LP = 2, RL = 16.
 template <int LP, int RL>
-__device__ __noinline__ void jacobi_warp(double* M, int ldm, int s) {
+__device__ __noinline__ void jacobi_warp(double* M, int ldm, int s, double floor_rel) {
   const int lane = threadIdx.x & 31, grp = lane / LP, h = lane % LP;
   const int np = (s + 1) & ~1, m = np / 2, ry = np - 1 - grp;
   const bool first = grp == 0, last = grp == m - 1;
@@ -556,7 +558,7 @@ __device__ __noinline__ void jacobi_warp(double* M, int ldm, int s) {
     }
     nx = sum(nx);
     ny = sum(ny);
-    if (sweep == 0) floor2 = 1e-28 * warp_max(fmax(nx, ny));
+    if (sweep == 0) floor2 = floor_rel * warp_max(fmax(nx, ny));
     bool big = false;
 #pragma unroll 1
     for (int round = 0; round < np - 1; ++round) {
@@ -597,8 +599,8 @@ __device__ __noinline__ void jacobi_warp(double* M, int ldm, int s) {
 // elements a lane in registers (s <= LP RL where they are to hold it all: lanes past s still take FP64 slots,
 // so the caller picks RL by s).
 template <int GT, int LP, int RL, bool SHARED>
-__device__ __noinline__ void jacobi_group(double* M, int ldm, int s, double* nn, unsigned long long* mx, int* flag, int tg,
-                                          int bar) {
+__device__ __noinline__ void jacobi_group(double* M, int ldm, int s, double floor_rel, double* nn, unsigned long long* mx,
+                                          int* flag, int tg, int bar) {
   if (SHARED) __builtin_assume(__isShared(M));
   __builtin_assume(__isShared(nn));
   const int h = tg % LP, sub = tg / LP;
@@ -632,7 +634,7 @@ __device__ __noinline__ void jacobi_group(double* M, int ldm, int s, double* nn,
       flag[(sweep + 1) & 1] = 0;
       mx[(sweep + 1) & 1] = 0ull;
     }
-    const double floor2 = 1e-28 * __longlong_as_double((long long)mx[sweep & 1]);
+    const double floor2 = floor_rel * __longlong_as_double((long long)mx[sweep & 1]);
 #pragma unroll 1
     for (int round = 0; round < np - 1; ++round) {
 #pragma unroll 1

@@ -42,6 +42,7 @@ constexpr int kFs = 32;      // largest core order kept in shared memory whole (
 constexpr int kFlong = 24;   // largest long side of W kept in shared memory
 constexpr int kLdq = 9;      // row pitch of the shared [C; R] arrays
 constexpr int kLdg = 32;     // row pitch of the shared G arrays
+constexpr double kFloor = 1e-28;  // rows of a core below 1e-14 of its largest are rounding noise
 constexpr int kSmall = kFs * (kFs + 1) + (kFs + kFlong) * kLdg + kFs * kLdg + 8 * kLdg;  // M, GU, GV, Gb
 
 __device__ __forceinline__ int tidx(int i, int j) { return i * (i - 1) / 2 + j; }
@@ -291,10 +292,10 @@ __global__ void __launch_bounds__(GW * 64, MINB)
       }
       bar_sync<2 * GT>(5);
       constexpr int kLp = MINB == 1 ? 4 : 8;  // one turn per round while the registers hold the rows
-      if (!near) jacobi_group<2 * GT, 8, 16, false>(M, ldm, s, sm.sig, sm.mx, sm.flag, tid, 6);
-      else if (s <= 64) jacobi_group<2 * GT, 8, 8, true>(M, ldm, s, sm.sig, sm.mx, sm.flag, tid, 6);
-      else if (s <= 96) jacobi_group<2 * GT, kLp, 96 / kLp, true>(M, ldm, s, sm.sig, sm.mx, sm.flag, tid, 6);
-      else jacobi_group<2 * GT, kLp, 128 / kLp, true>(M, ldm, s, sm.sig, sm.mx, sm.flag, tid, 6);
+      if (!near) jacobi_group<2 * GT, 8, 16, false>(M, ldm, s, kFloor, sm.sig, sm.mx, sm.flag, tid, 6);
+      else if (s <= 64) jacobi_group<2 * GT, 8, 8, true>(M, ldm, s, kFloor, sm.sig, sm.mx, sm.flag, tid, 6);
+      else if (s <= 96) jacobi_group<2 * GT, kLp, 96 / kLp, true>(M, ldm, s, kFloor, sm.sig, sm.mx, sm.flag, tid, 6);
+      else jacobi_group<2 * GT, kLp, 128 / kLp, true>(M, ldm, s, kFloor, sm.sig, sm.mx, sm.flag, tid, 6);
     };
     const bool prod = side == 0 ? short_v : !short_v;  // this side's panel is -P W
 #pragma unroll 1
@@ -401,16 +402,16 @@ __global__ void __launch_bounds__(GW * 64, MINB)
         if (sd.gw == 0) {
           if (s <= 8) {
             warp_core_r<8>(M, ldm, s, sm.srt);
-            jacobi_warp<4, 2>(M, ldm, s);
+            jacobi_warp<4, 2>(M, ldm, s, kFloor);
           } else if (s <= 16) {
             warp_core_r<16>(M, ldm, s, sm.srt);
-            jacobi_warp<4, 4>(M, ldm, s);
+            jacobi_warp<4, 4>(M, ldm, s, kFloor);
           } else if (s <= 24) {
             warp_core_r<24>(M, ldm, s, sm.srt);
-            jacobi_warp<2, 16>(M, ldm, s);
+            jacobi_warp<2, 16>(M, ldm, s, kFloor);
           } else {
             warp_core_r<32>(M, ldm, s, sm.srt);
-            jacobi_warp<2, 16>(M, ldm, s);
+            jacobi_warp<2, 16>(M, ldm, s, kFloor);
           }
         }
       }

@@ -9,7 +9,7 @@ import host_cuda
 MAIN = r"""
 #include "tlr_compress.cu"
 using namespace tlr;
-// usage: main b k in_smem scale seed cta_order thread_order flip_orth flip_finalize
+// usage: main b k in_smem scale seed cta_order thread_order flip_orth flip_finalize [threshold]
 int main(int argc, char** argv) {
   const int b = atoi(argv[1]), k = atoi(argv[2]), in_smem = atoi(argv[3]);
   const double scale = atof(argv[4]);
@@ -24,7 +24,7 @@ int main(int argc, char** argv) {
   cfg.flip_word = status;
   auto* prm = const_cast<EvalParams*>(eval_params(status));
   prm->rule_fixed = 1;
-  prm->thr_rel = 1e-7;
+  prm->thr_rel = argc > 10 ? atof(argv[10]) : 1e-7;
   const int ti[] = {2, 2}, tj[] = {0, 1};  // storage tiles 0 and 1; tile row 2 is ragged
   int need[] = {1, 1}, rank[] = {-1, -1};
   auto T = [&](int c, int a, int q) { return scale / (1.0 + 0.04 * (ti[c] * b + a - tj[c] * b - q)); };
@@ -101,7 +101,15 @@ int main(int argc, char** argv) {
     worst = std::max(worst, sqrt(e2) * (scale / fro[c]));
     if (!(e2 >= 0.0)) worst = 9.0;
   }
-  printf("error %.17g orth %.17g ranks %d %d\n", worst, orth, rank[0], rank[1]);
+  double vorth = 0.0;
+  for (int c = 0; c < nc; ++c)
+    for (int p = 0; p < rank[c]; ++p)
+      for (int q = 0; q <= p; ++q) {
+        double s = p == q ? -1.0 : 0.0;
+        for (int w = 0; w < b; ++w) s += V[((size_t)c * cap + p) * b + w] * V[((size_t)c * cap + q) * b + w];
+        vorth = std::max(vorth, s == s ? fabs(s) : 9.0);
+      }
+  printf("error %.17g orth %.17g ranks %d %d V %.17g\n", worst, orth, rank[0], rank[1], vorth);
   for (int c = 0; c < nc; ++c)
     for (int q = 0; q < rank[c]; ++q)
       for (int w = 0; w < b; ++w) printf("%a %a\n", U[((size_t)c * cap + q) * b + w], V[((size_t)c * cap + q) * b + w]);
@@ -142,3 +150,11 @@ def test_tiles_of_any_size(exe, k, in_smem, scale):
     """The columns of T^T T P are squares of the tile's entries, and their norms are squared once more: the basis
     and the pair are those of a tile of ordinary size."""
     _check(host_cuda.run(exe, 48, k, in_smem, scale, 1, 0, 0, -1, -1))
+
+
+@pytest.mark.parametrize("k", [24, 32, 64])
+def test_right_vectors_at_rounding_level(exe, k):
+    """A threshold below 1e-14 of the tile keeps singular values at rounding level: their right vectors are
+    orthonormal too (the recompression relies on it).  Bound: k eps with a margin."""
+    w = host_cuda.run(exe, 24, k, int(k <= 32), 1, 1, 0, 0, -1, -1, 1e-15).split()
+    assert w[0] == "error" and float(w[8]) <= 1e-13, w[:10]
