@@ -14,15 +14,15 @@ constexpr int kRu = 3;  // blocks of 8 columns per reduction of a product
 // root (an FP64 step costs about 23 cycles of latency here, a square root 120, a division 77).
 // The squared norm alpha^2 + sig2 has to lie within 2^-500 .. 2^500: past that kappa and the products with v
 // would leave the range of a double (kappa is infinite for norms below 7e-155, and the columns of T^T T P
-// are squares of a tile's entries).  A column outside is first multiplied by column_lift, a power of two, which
-// changes no bit of the reflector; beta is divided by it.
-__device__ __forceinline__ double column_lift(double norm2) {
+// are squares of a tile's entries).  A column outside is first multiplied by 2^(500 column_lift), which changes
+// no bit of the reflector; beta is divided by it.  Integers, so that an ordinary column pays a few cycles.
+__device__ __forceinline__ int column_lift(double norm2) {
   constexpr int kLow = (1023 - 500) << 20, kHigh = (1023 + 500) << 20;  // high words of 2^-500, 2^500
-  if ((unsigned)(__double2hiint(norm2) - kLow) <= (unsigned)(kHigh - kLow) || norm2 == 0.0) return 1.0;
-  return norm2 < 1.0 ? 0x1p500 : 0x1p-500;
+  if ((unsigned)(__double2hiint(norm2) - kLow) <= (unsigned)(kHigh - kLow) || norm2 == 0.0) return 0;
+  return norm2 < 1.0 ? 1 : -1;
 }
-__device__ __forceinline__ double unlift(double lift, double v) {
-  return lift == 1.0 ? v : v * (lift > 1.0 ? 0x1p-500 : 0x1p500);
+__device__ __forceinline__ double lifted(int lift, double v) {
+  return lift == 0 ? v : v * (lift > 0 ? 0x1p500 : 0x1p-500);
 }
 struct Reflector {
   double beta, d, kappa;
@@ -248,7 +248,7 @@ struct Side {
     // one body for every column (the code of a pair runs once per pair, so its size is instruction
     // fetches): the current column is y[.][0], the panel rotates by one column a step, and position j
     // holds column (j + c) mod 8
-    double lift = 1.0;
+    int lift = 0;
 #pragma unroll 1
     for (int c = 0, step = 0; c < nc; ++step) {
       const int piv = r0 + c, live = 8 - c;  // positions from `live` on: finished reflectors
@@ -297,12 +297,12 @@ struct Side {
       for (int w = 1; w < GW; ++w)
 #pragma unroll
         for (int j = 0; j < 8; ++j) s[j] += rb[w * 8 + j];
-      if (lift == 1.0) {
+      if (lift == 0) {
         lift = column_lift(fma(pv[0], pv[0], s[0]));
-        if (lift != 1.0) {  // the same in every thread: the rows from the pivot on, and the sums once more
+        if (lift != 0) {  // the same in every thread: the rows from the pivot on, and the sums once more
 #pragma unroll
           for (int i = 0; i < kRpt; ++i)
-            if (tg + GT * i >= piv) y[i][0] *= lift;
+            if (tg + GT * i >= piv) y[i][0] = lifted(lift, y[i][0]);
           continue;
         }
       }
@@ -323,12 +323,12 @@ struct Side {
 #pragma unroll
       for (int i = 0; i < kRpt; ++i) {
         double y0 = y[i][0];
-        if (i == 0 && tg == piv) y0 = unlift(lift, rf.beta);
+        if (i == 0 && tg == piv) y0 = lifted(-lift, rf.beta);
 #pragma unroll
         for (int j = 0; j < 7; ++j) y[i][j] = y[i][j + 1];
         y[i][7] = y0;
       }
-      lift = 1.0;
+      lift = 0;
       ++c;
     }
     if (tg < nrow) {
@@ -383,7 +383,8 @@ __device__ __noinline__ void warp_core_r(double* M, int ldm, int s, double* buf)
       for (int i = 0; i < NR; i += 2) *reinterpret_cast<double2*>(xb + i) = make_double2(m[i], m[i + 1]);
     }
     __syncwarp();
-    double x[NR], sig2, dt, lift = 1.0;
+    double x[NR], sig2, dt;
+    int lift = 0;
 #pragma unroll
     for (int i = 0; i < NR; i += 2) {
       const double2 v = *reinterpret_cast<const double2*>(xb + i);
@@ -400,15 +401,15 @@ __device__ __noinline__ void warp_core_r(double* M, int ldm, int s, double* buf)
       }
       sig2 = (sa[0] + sa[1]) + (sa[2] + sa[3]);
       dt = (da[0] + da[1]) + (da[2] + da[3]);
-      if (lift != 1.0) break;
+      if (lift != 0) break;
       lift = column_lift(fma(x[0], x[0], sig2));
-      if (lift == 1.0) break;
+      if (lift == 0) break;
 #pragma unroll
-      for (int i = 0; i < NR; ++i) x[i] *= lift;
+      for (int i = 0; i < NR; ++i) x[i] = lifted(lift, x[i]);
     }
     const Reflector rf = reflector(x[0], sig2);
     const double w = rf.kappa * fma(rf.d, m[0], dt);
-    if (j < s) M[c * ldm + j] = j < c ? 0.0 : (j == c ? unlift(lift, rf.beta) : fma(-w, rf.d, m[0]));
+    if (j < s) M[c * ldm + j] = j < c ? 0.0 : (j == c ? lifted(-lift, rf.beta) : fma(-w, rf.d, m[0]));
 #pragma unroll
     for (int i = 1; i < NR; ++i) m[i - 1] = fma(-w, x[i], m[i]);
     m[NR - 1] = 0.0;
@@ -422,7 +423,8 @@ __device__ __noinline__ void group_core_r(double* M, int ldm, int s, int tg, int
   if (SHARED) __builtin_assume(__isShared(M));
   const int nsp = s <= GT / 4 ? 4 : s <= GT / 2 ? 2 : 1, sp = tg % nsp;
   for (int c = 0; c < s - 1; ++c) {
-    double sig2, alpha = M[c * ldm + c], lift = 1.0;
+    double sig2, alpha = M[c * ldm + c];
+    int lift = 0;
 #pragma unroll 1
     for (;;) {
       double sg[4] = {0.0, 0.0, 0.0, 0.0};
@@ -435,12 +437,12 @@ __device__ __noinline__ void group_core_r(double* M, int ldm, int s, int tg, int
       }
       sig2 = (sg[0] + sg[1]) + (sg[2] + sg[3]);
       for (int o = 1; o < nsp; o <<= 1) sig2 += __shfl_xor_sync(0xffffffffu, sig2, o);
-      if (lift != 1.0) break;
+      if (lift != 0) break;
       lift = column_lift(fma(alpha, alpha, sig2));
-      if (lift == 1.0) break;
+      if (lift == 0) break;
       bar_sync<GT>(bar);  // the same in every thread: the column below the pivot is the reflector's alone
-      for (int r = c + 1 + tg; r < s; r += GT) M[r * ldm + c] *= lift;
-      alpha *= lift;
+      for (int r = c + 1 + tg; r < s; r += GT) M[r * ldm + c] = lifted(lift, M[r * ldm + c]);
+      alpha = lifted(lift, alpha);
       bar_sync<GT>(bar);
     }
     const Reflector rf = reflector(alpha, sig2);
@@ -481,7 +483,7 @@ __device__ __noinline__ void group_core_r(double* M, int ldm, int s, int tg, int
       }
     }
     bar_sync<GT>(bar);
-    if (tg == 0) M[c * ldm + c] = unlift(lift, rf.beta);
+    if (tg == 0) M[c * ldm + c] = lifted(-lift, rf.beta);
   }
   bar_sync<GT>(bar);
   for (int e = tg; e < s * s; e += GT) {
