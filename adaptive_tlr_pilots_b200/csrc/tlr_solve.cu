@@ -16,6 +16,8 @@
 // Per launch at b = 500, one column: diagonal solve 49 -> 33 us (L) and 43 -> 37 us (L^T), coupling
 // 26 -> 8.4 us against loads next to their use.  Kriging at N = 20,000, b = 500 with 300 sites (two solves
 // of one column, one of 300): 174 ms with one thread per column by substitution, 6.6 ms now.
+#include <float.h>
+
 #include "tlr_device.cuh"
 #include "tlr_kernels.h"
 
@@ -69,7 +71,9 @@ __global__ void __launch_bounds__(64) k_diag_inv(const double* TLR_RESTRICT D, i
 
 // X_k <- L_kk^{-1} X_k (TRANS false) or L_kk^{-T} X_k (true), kSC columns per CTA in shared memory, panels
 // of 32 rows: X_p <- inv_p X_p, then the other rows lose L[., p] X_p.  Tiles of the products have a column
-// of X as their row (lane (g, t) holds column g, rows 2t and 2t + 1).
+// of X as their row (lane (g, t) holds column g, rows 2t and 2t + 1).  A right-hand side with an infinity or NaN
+// is substituted row by row: the products multiply it by the zeros of the inverses and would carry it to rows
+// that do not depend on it.
 template <bool TRANS>
 __global__ void __launch_bounds__(kSW * 32) k_tri_solve(const double* TLR_RESTRICT D, const double* TLR_RESTRICT inv,
                                                        int n, int b, int np, int k, double* TLR_RESTRICT X, int ldx,
@@ -83,11 +87,36 @@ __global__ void __launch_bounds__(kSW * 32) k_tri_solve(const double* TLR_RESTRI
   __shared__ __align__(16) double xp[kSC * kXpPitch];
   const int ld = npk * 32 + (TRANS ? 8 : 4);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  auto store = [&]() {
+    for (int e = tid; e < npk * 32 * nc; e += kSW * 32) {
+      const int r = e % (npk * 32), c = e / (npk * 32);
+      if (r < bk) X[(size_t)(c0 + c) * ldx + (size_t)k * b + r] = xs[c * ld + r];
+    }
+  };
+  bool finite = true;
   for (int e = tid; e < npk * 32 * kSC; e += kSW * 32) {
     const int r = e % (npk * 32), c = e / (npk * 32);
-    xs[c * ld + r] = (c < nc && r < bk) ? X[(size_t)(c0 + c) * ldx + (size_t)k * b + r] : 0.0;
+    const double v = (c < nc && r < bk) ? X[(size_t)(c0 + c) * ldx + (size_t)k * b + r] : 0.0;
+    finite = finite && fabs(v) <= DBL_MAX;
+    xs[c * ld + r] = v;
   }
-  __syncthreads();
+  if (__syncthreads_or(!finite)) {
+    double* x = xs + warp * ld;  // a warp per column
+    for (int s = 0; s < bk && warp < nc; ++s) {
+      const int r = TRANS ? bk - 1 - s : s;
+      double acc = 0.0;
+      for (int q = lane; q < s; q += 32) {
+        const int o = TRANS ? bk - 1 - q : q;  // solved before row r
+        acc = fma(TRANS ? L[(size_t)r * b + o] : L[(size_t)o * b + r], x[o], acc);
+      }
+      acc = warp_sum(acc);
+      if (lane == 0) x[r] = (x[r] - acc) / L[(size_t)r * b + r];
+      __syncwarp();
+    }
+    __syncthreads();
+    store();
+    return;
+  }
   const bool al = (b & 1) == 0;
   // row blocks of 16 that panel pi leaves to be solved, the next panel's first
   auto rest = [&](int pi) { return (npk - 1 - pi) * 2; };
@@ -192,10 +221,7 @@ __global__ void __launch_bounds__(kSW * 32) k_tri_solve(const double* TLR_RESTRI
     }
     __syncthreads();
   }
-  for (int e = tid; e < npk * 32 * nc; e += kSW * 32) {
-    const int r = e % (npk * 32), c = e / (npk * 32);
-    if (r < bk) X[(size_t)(c0 + c) * ldx + (size_t)k * b + r] = xs[c * ld + r];
-  }
+  store();
 }
 
 // trans 0: X_i -= U_ik (V_ik^T X_k) for i > k;  trans 1: X_j -= V_kj (U_kj^T X_k) for j < k.
