@@ -69,6 +69,23 @@ __global__ void __launch_bounds__(64) k_diag_inv(const double* TLR_RESTRICT D, i
   for (int r = 0; r < 32; r += 2) *reinterpret_cast<double2*>(o + r) = make_double2(x[r], x[r + 1]);
 }
 
+// One column by one warp, row by row.
+template <bool TRANS>
+__device__ __noinline__ void substitute(const double* L, int b, int bk, double* x) {
+  const int lane = threadIdx.x & 31;
+  for (int s = 0; s < bk; ++s) {
+    const int r = TRANS ? bk - 1 - s : s;
+    double acc = 0.0;
+    for (int q = lane; q < s; q += 32) {
+      const int o = TRANS ? bk - 1 - q : q;  // solved before row r
+      acc = fma(TRANS ? L[(size_t)r * b + o] : L[(size_t)o * b + r], x[o], acc);
+    }
+    acc = warp_sum(acc);
+    if (lane == 0) x[r] = (x[r] - acc) / L[(size_t)r * b + r];
+    __syncwarp();
+  }
+}
+
 // X_k <- L_kk^{-1} X_k (TRANS false) or L_kk^{-T} X_k (true), kSC columns per CTA in shared memory, panels
 // of 32 rows: X_p <- inv_p X_p, then the other rows lose L[., p] X_p.  Tiles of the products have a column
 // of X as their row (lane (g, t) holds column g, rows 2t and 2t + 1).  A right-hand side with an infinity or NaN
@@ -101,18 +118,7 @@ __global__ void __launch_bounds__(kSW * 32) k_tri_solve(const double* TLR_RESTRI
     xs[c * ld + r] = v;
   }
   if (__syncthreads_or(!finite)) {
-    double* x = xs + warp * ld;  // a warp per column
-    for (int s = 0; s < bk && warp < nc; ++s) {
-      const int r = TRANS ? bk - 1 - s : s;
-      double acc = 0.0;
-      for (int q = lane; q < s; q += 32) {
-        const int o = TRANS ? bk - 1 - q : q;  // solved before row r
-        acc = fma(TRANS ? L[(size_t)r * b + o] : L[(size_t)o * b + r], x[o], acc);
-      }
-      acc = warp_sum(acc);
-      if (lane == 0) x[r] = (x[r] - acc) / L[(size_t)r * b + r];
-      __syncwarp();
-    }
+    if (warp < nc) substitute<TRANS>(L, b, bk, xs + warp * ld);
     __syncthreads();
     store();
     return;
