@@ -166,7 +166,7 @@ int launch_dgemm_batched(const GemmJob* jobs, int njobs, int max_m, int max_n, c
   if (njobs <= 0) return 0;
   auto blocks = [](int n, int per) { return (unsigned)((n + per - 1) / per); };
   const long large = (long)blocks(max_n, DgLarge::kN) * blocks(max_m, DgLarge::kM) * njobs;
-  if (large >= 4 * 148) {  // two waves of two CTAs an SM
+  if (large >= 4 * kSms) {  // two waves of two CTAs an SM
     cudaFuncSetAttribute(k_dgemm_batched<4, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DgLarge::kSmem);
     k_dgemm_batched<4, 2, 4><<<dim3(blocks(max_n, DgLarge::kN), blocks(max_m, DgLarge::kM), (unsigned)njobs), DgLarge::kT,
                                DgLarge::kSmem, s>>>(jobs, status, kind);

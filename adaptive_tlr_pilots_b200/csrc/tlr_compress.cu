@@ -293,9 +293,9 @@ __global__ void __launch_bounds__(W * 32, 16 / W)
 // Blocked Householder QR of a bt x k panel by one CTA (a tlr::Side of GW warps): blocks of 8 columns go
 // through the earlier reflector blocks and their own QR in registers, products and updates on the FP64
 // tensor cores.  Bound by its chain of k column steps (about 800 cycles each, one barrier) and, for k > 8,
-// the block applications between them; per FP64 evaluation at N = 50,000, b = 500: k_orth 25.8 -> 11.9 ms,
+// the block applications between them; per FP64 evaluation at N = 50,000, b = 500: k_orth 25.8 -> 12.6 ms,
 // k_finalize 15.9 -> 5.5 ms against a column-by-column QR with the core's SVD in shared memory; at
-// N = 1,030, b = 100: 0.54 -> 0.29 and 0.68 -> 0.16 ms.
+// N = 1,030, b = 100: 0.54 -> 0.30 and 0.68 -> 0.16 ms.
 template <int GW, int NBLK>
 struct PanelShared {
   static constexpr int kLdx = Side<GW, NBLK>::kLdx;

@@ -47,6 +47,8 @@ int launch_morton(const double* xy, int n, int order, unsigned* work, long long*
 int launch_gather_sites(const double* xy_in, const double* y_in, const long long* perm, int n, double* xy_out,
                         double* y_out, cudaStream_t s);
 
+constexpr int kSms = 148;  // of a B200, for the rules that choose a launch shape
+
 // initial compression
 size_t tile_doubles(int b);  // doubles of one generated tile T (row-major, even pitch)
 int launch_gen_offdiag(const double* xy, int n, int b, int tile_base, const int* ti, const int* tj, double* T,

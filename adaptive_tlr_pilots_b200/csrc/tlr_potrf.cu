@@ -22,7 +22,7 @@
 //     the panel is final, because every other access to the tile bypasses L1);
 //   * two cluster barriers per panel, split into arrive and wait: warp 0 runs past the first.
 // Measured (one tile alone): b = 100: 109 -> 35 us, b = 250: 300 -> 72 us, b = 500: 820 -> 162 us,
-// b = 1000: 8400 -> 610 us against the form that inverted each diagonal block and updated with
+// b = 1000: 8400 -> 623 us against the form that inverted each diagonal block and updated with
 // CUDA-core products from a staged panel.
 #include <cooperative_groups.h>
 
@@ -72,7 +72,7 @@ __device__ __forceinline__ int factor_block(double (&row)[kPB], double* lc, doub
   for (int c = 0; c < kPB; ++c) {
     bad |= !(d > 0.0);
     const double rs = rsqrt(d);
-    const double l = row[c] * rs;  // at lane c: sqrt(d)
+    const double l = row[c] * rs;  // at lane c: sqrt(d) to two roundings
     row[c] = l;
     if (c + 1 < kPB) {
       // the next pivot from its own lane, ahead of the other updates

@@ -29,8 +29,9 @@
 // the CTA's slot of global scratch (L2).
 //
 // Recompression per FP64 evaluation, against one group of 256 threads per pair with a column at a time in
-// shared memory: N = 1,030, b = 100 3.7 -> 0.77 ms; N = 10,007, b = 250 17.9 -> 4.7; N = 50,000, b = 500
-// 138 -> 44.7; N = 20,000, b = 500, range 0.1 (ranks to 65) 382 -> 53.
+// shared memory: N = 1,030, b = 100 3.7 -> 0.78 ms; N = 10,007, b = 250 17.9 -> 4.8; N = 50,000, b = 500
+// 138 -> 45.6; N = 20,000, b = 500, range 0.1 (ranks to 65) 382 -> 52.  The range test of the reflectors
+// (tlr_panel.cuh) is 1 to 4 % of that (43.9 without it at N = 50,000).
 #include "tlr_kernels.h"
 #include "tlr_panel.cuh"
 
@@ -569,23 +570,27 @@ struct RcShape {
   }
 };
 constexpr int kTallXu = 18496;  // doubles of xu that hold, with xv, a core of order 150
-constexpr int kFewPairs = 148;  // one per SM
+constexpr int kFewPairs = kSms;  // one per SM
 // calls f with the shape for a tile size, a rank capacity and whether the step has at most kFewPairs pairs
 // (all shapes of a tile size have the same rows, so the same scratch slots)
 template <class F>
 auto rc_shape(int b, int cap, bool few, F f) {
-  // past the default capacity a plan has met ranks above 64: cores that do not fit beside a second CTA's
-  // shared memory are then what a step waits for (1.8 ms each through L2), so one CTA keeps the SM
-  // (recompression at N = 20,000, range 0.1, ranks to 65: 62 -> 53 ms)
+  // A capacity past 64 (asked for, or a plan that grew at a rank above it) allows cores that do not fit beside a
+  // second CTA's shared memory; a step waits for them (1.8 ms each through L2), so one CTA keeps the SM:
+  // recompression at N = 20,000, range 0.1, ranks to 65, 62 -> 53 ms.  The host queues a step before its ranks
+  // are known, so the capacity decides and low ranks pay for it: capacity 128 against 64 at mean ranks of 5
+  // to 7, N = 1,030, b = 100 0.79 -> 0.81 ms, N = 4,000, b = 250 1.74 -> 1.83, N = 10,007, b = 250 4.8 -> 5.2,
+  // N = 50,000, b = 500 45.9 -> 49.2 (the forward pass 129.5 -> 133.0), N = 20,000, range 0.2 12.3 -> 11.9.
   if (cap > 64) {
     if (b <= 128) return f(RcShape<4, 4, 1, kTallXu>{});
     if (b <= 256) return f(RcShape<4, 8, 1, kTallXu>{});
     if (b <= 512) return f(RcShape<4, 16, 1, kTallXu>{});
     return f(RcShape<8, 16, 1>{});
   }
-  // No second CTA to share the SM with: all its registers to one (255 a thread, no spills).  Recompression
-  // per evaluation: N = 1,030, b = 100 0.83 -> 0.77 ms, N = 4,000, b = 250 1.93 -> 1.68, N = 4,000, b = 203
-  // 2.94 -> 2.56; sixteen warps in its place 0.83, 1.84, 2.78.
+  // No second CTA to share the SM with: all its registers to one (255 a thread; b > 256 spills nothing then, the
+  // smaller shapes 80 bytes against 150).  Recompression per evaluation: N = 1,030, b = 100 0.83 -> 0.77 ms,
+  // N = 4,000, b = 250 1.93 -> 1.68, N = 4,000, b = 203 2.94 -> 2.56; sixteen warps in its place 0.83, 1.84, 2.78
+  // (all without the reflectors' range test).
   if (few) {
     if (b <= 128) return f(RcShape<4, 4, 1>{});
     if (b <= 256) return f(RcShape<4, 8, 1>{});

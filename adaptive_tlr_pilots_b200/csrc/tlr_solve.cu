@@ -15,7 +15,7 @@
 // coupling kernel keeps eight row blocks of a column (four with several column blocks) in flight per warp.
 // Per launch at b = 500, one column: diagonal solve 49 -> 33 us (L) and 43 -> 37 us (L^T), coupling
 // 26 -> 8.4 us against loads next to their use.  Kriging at N = 20,000, b = 500 with 300 sites (two solves
-// of one column, one of 300): 174 ms with one thread per column by substitution, 6.6 ms now.
+// of one column, one of 300): 174 ms with one thread per column by substitution, 6.7 ms now.
 #include <float.h>
 
 #include "tlr_device.cuh"
