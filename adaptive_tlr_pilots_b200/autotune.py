@@ -3,7 +3,7 @@ each) a PlanBatch should run for a given problem.
 
 More workspaces overlap more of the factorizations' latency-bound steps (the late steps with few
 trailing pairs, the POTRF clusters, the backward pass's per-block-row launches), until the
-recompression kernel saturates the GPU; each one holds a whole plan's memory (about 10 GB at
+recompression kernel saturates the GPU; each one holds a whole plan's memory (19 GB with its backward arena at
 N = 50,000, b = 500).  tune_workspaces() times a short batched loglik+grad run for every
 candidate that fits the device's free memory and records evals/s per candidate in a JSON table
 keyed by (N, b, rule, value, precision); PlanBatch(..., workspaces="auto") reads the table and

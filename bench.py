@@ -66,7 +66,7 @@ def parse():
 # dram__bytes_read.sum + dram__bytes_write.sum over the 98 launches of one evaluation, from an ncu
 # capture of `bench.py --steps 1 --warmup 1 --cpu-sample 0 --plain-steps 0 --batch 1 --dense 0 --graphs 0`
 # (the same kernels launched one by one: ncu's driver reported a failed launch replaying the graph)
-RC_TRAFFIC_N50K = 128.4e6
+RC_TRAFFIC_N50K = 129.4e6
 RC_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum, mean over the 98 k_recompress launches of "
                      "one evaluation (batch 1, same workload, launches one by one, 1-pass capture)")
 METRIC = "TLR loglik+grad evals/s at N=50k vs plain FP64 on B200; |dl| vs FP64 dense"
